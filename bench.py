@@ -171,9 +171,9 @@ def alg_bytes(nn):
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum, pass A + pass B)
 # per vector-matvec of the kernels the library picks, keyed by (NN,
 # storage): one ncu capture of the block-of-2 matvec at N=6 (`--workload
-# matvec-n6`), both passes' bytes over 2 vectors: ev_kernel<float, 13> and
-# ev_kernel<double, 13>.  Kernels without a capture report null.
-NCU_TRAFFIC_PER_VECTOR = {(13, "f32"): 149.3e6, (13, "f64"): 342.6e6}
+# matvec-n6`), the three kernels' bytes over 2 vectors.  Kernels without a
+# capture report null.
+NCU_TRAFFIC_PER_VECTOR = {(13, "f32"): 237.0e6, (13, "f64"): 552.3e6}
 
 # The timed solves keep the library's matvec events on for the roofline
 # figures, on every 8th MATBLOCK call of each storage: all calls of one
@@ -322,16 +322,10 @@ def dist_setup():
 
 
 def matvec_kernel_name(nn, fp32):
-    """The kernels the library picks for a grid (de_set_matvec_kernel's
-    default): even/odd-split kernels for complex64 at NN 9..17 and
-    complex128 at NN 9..13, streaming kernels at NN 15..19, cube kernels
-    elsewhere."""
+    """The kernels the library picks (de_set_matvec_kernel's default): the
+    line kernels on every grid."""
     r = "float" if fp32 else "double"
-    if 9 <= nn <= (17 if fp32 else 13):
-        return f"hammult ev_kernel<{r}, {nn}> pass A + pass B"
-    if 13 <= nn <= 19:
-        return f"hammult stream_kernel<{r}, {nn}> pass A + pass B"
-    return f"hammult cube_kernel<{r}, {nn}> pass A + pass B"
+    return f"hammult plane_kernel + kline_kernel (pass A) + cube_line_kernel (pass B) <{r}, {nn}>"
 
 
 class OracleBlockStep:

@@ -100,8 +100,8 @@ class Problem:
         check(lib().de_set_stream(self._h, ctypes.c_void_p(cuda_stream)), "de_set_stream")
 
     def set_matvec_kernel(self, kind: str) -> None:
-        """'fma' (default): the CUDA-core kernels on even/odd-split
-        contractions; 'tensor': the axis contractions on the FP64 tensor
+        """'fma' (default): the CUDA-core kernels that contract whole lines
+        in registers, even/odd-split (every grid); 'tensor': the axis contractions on the FP64 tensor
         cores where built (NN 9..19); 'stream': the earlier CUDA-core
         streaming kernels (NN 13..19); 'tf32': the complex64 matvec's
         kinetic contractions on the TF32 tensor cores with head/tail split

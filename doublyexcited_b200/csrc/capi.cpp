@@ -349,6 +349,7 @@ DE_API int de_problem_create(const de_params *pin, de_problem **out)
     hd.m = h->m;
     std::vector<double> t = kematrix(nn, delta);
     for (int d = 0; d < nn; ++d) hd.t[d] = t[d];  // T(d,0) = T(0,d)
+    hd.id2 = 1.0 / (delta * delta);
     hd.s2re = s2.real();
     hd.s2im = s2.imag();
     hd.vsre = vs.real();
@@ -374,7 +375,6 @@ DE_API int de_problem_create(const de_params *pin, de_problem **out)
     hd.v12 = h->d_v12;
     // FP32 copies of T and of the potential tables for the mixed form
     for (int d = 0; d < nn; ++d) hd.tf[d] = (float)t[d];
-    fill_ev_coefficients(hd);
     DE_CUDA(cudaMallocAsync(&h->d_t1af, h->m * sizeof(float), h->stream));
     DE_CUDA(cudaMallocAsync(&h->d_v12f, w * w * w * sizeof(float), h->stream));
     ce = to_f32_launch(h->d_t1a, h->d_t1af, h->m, h->stream);

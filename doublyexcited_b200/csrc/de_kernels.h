@@ -11,13 +11,12 @@ namespace de {
 // Process-wide count of kernels launched by this library.
 void count_launch(int n = 1);
 int64_t launch_count();
-// Whether the even/odd matvec kernels are launched as programmatic dependent
-// launches (they wait on the grid dependency after their table preload);
-// on unless the environment sets DE_PDL=0.  Read once per process.
+// Whether the line kernels are launched as programmatic dependent launches
+// (they wait on the grid dependency before their first read); on unless the
+// environment sets DE_PDL=0.  Read once per process.
 bool programmatic_launch();
 
 constexpr int kMaxNN = 27;      // N <= 13 (the reference ran N = 5..15)
-constexpr int kEvCoef = 12 * 12;  // even/odd coefficient tables, N <= 11
 constexpr int kMaxCols = 128;   // columns per block-op operand list
 
 // Operator data for one problem (HAMILTONIAN, structs.F90:87-102).
@@ -36,23 +35,17 @@ struct HamDev {
     const float *t1af;
     const float *v12f;
     // Matvec kernels per [storage: 0 complex128, 1 complex64][pass: 0 A, 1 B]:
-    // fam 0 even/odd-split (hammult_ev.cu; streaming / cube where those are
-    // not built), 1 FP64 tensor cores (hammult_tc.cu), 2 streaming / cube
-    // (hammult.cu), 3 tcgen05 TF32 (hammult_tc32.cu, complex64 on NN 9..15;
-    // even/odd elsewhere); ctas = resident CTAs per SM of the persistent
-    // kernels, 0 = as many as fit.  Filled from the tuning table at creation
-    // (tuning.cpp) or by de_set_matvec_kernel / de_set_matvec_launch.
+    // fam 0 lines in registers, even/odd split (hammult_line.cu), 1 FP64
+    // tensor cores (hammult_tc.cu, NN 9..19), 2 streaming / cube
+    // (hammult.cu), 3 tcgen05 TF32 (hammult_tc32.cu, complex64 on NN 9..15);
+    // 1 and 3 run family 0 on the other grids.  ctas = resident CTAs per SM
+    // of the persistent kernels (families 2 and 3), 0 = as many as fit.
+    // Filled from the tuning table at creation (tuning.cpp) or by
+    // de_set_matvec_kernel / de_set_matvec_launch.
     signed char fam[2][2];
     signed char ctas[2][2];
-    // Even/odd-split coefficients of T for the grid (hammult_ev.cu), index
-    // a * (N+1) + b: ev_ce(a,0) = t(a), ev_ce(a,b) = (t(|a-b|) + t(a+b))/2,
-    // ev_co(a,b) = (t(|a-b|) - t(a+b))/2 (a, b >= 1); FP32 copies beside.
-    double ev_ce[kEvCoef], ev_co[kEvCoef];
-    float ev_cef[kEvCoef], ev_cof[kEvCoef];
+    double id2;             // 1/delta^2 (delta^2 T depends on NN alone: hammult_line.cu)
 };
-
-// Fills ev_ce / ev_co (and the FP32 copies) from h.t for grid h.nn.
-void fill_ev_coefficients(HamDev &h);
 
 // The kinetic-eigenbasis preconditioner MSOLVECPLX22 (kinpc.cu): pass 0
 // writes Y = P on the row cubes, pass 1 adds P on the column cubes; w_dev =
@@ -85,14 +78,17 @@ cudaError_t hammult_pass_launch(const HamDev &h, const double2 *x, double2 *y, i
 cudaError_t hammult_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride, int pass,
                                 cudaStream_t st, double2 shift = double2{0.0, 0.0});
 
-// Even/odd-split form of one pass (hammult_ev.cu) for the grids
-// hammult_ev_supported accepts (complex128: NN = 9..13; complex64: NN =
-// 9..17); shs is the diagonal shift times SCALE^2.
-bool hammult_ev_supported(int nn, bool fp64);
+// One pass on the line kernels (hammult_line.cu), NN = 3..23 and both
+// storages; the same arguments and results as hammult_pass_launch.
+cudaError_t hammult_line_pass_launch(const HamDev &h, const double2 *x, double2 *y, int nvec, int64_t vstride,
+                                     int pass, cudaStream_t st, double2 shift);
+cudaError_t hammult_line_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride,
+                                     int pass, cudaStream_t st, double2 shift);
 
 // The complex64 passes with the kinetic contractions on the tensor cores
 // (tcgen05 kind::tf32, head/tail split; hammult_tc32.cu) for the grids
-// hammult_tc32_supported accepts (NN = 9..15); shs as above.  The kernels
+// hammult_tc32_supported accepts (NN = 9..15); shs is the diagonal shift
+// times SCALE^2.  The kernels
 // record a timed-out mbarrier wait in a device flag that
 // hammult_tc32_error reads and clears (1 = a wait gave up, -1 = the read
 // failed).
@@ -100,11 +96,6 @@ bool hammult_tc32_supported(int nn);
 cudaError_t hammult_tc32_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride,
                                      int pass, cudaStream_t st, double2 shs, int ctas = 0);
 int hammult_tc32_error(cudaStream_t st);
-cudaError_t hammult_ev_pass_launch(const HamDev &h, const double2 *x, double2 *y, int nvec, int64_t vstride,
-                                   int pass, cudaStream_t st, double2 shs, int ctas = 0);
-cudaError_t hammult_ev_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride, int pass,
-                                   cudaStream_t st, double2 shs, int ctas = 0);
-
 // Tensor-core (DMMA) form of one pass, for the grids hammult_tc_supported
 // accepts; the same arguments and results as hammult_pass_launch.
 bool hammult_tc_supported(int nn);

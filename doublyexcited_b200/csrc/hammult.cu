@@ -1,4 +1,6 @@
-// hammult.cu -- FP64 two-electron Hamiltonian matvec for sm_100a.
+// hammult.cu -- the streaming / shared-memory cube form of the two-electron
+// matvec (DE_MATVEC_STREAM), the one-electron operator, and the dispatch of a
+// pass over the kernel families (the default is hammult_line.cu).
 //
 // Reference: HAMMULT hammod.F90:19-67 -> KEMULT2 :138-187 -> KEMULTS
 // :264-286, plus Y = Y + V*X (:58-59) with V from POTENTIAL2 :502-582 scaled
@@ -627,24 +629,6 @@ cudaError_t dispatch(const HamDev &h, const CubeArgs<R> &a, int64_t ncubes, cuda
 
 }  // namespace
 
-void fill_ev_coefficients(HamDev &h)
-{
-    const int nn = h.nn, n = nn / 2;
-    for (int i = 0; i < kEvCoef; ++i) h.ev_ce[i] = h.ev_co[i] = 0.0;
-    if (n + 1 > 12) return;
-    auto t = [&](int d) { return d < nn ? h.t[d] : 0.0; };
-    for (int a = 0; a <= n; ++a)
-        for (int b = 0; b <= n; ++b) {
-            const int idx = a * (n + 1) + b;
-            h.ev_ce[idx] = b == 0 ? t(a) : 0.5 * (t(std::abs(a - b)) + t(a + b));
-            h.ev_co[idx] = (a >= 1 && b >= 1) ? 0.5 * (t(std::abs(a - b)) - t(a + b)) : 0.0;
-        }
-    for (int i = 0; i < kEvCoef; ++i) {
-        h.ev_cef[i] = (float)h.ev_ce[i];
-        h.ev_cof[i] = (float)h.ev_co[i];
-    }
-}
-
 template <class R>
 static CubeArgs<R> make_args(const HamDev &h, const C2<R> *x, C2<R> *y, int64_t vstride, double2 shift)
 {
@@ -670,9 +654,8 @@ static cudaError_t pass_go(const HamDev &h, const C2<R> *x, C2<R> *y, int nvec, 
         if (fam == 3 && hammult_tc32_supported(h.nn))
             return hammult_tc32_pass_launch(h, x, y, nvec, vstride, pass, st, a.shs, ctas);
     }
-    // even/odd kernels where they are built (hammult_ev_supported)
-    if ((fam == 0 || fam == 1 || fam == 3) && hammult_ev_supported(h.nn, sizeof(R) == 8))
-        return hammult_ev_pass_launch(h, x, y, nvec, vstride, pass, st, a.shs, ctas);
+    // the line kernels serve every grid; 2 asks for the streaming / cube kernels
+    if (fam != 2) return hammult_line_pass_launch(h, x, y, nvec, vstride, pass, st, shift);
     const int64_t ncubes = h.m * (int64_t)nvec;
     if (ncubes > 0x7fffffffLL) return cudaErrorInvalidValue;
     return pass == 0 ? dispatch<R, kRowsPot>(h, a, ncubes, st, ctas) : dispatch<R, kColsAcc>(h, a, ncubes, st, ctas);

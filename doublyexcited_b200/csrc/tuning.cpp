@@ -12,8 +12,8 @@
 // doublyexcited_b200.tune` writes it from timings on the GPU.  A problem
 // handle reads it at creation: the file DE_MATVEC_TUNING names (set but
 // empty: no table), else matvec_tuning.txt beside the library.  Grids,
-// passes or files without an entry keep the built-in choice (even/odd
-// kernels where built, all resident CTAs).
+// passes or files without an entry keep the built-in choice (the line
+// kernels, "ev").
 #include <dlfcn.h>
 
 #include <cstdio>

@@ -10,10 +10,11 @@ at creation (``matvec_tuning.txt`` beside the library, or ``--out``):
 
     <storage> <NN> <pass> <family> <ctas_per_sm> <ms_per_vector>
 
-Families: ``ev`` even/odd-split CUDA-core kernels, ``dmma`` FP64 tensor
-cores, ``stream`` streaming / cube CUDA-core kernels, ``tf32`` tcgen05 TF32
-tensor cores (complex64).  Candidates a grid does not build fall back to
-another family inside the library, so they are skipped here.  Timing: CUDA
+Families: ``ev`` even/odd-split lines in registers (CUDA cores, every grid),
+``dmma`` FP64 tensor cores, ``stream`` streaming / cube CUDA-core kernels,
+``tf32`` tcgen05 TF32 tensor cores (complex64).  Candidates a grid does not
+build fall back to another family inside the library, so they are skipped
+here.  Timing: CUDA
 events on the handle's stream, a block of vectors larger than L2 (at least
 256 MB), 2 warm-up and 5 timed matvecs per candidate, median of 3 rounds.
 """
@@ -24,8 +25,10 @@ import os
 import statistics
 import sys
 
-# grids each family builds (the library's *_supported functions)
+# grids each family builds (the library's *_supported functions); the line
+# kernels serve every grid and are timed first on these, last on larger ones
 EV = {"c128": range(9, 14, 2), "c64": range(9, 18, 2)}
+EV_LAST = range(15, 24, 2)
 DMMA = range(9, 20, 2)
 TF32 = range(9, 16, 2)
 STREAM_PERSISTENT = range(13, 20, 2)  # smaller grids run the non-persistent cube kernels
@@ -36,12 +39,14 @@ MARGIN = 0.02  # a candidate replaces the built-in choice only when this much fa
 def candidates(storage: str, nn: int):
     out = []
     if nn in EV[storage]:
-        out += [("ev", c) for c in (0, 1)]
+        out.append(("ev", 0))
     out += [("stream", c) for c in ((0, 1) if nn in STREAM_PERSISTENT else (0,))]
     if nn in DMMA:
         out.append(("dmma", 0))
     if storage == "c64" and nn in TF32:
         out += [("tf32", 0), ("tf32", 1)]
+    if nn in EV_LAST and nn not in EV[storage]:
+        out.append(("ev", 0))
     return out
 
 

@@ -150,12 +150,11 @@ DE_API int de_set_stream(de_problem *h, void *cuda_stream);
  * (gplmr.F90:42-57). */
 DE_API int de_set_profiling(de_problem *h, int on);
 /* Which matvec kernels a handle uses: DE_MATVEC_FMA (the default) the
- * fastest CUDA-core kernels per grid: even/odd-split contractions for the
- * mixed form's complex64 matvec at NN = 9..17 and the plain form's at NN =
- * 9..13, streaming kernels at NN = 15..19 otherwise, shared-memory cube
- * kernels elsewhere; DE_MATVEC_TENSOR the axis contractions on the FP64
- * tensor cores (DMMA) for NN = 9..19; DE_MATVEC_STREAM the streaming / cube
- * kernels everywhere (for comparison); DE_MATVEC_TF32 the mixed form's
+ * CUDA-core kernels that hold whole lines in registers and contract them
+ * even/odd-split, on every grid and in both storages; DE_MATVEC_TENSOR the
+ * axis contractions on the FP64 tensor cores (DMMA) for NN = 9..19;
+ * DE_MATVEC_STREAM the streaming kernels for NN = 13..19 and shared-memory
+ * cube kernels elsewhere (for comparison); DE_MATVEC_TF32 the mixed form's
  * complex64 matvec with its kinetic contractions on the 5th-generation
  * tensor cores (tcgen05, TF32 products of head/tail-split operands, FP32
  * accuracy) for NN = 9..15, the FMA kernels elsewhere and for complex128.
@@ -165,10 +164,9 @@ DE_API int de_set_matvec_kernel(de_problem *h, int kind);
 /* The kernels of one matvec pass.  storage 0 = complex128 matvecs, 1 =
  * complex64 (the mixed form's inner solve); pass 0 = electron-2 axes and
  * potential, 1 = electron-1 axes; family a DE_MATVEC_* kind (where a
- * family is not built for the grid, the even/odd kernels run, or the
- * streaming / cube kernels where those are not built either);
+ * family is not built for the grid, the FMA kernels run);
  * ctas_per_sm caps the resident CTAs per SM of the persistent kernels
- * (0 = as many as fit).  A handle starts from the tuning table written by
+ * (streaming and TF32; 0 = as many as fit; no effect on the others).  A handle starts from the tuning table written by
  * `python -m doublyexcited_b200.tune`: the file DE_MATVEC_TUNING names (set
  * but empty: none), else matvec_tuning.txt beside the library; entries it
  * lacks keep the FMA kernels with all resident CTAs.  No reference
