@@ -539,65 +539,6 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// G = op(L)^T R for up to 16 tiles of NLM x NRM outputs (nl*nr <= 512):
-// block b works on tile g = b % ntiles over the rows of row-block
-// b / ntiles, so the blocks that read the same rows run side by side and
-// share them through L2.  Partials of block b at work + 1 + 32*b; the last
-// block reduces each tile in a fixed order.
-template <class S, int NLM, int NRM>
-__global__ void __launch_bounds__(256)
-    gram_grouped(const __grid_constant__ ColListT<S> L, const __grid_constant__ ColListT<S> R, int64_t len,
-                 int herm, int ngl, int ntiles, double2 *__restrict__ work, double2 *__restrict__ out, int ldo)
-{
-    const int g = blockIdx.x % ntiles, rb = blockIdx.x / ntiles, nrb = gridDim.x / ntiles;
-    const int li0 = (g % ngl) * NLM, rj0 = (g / ngl) * NRM;
-    const int nl = min(NLM, L.n - li0), nr = min(NRM, R.n - rj0);
-    double ar[NLM * NRM], ai[NLM * NRM];
-#pragma unroll
-    for (int k = 0; k < NLM * NRM; ++k) ar[k] = ai[k] = 0.0;
-    const double sg = herm ? -1.0 : 1.0;
-    const int64_t stride = (int64_t)nrb * blockDim.x;
-    for (int64_t r = (int64_t)rb * blockDim.x + threadIdx.x; r < len; r += stride) {
-        double2 rv[NRM];
-#pragma unroll
-        for (int j = 0; j < NRM; ++j) rv[j] = (j < nr) ? col_elem(R, rj0 + j, r) : make_double2(0.0, 0.0);
-#pragma unroll
-        for (int i = 0; i < NLM; ++i) {
-            if (i < nl) {
-                double2 lv = col_elem(L, li0 + i, r);
-                lv.y *= sg;
-#pragma unroll
-                for (int j = 0; j < NRM; ++j) {
-                    const int k = i * NRM + j;
-                    ar[k] = fma(lv.x, rv[j].x, ar[k]);
-                    ar[k] = fma(-lv.y, rv[j].y, ar[k]);
-                    ai[k] = fma(lv.x, rv[j].y, ai[k]);
-                    ai[k] = fma(lv.y, rv[j].x, ai[k]);
-                }
-            }
-        }
-    }
-    unsigned *ticket = reinterpret_cast<unsigned *>(work);
-    double2 *part = work + 1;
-    constexpr int nout = NLM * NRM;
-    block_sum<nout>(ar, ai, part + (int64_t)blockIdx.x * 32, nout);
-    if (last_block(ticket, gridDim.x)) {
-        __shared__ double2 res[32];
-        for (int t = 0; t < ntiles; ++t) {
-            // tile t's partials: blocks t, t + ntiles, ... (stride ntiles*32)
-            reduce_partials(part + (int64_t)t * 32, nrb, ntiles * 32, nout, res);
-            const int ti0 = (t % ngl) * NLM, tj0 = (t / ngl) * NRM;
-            const int tnl = min(NLM, L.n - ti0), tnr = min(NRM, R.n - tj0);
-            for (int o = threadIdx.x; o < tnl * tnr; o += blockDim.x) {
-                const int i = o / tnr, j = o % tnr;
-                out[(ti0 + i) + (int64_t)ldo * (tj0 + j)] = res[i * NRM + j];
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) *ticket = 0u;
-    }
-}
-
 // Gram-Schmidt step of myhgramschmidt_many (harmonic_ritz_small.F90:52-59):
 //   q -= sum_i Qp_i d_i ; v -= sum_i Vp_i d_i ; c = 1/sqrt(|<q,q>|)
 // with d (m values) and the output c in device memory.
@@ -1237,23 +1178,6 @@ cudaError_t gs_update_launch(const float2 *const *qp, const float2 *const *vp, i
     return gs_update_go(qp, vp, m, q, v, d, len, work, cout, st);
 }
 
-template <class S>
-static cudaError_t gram_grouped_go(const ColListT<S> &L, const ColListT<S> &R, int64_t len, int herm, double2 *out,
-                                   int ldo, double2 *work, cudaStream_t st)
-{
-    constexpr int TL = 4, TR = 2;  // 8 outputs a tile: few registers, several blocks per SM
-    const int ngl = (L.n + TL - 1) / TL, ngr = (R.n + TR - 1) / TR;
-    const int ntiles = ngl * ngr;
-    if (ntiles > 16) return cudaErrorInvalidValue;
-    // one wave of blocks, a whole number of row-blocks per tile
-    const int64_t rows_blocks =
-        std::max<int64_t>(1, std::min<int64_t>((len + 255) / 256, wave_blocks<gram_grouped<S, TL, TR>>() / ntiles));
-    gram_grouped<S, TL, TR><<<(unsigned)(rows_blocks * ntiles), 256, 0, st>>>(L, R, len, herm, ngl, ntiles, work, out,
-                                                                             ldo);
-    count_launch();
-    return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------- Gram on the FP64 tensor cores
 // G = op(L)^T R as real GEMMs over the rows on DMMA (mma.sync m8n8k4 f64):
 // with L = Lr + i Li, R = Rr + i Ri,
@@ -1440,31 +1364,29 @@ static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t 
         if (L.n <= 16) return gram_small_go<16, 1>(L, R, len, herm, out, ldo, work, st);
         return gram_small_go<32, 1>(L, R, len, herm, out, ldo, work, st);
     }
-    if (L.n <= 2 && R.n <= 2) return gram_small_go<2, 2>(L, R, len, herm, out, ldo, work, st);
-    if (L.n <= 4 && R.n <= 4) return gram_small_go<4, 4>(L, R, len, herm, out, ldo, work, st);
-    if (L.n <= 8 && R.n <= 4) return gram_small_go<8, 4>(L, R, len, herm, out, ldo, work, st);
-    if (L.n <= 4 && R.n <= 8) return gram_small_go<4, 8>(L, R, len, herm, out, ldo, work, st);
-    // a few grouped tiles beat the tiled kernel; at 8 x 16 (the K/M projection
-    // of NEV = 1) the tiled kernel is faster (2.2 vs 1.2 ms at N = 6)
-    if (((L.n + 3) / 4) * ((R.n + 1) / 2) <= 6) return gram_grouped_go(L, R, len, herm, out, ldo, work, st);
-    {  // everything else on the FP64 tensor cores
-        // warp tiles sized to the output: no more padded tiles than needed
-        const int mt = (L.n + 7) / 8, nt = (R.n + 7) / 8;
-        if (L.n == 8 && R.n == 16 && herm) {  // the projection of one column with a P block
-            bool km8 = R.sigma.x == L.sigma.x && R.sigma.y == L.sigma.y;
-            for (int c = 0; c < 8 && km8; ++c)
-                km8 = L.b[c] && R.a[c] == L.a[c] && R.b[c] == L.b[c] && R.a[8 + c] == L.b[c] && !R.b[8 + c];
-            if (km8) return gram_tc_go<S, 1, 2, true>(L, R, len, herm, out, ldo, work, st);
-        }
-        if (mt == 1) {
-            if (nt == 1) return gram_tc_go<S, 1, 1>(L, R, len, herm, out, ldo, work, st);
-            if (nt <= 4) return gram_tc_go<S, 1, 2>(L, R, len, herm, out, ldo, work, st);
-            return gram_tc_go<S, 1, 4>(L, R, len, herm, out, ldo, work, st);
-        }
-        if (nt == 1) return gram_tc_go<S, 2, 1>(L, R, len, herm, out, ldo, work, st);
-        if (nt <= 4) return gram_tc_go<S, 2, 2>(L, R, len, herm, out, ldo, work, st);
-        return gram_tc_go<S, 2, 4>(L, R, len, herm, out, ldo, work, st);
+    // up to 4 x 4 of a short vector in one fused launch, all operands straight
+    // into registers: 13 us against 15 for the tiles at 118 K rows, 70 against
+    // 33 at 1.8 M
+    if (L.n <= 4 && R.n <= 4 && len < (1 << 18)) {
+        if (L.n <= 2 && R.n <= 2) return gram_small_go<2, 2>(L, R, len, herm, out, ldo, work, st);
+        return gram_small_go<4, 4>(L, R, len, herm, out, ldo, work, st);
     }
+    if (L.n == 8 && R.n == 16 && herm) {  // the projection of one column with a P block
+        bool km8 = R.sigma.x == L.sigma.x && R.sigma.y == L.sigma.y;
+        for (int c = 0; c < 8 && km8; ++c)
+            km8 = L.b[c] && R.a[c] == L.a[c] && R.b[c] == L.b[c] && R.a[8 + c] == L.b[c] && !R.b[8 + c];
+        if (km8) return gram_tc_go<S, 1, 2, true>(L, R, len, herm, out, ldo, work, st);
+    }
+    // the tiles keep one shift; no caller has two
+    bool one_shift = true;
+    if (R.sigma.x != L.sigma.x || R.sigma.y != L.sigma.y)
+        for (int j = 0; j < R.n; ++j) one_shift = one_shift && !R.b[j];
+    if (one_shift && gram_tile_supported(L.n, R.n)) return gram_tile_launch(L, R, len, herm, out, ldo, work, st);
+    // everything else on the FP64 tensor cores, warp tiles sized to the output
+    const int mt = (L.n + 7) / 8, nt = (R.n + 7) / 8;
+    if (mt == 1) return gram_tc_go<S, 1, 4>(L, R, len, herm, out, ldo, work, st);
+    if (nt <= 4) return gram_tc_go<S, 2, 2>(L, R, len, herm, out, ldo, work, st);
+    return gram_tc_go<S, 2, 4>(L, R, len, herm, out, ldo, work, st);
 }
 
 cudaError_t gram_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out, int ldo,

@@ -130,6 +130,14 @@ cudaError_t gram_launch(const ColList &L, const ColList &R, int64_t len, int her
 cudaError_t gram_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,
                         double2 *work, cudaStream_t st);
 
+// The same on output tiles fed through shared memory (gram_tile.cu), for the
+// shapes gram_tile_supported accepts; L and R share one shift (L.sigma).
+bool gram_tile_supported(int nl, int nr);
+cudaError_t gram_tile_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out, int ldo,
+                             double2 *work, cudaStream_t st);
+cudaError_t gram_tile_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,
+                             double2 *work, cudaStream_t st);
+
 // Hermitian Gram G = Z^H Z of n <= 7 complex64 vectors (FP64 sums), all n x n
 // entries written to DEVICE out (column-major, ldo); work as for gram.
 cudaError_t gram_herm_launch(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st);

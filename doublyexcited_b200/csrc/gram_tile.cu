@@ -1,0 +1,316 @@
+// gram_tile.cu -- Gram matrices of a few columns against a few columns,
+// G(i,j) = sum_r op(L_i[r]) R_j[r] (crossmult lamod.f90:51-125, the K/M
+// projection ZGEMMs gplmr.F90:207-267), up to 32 4 x 4 output tiles.
+//
+// Bound by HBM: 16 bytes per row and distinct column (8 in complex64) against
+// 8 nl nr FP64 flops.  The earlier kernels read every column straight into
+// registers, once per output tile and with a few loads in flight.  Here a CTA
+// streams row tiles of the distinct columns through a cp.async ring (a column
+// that occurs in L and in R, or as the partner of a shift, is read once), and
+// each warp forms one 4 x 4 tile of outputs, a lane per row: 8 shared-memory
+// reads for 64 FP64 multiply-adds, so shared memory and the FP64 pipe take
+// about the same time, both below the HBM time up to 8 x 16 outputs.
+//
+// us on B200, complex128, before -> now (HBM time of the distinct columns in
+// brackets):
+//   4.8 M rows   8 x 16    837 -> 384 [283]      5 x 3   547 -> 117 [94]
+//                16 x 16  1440 -> 769 [378]      24 x 8 1443 -> 606 [378]
+//                7 x 14 shifted projection       460 -> 433 [165]
+//   1.8 M rows   8 x 4     308 ->  73 [52]      20 x 4   494 -> 123 [104]
+//                4 x 4 of itself  70 ->  33 [17]
+//   118 K rows   8 x 16     46 ->  23           20 x 4    52 ->  21
+// complex64 (1.8 M rows): 10 x 12 502 -> 196, 20 x 24 1259 -> 737.  The shifted
+// 8 x 16 projection stays on gram_tc's one-load form (294 us against 446).
+#include "de_kernels.h"
+
+#include <algorithm>
+#include <atomic>
+
+namespace de {
+namespace {
+
+constexpr int kTile = 4;       // outputs of a warp: kTile x kTile
+constexpr int kWarps = 8;      // output tiles x row groups of a CTA
+constexpr int kFusedOut = 32;  // up to as many outputs the last CTA adds the partials
+constexpr int kMaxSlots = 40;  // distinct columns: 4 (tl + tr), and as many shift partners
+
+template <class S>
+struct GramTileArgs {
+    const S *col[kMaxSlots];            // the distinct columns
+    unsigned char shifted[kMaxSlots], partner[kMaxSlots];  // slots that become a - sigma b, and b's
+    unsigned char lslot[kTile * kWarps], rslot[kTile * kWarps];
+    double2 sigma;
+    int64_t len;
+    int nslots, nshift, nl, nr, tl, tr, stages;
+    double sign;  // -1: conj(L)
+    double2 *work, *out;  // work[0]: the fused reductions' ticket, zero between launches
+    int ldo;
+};
+
+template <class S>
+__device__ __forceinline__ void copy_async(S *s, const S *g, bool in)
+{
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(s);
+    const int n = in ? (int)sizeof(S) : 0;  // rows past the end read as zero
+    if constexpr (sizeof(S) == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(g), "r"(n) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(g), "r"(n) : "memory");
+}
+
+// Output o: its nblk partials added by one warp in a fixed order.
+__device__ __forceinline__ void sum_partials(const double2 *work, int nblk, int nl, int nout, int o, int lane,
+                                             double2 *out, int ldo)
+{
+    double x = 0.0, y = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < nblk; b += 32) {
+        const double2 v = __ldcg(work + (int64_t)b * nout + o);
+        x += v.x;
+        y += v.y;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        x += __shfl_down_sync(0xffffffffu, x, off);
+        y += __shfl_down_sync(0xffffffffu, y, off);
+    }
+    if (lane == 0) out[o % nl + (int64_t)ldo * (o / nl)] = make_double2(x, y);
+}
+
+// RT rows a stage.  Warp w: tile
+// w % (tl tr), row group w / (tl tr).
+template <class S, int RT>
+__global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_constant__ GramTileArgs<S> a)
+{
+    extern __shared__ __align__(16) unsigned char gt_smem[];
+    S *ring = reinterpret_cast<S *>(gt_smem);  // [stage][slot][RT]
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nt = blockDim.x;
+    const int tiles = a.tl * a.tr, tile = warp % tiles, group = warp / tiles, groups = (nt >> 5) / tiles;
+    const int i0 = tile % a.tl * kTile, j0 = tile / a.tl * kTile;
+    int ls[kTile], rs[kTile];
+#pragma unroll
+    for (int i = 0; i < kTile; ++i) {
+        ls[i] = a.lslot[i0 + i] * RT;
+        rs[i] = a.rslot[j0 + i] * RT;
+    }
+    const int64_t ntiles = (a.len + RT - 1) / RT;
+    const int elems = a.nslots * RT, stride = elems;
+    auto issue = [&](int64_t tl, int st) {
+        if (tl < ntiles) {
+            const int64_t r0 = tl * RT;
+            for (int e = t; e < elems; e += nt) {
+                const int s = e / RT, r = e % RT;
+                const bool in = r0 + r < a.len;
+                copy_async<S>(ring + st * stride + e, a.col[s] + (in ? r0 + r : 0), in);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    double gr[kTile][kTile], gi[kTile][kTile];
+#pragma unroll
+    for (int i = 0; i < kTile; ++i)
+#pragma unroll
+        for (int j = 0; j < kTile; ++j) gr[i][j] = gi[i][j] = 0.0;
+    const int ns = a.stages;
+    for (int k = 0; k + 1 < ns; ++k) issue(blockIdx.x + (int64_t)k * gridDim.x, k);
+    int st = 0;
+    for (int64_t tl = blockIdx.x; tl < ntiles; tl += gridDim.x, st = st + 1 == ns ? 0 : st + 1) {
+        if (ns == 4) asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+        else if (ns == 3) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        S *xs = ring + st * stride;
+        // the slot freed by the previous step takes the copies ns - 1 ahead
+        issue(tl + (int64_t)(ns - 1) * gridDim.x, st == 0 ? ns - 1 : st - 1);
+        if (a.nshift) {  // a <- a - sigma b; partners are never shifted themselves
+            for (int e = t; e < a.nshift * RT; e += nt) {
+                const int k = e / RT, r = e % RT;
+                S *xa = xs + a.shifted[k] * RT + r;
+                const S av = *xa, bv = xs[a.partner[k] * RT + r];
+                S v;
+                v.x = av.x - (a.sigma.x * bv.x - a.sigma.y * bv.y);
+                v.y = av.y - (a.sigma.x * bv.y + a.sigma.y * bv.x);
+                *xa = v;
+            }
+            __syncthreads();
+        }
+        for (int r = group * 32 + lane; r < RT; r += groups * 32) {
+            double2 l[kTile], x[kTile];
+#pragma unroll
+            for (int i = 0; i < kTile; ++i) {
+                const S lv = xs[ls[i] + r], xv = xs[rs[i] + r];
+                l[i] = make_double2(lv.x, a.sign * lv.y);
+                x[i] = make_double2(xv.x, xv.y);
+            }
+#pragma unroll
+            for (int i = 0; i < kTile; ++i)
+#pragma unroll
+                for (int j = 0; j < kTile; ++j) {
+                    gr[i][j] = fma(l[i].x, x[j].x, gr[i][j]);
+                    gr[i][j] = fma(-l[i].y, x[j].y, gr[i][j]);
+                    gi[i][j] = fma(l[i].x, x[j].y, gi[i][j]);
+                    gi[i][j] = fma(l[i].y, x[j].x, gi[i][j]);
+                }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    // lanes, then row groups, then one partial per CTA; the last CTA or
+    // gram_reduce adds the partials in a fixed order
+    double2 *acc = reinterpret_cast<double2 *>(gt_smem);  // [warp][16]
+#pragma unroll
+    for (int i = 0; i < kTile; ++i)
+#pragma unroll
+        for (int j = 0; j < kTile; ++j) {
+            double x = gr[i][j], y = gi[i][j];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                x += __shfl_down_sync(0xffffffffu, x, off);
+                y += __shfl_down_sync(0xffffffffu, y, off);
+            }
+            if (lane == 0) acc[warp * 16 + i * kTile + j] = make_double2(x, y);
+        }
+    __syncthreads();
+    const int nout = a.nl * a.nr;
+    double2 *part = a.work + 1 + (int64_t)blockIdx.x * nout;
+    for (int o = t; o < nout; o += nt) {
+        const int i = o % a.nl, j = o / a.nl;
+        const int w = i / kTile + a.tl * (j / kTile), k = (i % kTile) * kTile + j % kTile;
+        double x = 0.0, y = 0.0;
+        for (int g = 0; g < groups; ++g) {
+            x += acc[(g * tiles + w) * 16 + k].x;
+            y += acc[(g * tiles + w) * 16 + k].y;
+        }
+        part[o] = make_double2(x, y);
+    }
+    if (nout > kFusedOut) return;  // gram_tile_reduce follows
+    __shared__ bool last;
+    unsigned *ticket = reinterpret_cast<unsigned *>(a.work);
+    __threadfence();
+    __syncthreads();
+    if (t == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int o = warp; o < nout; o += nt >> 5) sum_partials(a.work + 1, gridDim.x, a.nl, nout, o, lane, a.out, a.ldo);
+    if (t == 0) *ticket = 0u;
+}
+
+// Sum of the nblk partials, a warp per output.
+__global__ void __launch_bounds__(256)
+    gram_tile_reduce(const double2 *__restrict__ work, int nblk, int nl, int nr, double2 *__restrict__ out, int ldo)
+{
+    const int o = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (o < nl * nr) sum_partials(work, nblk, nl, nl * nr, o, threadIdx.x & 31, out, ldo);
+}
+
+template <class S, int RT>
+cudaError_t tile_launch(const GramTileArgs<S> &a, int threads, size_t smem, cudaStream_t st)
+{
+    static std::atomic<int> sms[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    int n = sms[dev].load(std::memory_order_relaxed);
+    if (!n) {
+        cudaError_t e = cudaFuncSetAttribute(gram_tile_kernel<S, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+        if (e != cudaSuccess) return e;
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 148;
+        sms[dev].store(n, std::memory_order_relaxed);
+    }
+    // two CTAs per SM: 112 KB of shared memory and 128 registers a thread
+    const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((a.len + RT - 1) / RT, std::min(2 * n, 296)));
+    gram_tile_kernel<S, RT><<<nblk, threads, smem, st>>>(a);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || a.nl * a.nr <= kFusedOut) return e;
+    gram_tile_reduce<<<(a.nl * a.nr + 7) / 8, 256, 0, st>>>(a.work + 1, nblk, a.nl, a.nr, a.out, a.ldo);
+    count_launch();
+    return cudaGetLastError();
+}
+
+// One launch: L columns [l0, l0 + nl) against R columns [r0, r0 + nr), at
+// most kWarps tiles.
+template <class S>
+cudaError_t tile_go(const ColListT<S> &L, const ColListT<S> &R, int l0, int nl, int r0, int nr, int64_t len, int herm,
+                    double2 *out, int ldo, double2 *work, cudaStream_t st)
+{
+    GramTileArgs<S> a{};
+    a.sigma = L.sigma;
+    // slot of the column x - sigma y (y null: x)
+    const S *bs[kMaxSlots];
+    auto find = [&](const S *x, const S *y) {
+        for (int s = 0; s < a.nslots; ++s)
+            if (a.col[s] == x && bs[s] == y) return s;
+        const int s = a.nslots++;
+        a.col[s] = x;
+        bs[s] = y;
+        return s;
+    };
+    for (int i = 0; i < nl; ++i) a.lslot[i] = (unsigned char)find(L.a[l0 + i], L.b[l0 + i]);
+    for (int j = 0; j < nr; ++j) a.rslot[j] = (unsigned char)find(R.a[r0 + j], R.b[r0 + j]);
+    for (int s = 0, n = a.nslots; s < n; ++s)
+        if (bs[s]) {
+            a.shifted[a.nshift] = (unsigned char)s;
+            a.partner[a.nshift++] = (unsigned char)find(bs[s], nullptr);
+        }
+    a.tl = (nl + kTile - 1) / kTile;
+    a.tr = (nr + kTile - 1) / kTile;
+    for (int i = nl; i < a.tl * kTile; ++i) a.lslot[i] = a.lslot[0];  // padding, dropped
+    for (int j = nr; j < a.tr * kTile; ++j) a.rslot[j] = a.rslot[0];
+    a.len = len;
+    a.nl = nl;
+    a.nr = nr;
+    a.sign = herm ? -1.0 : 1.0;
+    a.work = work;
+    a.out = out + l0 + (int64_t)ldo * r0;
+    a.ldo = ldo;
+    const int tiles = a.tl * a.tr, groups = kWarps / tiles, threads = 32 * tiles * groups;
+    const int rt = groups >= 8 ? 256 : groups >= 4 ? 128 : 64;
+    const size_t stage = (size_t)a.nslots * rt * sizeof(S);
+    a.stages = (int)std::max<size_t>(2, std::min<size_t>(4, 111 * 1024 / stage));
+    const size_t smem = std::max<size_t>(stage * a.stages, kWarps * 16 * sizeof(double2));
+    if (rt == 256) return tile_launch<S, 256>(a, threads, smem, st);
+    if (rt == 128) return tile_launch<S, 128>(a, threads, smem, st);
+    return tile_launch<S, 64>(a, threads, smem, st);
+}
+
+template <class S>
+cudaError_t tiles_go(const ColListT<S> &L, const ColListT<S> &R, int64_t len, int herm, double2 *out, int ldo,
+                     double2 *work, cudaStream_t st)
+{
+    if (!gram_tile_supported(L.n, R.n)) return cudaErrorInvalidValue;
+    const int tl = (L.n + kTile - 1) / kTile, tr = (R.n + kTile - 1) / kTile;
+    // blocks of at most kWarps tiles; the side with fewer tiles stays whole
+    const int bl = tr <= tl ? std::max(1, kWarps / tr) : tl, br = tr <= tl ? tr : std::max(1, kWarps / tl);
+    for (int i = 0; i < L.n; i += bl * kTile)
+        for (int j = 0; j < R.n; j += br * kTile) {
+            cudaError_t e = tile_go(L, R, i, std::min(bl * kTile, L.n - i), j, std::min(br * kTile, R.n - j), len, herm,
+                                    out, ldo, work, st);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
+}  // namespace
+
+// More tiles re-read the columns of the other side too often: those go to the
+// FP64 tensor cores (gram_tc).
+bool gram_tile_supported(int nl, int nr)
+{
+    const int tl = (nl + kTile - 1) / kTile, tr = (nr + kTile - 1) / kTile;
+    return std::min(tl, tr) <= kWarps && tl * tr <= 32;
+}
+
+cudaError_t gram_tile_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out, int ldo,
+                             double2 *work, cudaStream_t st)
+{
+    return tiles_go(L, R, len, herm, out, ldo, work, st);
+}
+
+cudaError_t gram_tile_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,
+                             double2 *work, cudaStream_t st)
+{
+    return tiles_go(L, R, len, herm, out, ldo, work, st);
+}
+
+}  // namespace de
