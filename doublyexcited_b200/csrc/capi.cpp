@@ -293,15 +293,18 @@ int de_problem::prof_end(Rec &r)
     return DE_OK;
 }
 
-int de_problem::matblock32(const float2 *x, float2 *y, int nvec, double2 shift)
+int de_problem::matblock32(const float2 *x, float2 *y, int nvec, double2 shift, double exch)
 {
     if (p.nelec != 2) return set_error(DE_E_INVALID, "the FP32 matvec is built for the two-electron operator");
+    if (ham.fam[1][0] != DE_MATVEC_FMA || ham.fam[1][1] != DE_MATVEC_FMA) exch = 0.0;
     Rec r{{nullptr, nullptr, nullptr}, nvec, 1};
     DE_TRY(prof_begin(r));
-    cudaError_t e = hammult_pass_launch(ham, x, y, nvec, dim, 0, stream, shift);
+    cudaError_t e = exch != 0.0 ? hammult_exch_pass_launch(ham, x, y, nvec, dim, 0, exch, stream, shift)
+                                : hammult_pass_launch(ham, x, y, nvec, dim, 0, stream, shift);
     if (e != cudaSuccess) return cuda_error(e, "hammult FP32 pass A");
     DE_TRY(prof_mid(r));
-    e = hammult_pass_launch(ham, x, y, nvec, dim, 1, stream);
+    e = exch != 0.0 ? hammult_exch_pass_launch(ham, x, y, nvec, dim, 1, exch, stream, shift)
+                    : hammult_pass_launch(ham, x, y, nvec, dim, 1, stream);
     if (e != cudaSuccess) return cuda_error(e, "hammult FP32 pass B");
     return prof_end(r);
 }

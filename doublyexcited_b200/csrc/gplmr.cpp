@@ -76,6 +76,7 @@ struct Solver {
     float2 *Z32 = nullptr;  // mixed inner solve: the power basis Z_0..Z_order (complex64)
     bool mixed = false;
     double exch_sign = 0.0;     // +1 / -1: exchange symmetry of the start block, 0: none
+    double exch_mult = 0.0;     // the same where the start holds it to rounding: the inner products use it
     unsigned refl_keep = 0xFFu;  // reflection sectors the start block reaches (bit c: sector c)
     bool exch_done = false;      // the last inner solve's output is already exchange-projected
     bool z0_staged = false;      // the next inner solve's complex64 start Z_0 is already in Z32
@@ -538,7 +539,7 @@ struct Solver {
             mv_exec += k;
             mv_ref += k;
             const cplx ms = -sigma;
-            return h->matblock32(x, y, k, make_double2(ms.real(), ms.imag()));
+            return h->matblock32(x, y, k, make_double2(ms.real(), ms.imag()), exch_mult);
         }
     }
 
@@ -1008,7 +1009,7 @@ struct Solver {
     // projection off.
     int detect_symmetry()
     {
-        double sign = 0.0;
+        double sign = 0.0, worst = 0.0;  // worst: largest | |<x, x^T>| - 1 |
         for (int j = 0; j < nev; ++j) {
             cudaError_t e = exch_dot_launch(col(X, j), h->m, dR + j, h->d_work, st);
             if (e != cudaSuccess) return cuda_error(e, "exch_dot");
@@ -1024,6 +1025,7 @@ struct Solver {
             const double sj = std::fabs(r - 1.0) < 1e-8 ? 1.0 : std::fabs(r + 1.0) < 1e-8 ? -1.0 : 0.0;
             if (j == 0) sign = sj;
             else if (sj != sign) sign = 0.0;
+            worst = std::max(worst, std::fabs(std::fabs(r) - 1.0));
             const double2 *corr = hbuf + nev + 8 * j;  // <x, R_r x>, r = 0..7; r = 0 is |x|^2
             for (int c = 0; c < 8; ++c) {
                 double n2 = 0.0;
@@ -1032,6 +1034,10 @@ struct Solver {
             }
         }
         exch_sign = sign;
+        // a part of squared norm worst / 2 is outside the sector; below
+        // complex64 rounding (6e-8 squared, with the reduction's own rounding
+        // allowed for) the inner products may take X^T = sign X for granted
+        exch_mult = worst < 2e-14 ? sign : 0.0;
         refl_keep = keep;
         return DE_OK;
     }

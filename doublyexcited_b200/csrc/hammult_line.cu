@@ -410,9 +410,10 @@ __global__ void __launch_bounds__(Cfg<R, NN>::KT, Cfg<R, NN>::KB) kline_kernel(c
     }
 }
 
-// Y += S2 (T_i1 + T_j1 + T_k1) X on one column X(:, q): k lines straight from
-// global memory (lanes along i, j), the i and j lines through shared memory.
-template <class R, int NN>
+// Y += S2 (T_i1 + T_j1 + T_k1) X (ADD; else Y = ...) on one column X(:, q): k
+// lines straight from global memory (lanes along i, j), the i and j lines
+// through shared memory.
+template <class R, int NN, bool ADD>
 __global__ void __launch_bounds__(Cfg<R, NN>::CT, Cfg<R, NN>::CB) cube_line_kernel(const __grid_constant__ LineArgs<R> a)
 {
     using K = Cfg<R, NN>;
@@ -470,22 +471,100 @@ __global__ void __launch_bounds__(Cfg<R, NN>::CT, Cfg<R, NN>::CB) cube_line_kern
                 };
 #pragma unroll
                 for (int j = 0; j < NN; ++j) v[j] = xl[NN * j];
-                line_transform<R, NN, sizeof(R) == 8 ? 2 : 0, ORDER>(
+                line_transform<R, NN, ADD && sizeof(R) == 8 ? 2 : 0, ORDER>(
                     v,
                     [&](int j) {
                         L r;
                         r.s = yl[NN * j];
-                        if constexpr (sizeof(R) == 8) r.y = g[NN * j];
+                        if constexpr (ADD && sizeof(R) == 8) r.y = g[NN * j];
                         return r;
                     },
                     [&](int j, CC<R> z, L r) {
                         R yr, yi;
                         times_s2(a, X::add(r.s, z), yr, yi);
-                        if constexpr (sizeof(R) == 8) g[NN * j] = X::make(r.y.x + yr, r.y.y + yi);
+                        if constexpr (!ADD) g[NN * j] = X::make(yr, yi);
+                        else if constexpr (sizeof(R) == 8) g[NN * j] = X::make(r.y.x + yr, r.y.y + yi);
                         else add_to(g + NN * j, yr, yi);
                     });
             }
             if (G < NN || more) __syncthreads();
+        }
+    }
+}
+
+// Electron exchange: for X^T = s X (s = 1 or -1) the electron-2 axes need no
+// pass of their own, T_2 X = s (T_1 X)^T, so from Z = T_1 X in Y
+//   Y <- Z + s Z^T + (V + shift) X
+// in place on pairs of 32 x 32 tiles (bi <= bj).  V is symmetric, so the
+// partner tile is s times the transpose: only the upper half of X is read,
+// and Y is exactly (anti)symmetric.  Complex64, memory-bound: 2.5 vector
+// passes after the cube kernel's 2, against 8 for the general product.
+// Inside the mixed solve at NN = 13 the two take 44 us a product against 59.
+// 512 threads with two elements each and three CTAs per SM, measured there (ms
+// per outer iteration of 30 products): 5.18; four CTAs 5.39, two 5.26; 256
+// threads 5.18 at four CTAs, 5.26 at three; 128 threads 5.38.
+constexpr int kExchThreads = 512;
+__global__ void __launch_bounds__(kExchThreads, 3)
+    exch_add_kernel(const __grid_constant__ LineArgs<float> a, int nn, float s)
+{
+    constexpr int RY = kExchThreads / 32, E = 32 / RY;
+    __shared__ float2 ta[32][33], tb[32][33];
+    __shared__ int bp[32], bq[32];
+    const int m = nn * nn * nn, w = 2 * nn - 1;
+    // the tile pair: blocks enumerate bi <= bj
+    int bj = (int)((sqrtf(8.0f * blockIdx.x + 1.0f) - 1.0f) * 0.5f);
+    while ((bj + 1) * (bj + 2) / 2 <= (int)blockIdx.x) ++bj;
+    while (bj * (bj + 1) / 2 > (int)blockIdx.x) --bj;
+    const int bi = (int)blockIdx.x - bj * (bj + 1) / 2;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int p0 = bi * 32, q0 = bj * 32;
+    if (threadIdx.x < 64) {  // TINV(r_q - r_p) sits at bq - bp of the table
+        const int r = min((threadIdx.x < 32 ? p0 : q0) + tx, m - 1);
+        const int b = r % nn + w * ((r / nn) % nn + w * (r / (nn * nn)));
+        if (threadIdx.x < 32) bp[tx] = b;
+        else bq[tx] = b + (nn - 1) * (1 + w + w * w);
+    }
+    __syncthreads();
+    const int p = p0 + tx, pt = q0 + tx;
+    const float tp = __ldg(a.t1a + min(p, m - 1));
+    grid_wait();
+    grid_release();
+    for (int vec = blockIdx.y; vec < a.nvec; vec += gridDim.y) {
+        const float2 *x = reinterpret_cast<const float2 *>(a.x) + vec * a.vstride;
+        float2 *y = reinterpret_cast<float2 *>(a.y) + vec * a.vstride;
+        float2 za[E], zb[E], xa[E];
+        float v[E];
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const int c = ty + RY * u;
+            const bool oka = p < m && q0 + c < m, okb = pt < m && p0 + c < m;
+            zb[u] = okb ? y[pt + (int64_t)m * (p0 + c)] : make_float2(0.f, 0.f);
+            za[u] = oka ? y[p + (int64_t)m * (q0 + c)] : make_float2(0.f, 0.f);
+            xa[u] = oka ? __ldg(x + p + (int64_t)m * (q0 + c)) : make_float2(0.f, 0.f);
+            v[u] = (__ldg(a.t1a + min(q0 + c, m - 1)) + tp) + __ldg(a.v12 + bq[c] - bp[tx]);
+        }
+#pragma unroll
+        for (int u = 0; u < E; ++u) tb[tx][ty + RY * u] = zb[u];  // tb[r][c] = Z(q0 + r, p0 + c)
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const int c = ty + RY * u, q = q0 + c;
+            const float pr = fmaf(v[u], a.vsr, a.shr), pi = fmaf(v[u], a.vsi, a.shi);
+            const float2 zt = tb[c][tx];
+            float yr = za[u].x + s * zt.x, yi = za[u].y + s * zt.y;
+            yr += pr * xa[u].x - pi * xa[u].y;
+            yi += pr * xa[u].y + pi * xa[u].x;
+            ta[tx][c] = make_float2(yr, yi);  // ta[r][c] = Y(p0 + r, q0 + c)
+            if (p < m && q < m) y[p + (int64_t)m * q] = make_float2(yr, yi);
+        }
+        __syncthreads();
+        if (bi != bj) {
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                const int c = ty + RY * u;
+                const float2 t = ta[c][tx];  // Y(p0 + c, q0 + tx)
+                if (pt < m && p0 + c < m) y[pt + (int64_t)m * (p0 + c)] = make_float2(s * t.x, s * t.y);
+            }
         }
     }
 }
@@ -523,7 +602,13 @@ cudaError_t prepare()
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kline_kernel<R, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::KSMEM);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(cube_line_kernel<R, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::CSMEM);
+        e = cudaFuncSetAttribute(cube_line_kernel<R, NN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)K::CSMEM);
+    if constexpr (sizeof(R) == 4) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(cube_line_kernel<R, NN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)K::CSMEM);
+    }
     if (e == cudaSuccess) done[dev].store(true, std::memory_order_release);
     return e;
 }
@@ -540,12 +625,14 @@ cudaError_t pass(const LineArgs<R> &a, int which, cudaStream_t st)
         if (e != cudaSuccess) return e;
         return launch<R>(kline_kernel<R, NN>, dim3((K::M * K::P2 + K::KT - 1) / K::KT, ny), K::KT, K::KSMEM, a, st);
     }
-    const int64_t units = std::min<int64_t>((int64_t)K::M * a.nvec, 0x7fffffff);
-    return launch<R>(cube_line_kernel<R, NN>, dim3((unsigned)units), K::CT, K::CSMEM, a, st);
+    const unsigned units = (unsigned)std::min<int64_t>((int64_t)K::M * a.nvec, 0x7fffffff);
+    if (which == 1) return launch<R>(cube_line_kernel<R, NN, true>, dim3(units), K::CT, K::CSMEM, a, st);
+    if constexpr (sizeof(R) == 4) return launch<R>(cube_line_kernel<R, NN, false>, dim3(units), K::CT, K::CSMEM, a, st);
+    else return cudaErrorInvalidValue;
 }
 
 template <class R, class G>
-cudaError_t go(const HamDev &h, const G *x, G *y, int nvec, int64_t vstride, int which, cudaStream_t st, double2 shift)
+LineArgs<R> line_args(const HamDev &h, const G *x, G *y, int nvec, int64_t vstride, double2 shift)
 {
     LineArgs<R> a{};
     a.x = reinterpret_cast<const CC<R> *>(x);
@@ -565,6 +652,12 @@ cudaError_t go(const HamDev &h, const G *x, G *y, int nvec, int64_t vstride, int
     a.vsi = (R)h.vsim;
     a.shr = (R)shift.x;
     a.shi = (R)shift.y;
+    return a;
+}
+
+template <class R>
+cudaError_t go(const HamDev &h, const LineArgs<R> &a, int which, cudaStream_t st)
+{
     switch (h.nn) {
     case 3: return pass<R, 3>(a, which, st);
     case 5: return pass<R, 5>(a, which, st);
@@ -586,13 +679,34 @@ cudaError_t go(const HamDev &h, const G *x, G *y, int nvec, int64_t vstride, int
 cudaError_t hammult_line_pass_launch(const HamDev &h, const double2 *x, double2 *y, int nvec, int64_t vstride,
                                      int pass, cudaStream_t st, double2 shift)
 {
-    return go<double>(h, x, y, nvec, vstride, pass, st, shift);
+    return go<double>(h, line_args<double>(h, x, y, nvec, vstride, shift), pass, st);
 }
 
 cudaError_t hammult_line_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride,
                                      int pass, cudaStream_t st, double2 shift)
 {
-    return go<float>(h, x, y, nvec, vstride, pass, st, shift);
+    return go<float>(h, line_args<float>(h, x, y, nvec, vstride, shift), pass, st);
+}
+
+cudaError_t hammult_exch_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride, int pass,
+                                     double sign, cudaStream_t st, double2 shift)
+{
+    if (h.nelec != 2 || nvec <= 0 || !h.t1af || !h.v12f) return cudaErrorInvalidValue;
+    const LineArgs<float> a = line_args<float>(h, x, y, nvec, vstride, shift);
+    if (pass == 0) return go<float>(h, a, 2, st);
+    const int tiles = (int)((h.m + 31) / 32);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(tiles * (tiles + 1) / 2), (unsigned)std::min(nvec, 65535));
+    cfg.blockDim = dim3(kExchThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = programmatic_launch() ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, exch_add_kernel, a, h.nn, (float)sign);
+    count_launch();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace de
