@@ -159,7 +159,9 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < len; r += stride) {
+    // from the last row to the first: an update follows the Gram that read the
+    // same columns from first to last, and finds its last rows in L2
+    for (int64_t r = len - 1 - ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); r >= 0; r -= stride) {
         T ar[NOUT], ai[NOUT];
         double2 yb[NOUT];
 #pragma unroll
@@ -204,6 +206,52 @@ __global__ void __launch_bounds__(256)
             const double2 sj = cmul(U.alpha, make_double2((double)ar[j], (double)ai[j]));
             if (j < nout) U.y[j][r] = st2<SO>(yb[j].x + sj.x, yb[j].y + sj.y);
         }
+    }
+}
+
+// Y = alpha sum_i X_i c_i of NC columns (one output, nothing kept of Y): the
+// loads of two rows in flight before the sums.  HBM-bound; us at 4.8 M rows,
+// update_kernel -> here (HBM time): 3 columns 64 -> 50 (47), 5 88 -> 76 (71),
+// 7 113 -> 94 (94), 8 152 -> 105 (106).
+template <int NC>
+__global__ void __launch_bounds__(256, 3)
+    update_col(const __grid_constant__ UpdListT<double2, double2> U, const double2 *__restrict__ C, int64_t len)
+{
+    __shared__ double2 cs[NC];
+    if (threadIdx.x < NC) cs[threadIdx.x] = cmul(U.alpha, C[threadIdx.x]);
+    __syncthreads();
+    const double2 *x[NC];
+    double2 c[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+        x[i] = U.x[i];
+        c[i] = cs[i];
+    }
+    double2 *y = U.y[0];
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    // from the last row to the first, as update_kernel
+    for (int64_t r = len - 1 - ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); r >= 0; r -= 2 * stride) {
+        const int64_t r1 = r - stride;
+        double2 v0[NC], v1[NC];
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            v0[i] = ldp(x[i] + r);
+            v1[i] = r1 >= 0 ? ldp(x[i] + r1) : make_double2(0.0, 0.0);
+        }
+        double2 s0 = make_double2(0.0, 0.0), s1 = s0;
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            s0.x = fma(v0[i].x, c[i].x, s0.x);
+            s0.x = fma(-v0[i].y, c[i].y, s0.x);
+            s0.y = fma(v0[i].x, c[i].y, s0.y);
+            s0.y = fma(v0[i].y, c[i].x, s0.y);
+            s1.x = fma(v1[i].x, c[i].x, s1.x);
+            s1.x = fma(-v1[i].y, c[i].y, s1.x);
+            s1.y = fma(v1[i].x, c[i].y, s1.y);
+            s1.y = fma(v1[i].y, c[i].x, s1.y);
+        }
+        y[r] = s0;
+        if (r1 >= 0) y[r1] = s1;
     }
 }
 
@@ -535,6 +583,59 @@ __global__ void __launch_bounds__(256)
             const int i = o / nr, j = o % nr;
             out[i + (int64_t)ldo * j] = res[i * NRM + j];
         }
+        if (threadIdx.x == 0) *ticket = 0u;
+    }
+}
+
+// NC columns against one: all of a row pair's loads in flight before the sums
+// (gram_small checks each column's presence in between).  SELF: the one is
+// the last of the NC, as in orthogonalise-and-normalise, and is read once.
+// HBM-bound; inside the mixed solve at 4.8 M rows, us before -> now (HBM time):
+// 3-4 columns 79 -> 44-56 (35-47), 5-8 columns 133 -> 70-108 (59-94).
+template <int NC, bool SELF>
+__global__ void __launch_bounds__(256, 2)
+    gram_col(const __grid_constant__ ColListT<double2> L, const double2 *__restrict__ b, int64_t len, int herm,
+             double2 *__restrict__ work, double2 *__restrict__ out)
+{
+    constexpr int U = 2;
+    const double2 *col[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) col[i] = L.a[i];
+    double ar[NC], ai[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) ar[i] = ai[i] = 0.0;
+    const double sg = herm ? -1.0 : 1.0;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < len; r += U * stride) {
+        double2 l[U][NC], x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t ru = r + u * stride;
+            const bool in = ru < len;
+#pragma unroll
+            for (int i = 0; i < NC; ++i) l[u][i] = in ? __ldg(col[i] + ru) : make_double2(0.0, 0.0);
+            if constexpr (!SELF) x[u] = in ? __ldg(b + ru) : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if constexpr (SELF) x[u] = l[u][NC - 1];
+#pragma unroll
+            for (int i = 0; i < NC; ++i) {
+                const double ly = sg * l[u][i].y;
+                ar[i] = fma(l[u][i].x, x[u].x, ar[i]);
+                ar[i] = fma(-ly, x[u].y, ar[i]);
+                ai[i] = fma(l[u][i].x, x[u].y, ai[i]);
+                ai[i] = fma(ly, x[u].x, ai[i]);
+            }
+        }
+    }
+    unsigned *ticket = reinterpret_cast<unsigned *>(work);
+    double2 *part = work + 1;
+    block_sum<NC>(ar, ai, part + (int64_t)blockIdx.x * NC, NC);
+    if (last_block(ticket, gridDim.x)) {
+        __shared__ double2 res[32];
+        reduce_partials(part, gridDim.x, NC, NC, res);
+        if (threadIdx.x < NC) out[threadIdx.x] = res[threadIdx.x];
         if (threadIdx.x == 0) *ticket = 0u;
     }
 }
@@ -1351,11 +1452,46 @@ static cudaError_t gram_tc_go(const ColListT<S> &L, const ColListT<S> &R, int64_
     return cudaGetLastError();
 }
 
+template <int NC, bool SELF>
+static cudaError_t gram_col_go(const ColList &L, const double2 *b, int64_t len, int herm, double2 *out, double2 *work,
+                               cudaStream_t st)
+{
+    const int blocks = fused_blocks<gram_col<NC, SELF>>((len + 1) / 2, NC);
+    gram_col<NC, SELF><<<blocks, 256, 0, st>>>(L, b, len, herm, work, out);
+    count_launch();
+    return cudaGetLastError();
+}
+
+// L unshifted, 2 <= L.n <= 9, one unshifted column in R
+template <bool SELF>
+static cudaError_t gram_col_any(const ColList &L, const double2 *b, int64_t len, int herm, double2 *out, double2 *work,
+                                cudaStream_t st)
+{
+    switch (L.n) {
+    case 2: return gram_col_go<2, SELF>(L, b, len, herm, out, work, st);
+    case 3: return gram_col_go<3, SELF>(L, b, len, herm, out, work, st);
+    case 4: return gram_col_go<4, SELF>(L, b, len, herm, out, work, st);
+    case 5: return gram_col_go<5, SELF>(L, b, len, herm, out, work, st);
+    case 6: return gram_col_go<6, SELF>(L, b, len, herm, out, work, st);
+    case 7: return gram_col_go<7, SELF>(L, b, len, herm, out, work, st);
+    case 8: return gram_col_go<8, SELF>(L, b, len, herm, out, work, st);
+    case 9: return gram_col_go<9, SELF>(L, b, len, herm, out, work, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
 template <class S>
 static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t len, int herm, double2 *out, int ldo,
                             double2 *work, cudaStream_t st)
 {
     if (L.n < 1 || L.n > 64 || R.n < 1 || R.n > 128 || len < 1) return cudaErrorInvalidValue;
+    if constexpr (sizeof(S) == 16) {
+        bool plain = R.n == 1 && L.n >= 2 && L.n <= 9 && !R.b[0];
+        for (int i = 0; i < L.n && plain; ++i) plain = !L.b[i];
+        if (plain)
+            return L.a[L.n - 1] == R.a[0] ? gram_col_any<true>(L, R.a[0], len, herm, out, work, st)
+                                          : gram_col_any<false>(L, R.a[0], len, herm, out, work, st);
+    }
     if (R.n == 1 && L.n <= 32) {
         if (L.n <= 1) return gram_small_go<1, 1>(L, R, len, herm, out, ldo, work, st);
         if (L.n <= 2) return gram_small_go<2, 1>(L, R, len, herm, out, ldo, work, st);
@@ -1550,11 +1686,34 @@ cudaError_t gram_herm_launch(const ColListF &Z, int64_t len, double2 *out, int l
     }
 }
 
+template <int NC>
+static cudaError_t update_col_go(const UpdList &U, const double2 *c_dev, int64_t len, cudaStream_t st)
+{
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((len + 511) / 512, wave_blocks<update_col<NC>>()));
+    update_col<NC><<<blocks, 256, 0, st>>>(U, c_dev, len);
+    count_launch();
+    return cudaGetLastError();
+}
+
 template <class SI, class SO>
 static cudaError_t update_any(const UpdListT<SI, SO> &U, const double2 *c_dev, int ldc, int64_t len, cudaStream_t st)
 {
     if (U.nin < 1 || U.nin > kMaxCols || U.nout < 1 || U.nout > 16 || len < 1)
         return cudaErrorInvalidValue;
+    if constexpr (sizeof(SI) == 16 && sizeof(SO) == 16) {
+        if (U.nout == 1 && U.nin >= 2 && U.nin <= 9 && U.beta[0].x == 0.0 && U.beta[0].y == 0.0) {
+            switch (U.nin) {
+            case 2: return update_col_go<2>(U, c_dev, len, st);
+            case 3: return update_col_go<3>(U, c_dev, len, st);
+            case 4: return update_col_go<4>(U, c_dev, len, st);
+            case 5: return update_col_go<5>(U, c_dev, len, st);
+            case 6: return update_col_go<6>(U, c_dev, len, st);
+            case 7: return update_col_go<7>(U, c_dev, len, st);
+            case 8: return update_col_go<8>(U, c_dev, len, st);
+            default: return update_col_go<9>(U, c_dev, len, st);
+            }
+        }
+    }
     if (U.nout <= 1) return update_go<1>(U, c_dev, ldc, len, st);
     if (U.nout <= 2) return update_go<2>(U, c_dev, ldc, len, st);
     if (U.nout <= 4) return update_go<4>(U, c_dev, ldc, len, st);

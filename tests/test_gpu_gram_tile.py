@@ -40,3 +40,24 @@ def test_dots_tiles(de, size, nbra, nket, herm):
         same = dots(bras, bras, m, m)
         want = (bras[:m] @ (bras[:m].conj() if herm else bras[:m]).T).cpu().numpy()
         assert np.abs(same - want).max() < tol
+
+
+@pytest.mark.parametrize("size", [1, 255, 257, 513, 300007])
+@pytest.mark.parametrize("nbra", [2, 3, 5, 8, 9, 10])
+def test_dots_one_ket(de, size, nbra):
+    """One ket against 2..9 bras (their own kernel, the ket being the last bra
+    or not) and 10 (the general one)."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(size + nbra)
+    both = torch.randn(nbra + 1, size, dtype=torch.complex128, device="cuda", generator=gen)
+    L = de.lib()
+    with de.Problem(n=1, delta=2.0, theta=0.3) as g:
+        g.set_stream(torch.cuda.current_stream().cuda_stream)
+        for herm in (0, 1):
+            for ket in (both[nbra], both[nbra - 1]):
+                out = np.full(nbra, np.nan, np.complex128)
+                assert L.de_dots_d(g.handle, ctypes.c_void_p(both.data_ptr()), ctypes.c_void_p(ket.data_ptr()), size,
+                                   nbra, 1, ctypes.c_void_p(out.ctypes.data), herm) == de.DE_OK
+                want = ((both[:nbra].conj() if herm else both[:nbra]) @ ket).cpu().numpy()
+                assert np.abs(out - want).max() < 1e-15 * (size + 100)
