@@ -251,19 +251,22 @@ int de_problem::harvest()
     return DE_OK;
 }
 
-int de_problem::matblock(const double2 *x, double2 *y, int nvec, double2 shift)
+int de_problem::matblock(const double2 *x, double2 *y, int nvec, double2 shift, double exch)
 {
     if (p.nelec != 2) {
         cudaError_t e = hammult1_launch(ham, d_t1a, x, y, nvec, dim, stream);
         if (e != cudaSuccess) return cuda_error(e, "hammult1");
         return DE_OK;
     }
+    if (ham.fam[0][0] != DE_MATVEC_FMA || ham.fam[0][1] != DE_MATVEC_FMA) exch = 0.0;
     Rec r{{nullptr, nullptr, nullptr}, nvec, 0};
     DE_TRY(prof_begin(r));
-    cudaError_t e = hammult_pass_launch(ham, x, y, nvec, dim, 0, stream, shift);
+    cudaError_t e = exch != 0.0 ? hammult_exch_pass_launch(ham, x, y, nvec, dim, 0, exch, stream, shift)
+                                : hammult_pass_launch(ham, x, y, nvec, dim, 0, stream, shift);
     if (e != cudaSuccess) return cuda_error(e, "hammult pass A");
     DE_TRY(prof_mid(r));
-    e = hammult_pass_launch(ham, x, y, nvec, dim, 1, stream);
+    e = exch != 0.0 ? hammult_exch_pass_launch(ham, x, y, nvec, dim, 1, exch, stream, shift)
+                    : hammult_pass_launch(ham, x, y, nvec, dim, 1, stream);
     if (e != cudaSuccess) return cuda_error(e, "hammult pass B");
     return prof_end(r);
 }

@@ -119,11 +119,11 @@ struct de_problem {
 
     int ensure_stage(int64_t elems);
     int ensure_work(int64_t elems);
-    // device pointers; y = (H + shift) x
-    int matblock(const double2 *x, double2 *y, int nvec, double2 shift = double2{0.0, 0.0});
+    // device pointers; y = (H + shift) x (exch: 1 or -1 when every vector has
+    // X^T = exch X, which halves the kinetic work where the default kernels
+    // run; 0 otherwise)
+    int matblock(const double2 *x, double2 *y, int nvec, double2 shift = double2{0.0, 0.0}, double exch = 0.0);
     // the same in FP32 on complex64 vectors (the mixed form's inner solve)
-    // (exch: 1 or -1 when every vector has X^T = exch X, which halves the
-    // kinetic work where the default kernels run; 0 otherwise)
     int matblock32(const float2 *x, float2 *y, int nvec, double2 shift = double2{0.0, 0.0}, double exch = 0.0);
     // the kinetic-eigenbasis preconditioner MSOLVECPLX22 (kinpc.cu), y = P x
     // on device vectors (y must not alias x); W and 1/D are built on first

@@ -85,10 +85,12 @@ cudaError_t hammult_line_pass_launch(const HamDev &h, const double2 *x, double2 
 cudaError_t hammult_line_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride,
                                      int pass, cudaStream_t st, double2 shift);
 
-// The complex64 product on vectors with X^T = sign X (sign = 1 or -1; exact,
-// or to the storage's rounding): pass 0 writes T_1 X, pass 1 completes Y = (H
+// The product on vectors with X^T = sign X (sign = 1 or -1; exact, or to the
+// storage's rounding): pass 0 writes T_1 X, pass 1 completes Y = (H
 // + shift) X from it in place, exactly (anti)symmetric.
 cudaError_t hammult_exch_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride, int pass,
+                                     double sign, cudaStream_t st, double2 shift);
+cudaError_t hammult_exch_pass_launch(const HamDev &h, const double2 *x, double2 *y, int nvec, int64_t vstride, int pass,
                                      double sign, cudaStream_t st, double2 shift);
 
 // The complex64 passes with the kinetic contractions on the tensor cores

@@ -76,7 +76,9 @@ struct Solver {
     float2 *Z32 = nullptr;  // mixed inner solve: the power basis Z_0..Z_order (complex64)
     bool mixed = false;
     double exch_sign = 0.0;     // +1 / -1: exchange symmetry of the start block, 0: none
-    double exch_mult = 0.0;     // the same where the start holds it to rounding: the inner products use it
+    // the same where the start held it to rounding (and now holds it exactly):
+    // every vector of the iteration has it, and the products use it
+    double exch_mult = 0.0;
     unsigned refl_keep = 0xFFu;  // reflection sectors the start block reaches (bit c: sector c)
     bool exch_done = false;      // the last inner solve's output is already exchange-projected
     bool z0_staged = false;      // the next inner solve's complex64 start Z_0 is already in Z32
@@ -172,7 +174,7 @@ struct Solver {
         auto t0 = clk::now();
         mv_exec += k;
         mv_ref += k;
-        int s = h->matblock(x, y, k);
+        int s = h->matblock(x, y, k, double2{0.0, 0.0}, exch_mult);
         t_mv += secs(t0, clk::now());
         return s;
     }
@@ -183,7 +185,7 @@ struct Solver {
         if (!compat) {
             mv_exec += k;
             mv_ref += k;
-            return h->matblock(x, y, k);
+            return h->matblock(x, y, k, double2{0.0, 0.0}, exch_mult);
         }
         mv_exec += 1;
         mv_ref += 1;
@@ -203,7 +205,7 @@ struct Solver {
         mv_exec += k;
         mv_ref += k;
         const cplx ms = -sigma;
-        return h->matblock(x, y, k, make_double2(ms.real(), ms.imag()));
+        return h->matblock(x, y, k, make_double2(ms.real(), ms.imag()), exch_mult);
     }
 
     static ColList cols(double2 *base, int k, int64_t D, double2 *sub = nullptr, cplx sg = 0.0)
@@ -1034,10 +1036,18 @@ struct Solver {
             }
         }
         exch_sign = sign;
-        // a part of squared norm worst / 2 is outside the sector; below
-        // complex64 rounding (6e-8 squared, with the reduction's own rounding
-        // allowed for) the inner products may take X^T = sign X for granted
+        // A part of squared norm worst / 2 lies outside the sector.  Where that
+        // is rounding, the start is put into the sector exactly; every step
+        // then keeps X^T = sign X bit for bit (the products write it, the
+        // blocks are projected, and all else acts element by element).
         exch_mult = worst < 2e-14 ? sign : 0.0;
+        if (exch_mult != 0.0) {
+            for (int j = 0; j < nev; ++j) {
+                cudaError_t e = exch_project_launch(col(X, j), h->m, exch_mult, st);
+                if (e != cudaSuccess) return cuda_error(e, "exch_project");
+            }
+            DE_TRY(normalize(X, nev));
+        }
         refl_keep = keep;
         return DE_OK;
     }

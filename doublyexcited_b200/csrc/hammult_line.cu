@@ -497,18 +497,20 @@ __global__ void __launch_bounds__(Cfg<R, NN>::CT, Cfg<R, NN>::CB) cube_line_kern
 //   Y <- Z + s Z^T + (V + shift) X
 // in place on pairs of 32 x 32 tiles (bi <= bj).  V is symmetric, so the
 // partner tile is s times the transpose: only the upper half of X is read,
-// and Y is exactly (anti)symmetric.  Complex64, memory-bound: 2.5 vector
-// passes after the cube kernel's 2, against 8 for the general product.
+// and Y is exactly (anti)symmetric.  Memory-bound: 2.5 vector passes after
+// the cube kernel's 2, against 8 for the general product.
 // Inside the mixed solve at NN = 13 the two take 44 us a product against 59.
 // 512 threads with two elements each and three CTAs per SM, measured there (ms
 // per outer iteration of 30 products): 5.18; four CTAs 5.39, two 5.26; 256
 // threads 5.18 at four CTAs, 5.26 at three; 128 threads 5.38.
 constexpr int kExchThreads = 512;
+template <class R>
 __global__ void __launch_bounds__(kExchThreads, 3)
-    exch_add_kernel(const __grid_constant__ LineArgs<float> a, int nn, float s)
+    exch_add_kernel(const __grid_constant__ LineArgs<R> a, int nn, R s)
 {
+    using G = std::conditional_t<sizeof(R) == 8, double2, float2>;
     constexpr int RY = kExchThreads / 32, E = 32 / RY;
-    __shared__ float2 ta[32][33], tb[32][33];
+    __shared__ G ta[32][33], tb[32][33];
     __shared__ int bp[32], bq[32];
     const int m = nn * nn * nn, w = 2 * nn - 1;
     // the tile pair: blocks enumerate bi <= bj
@@ -526,21 +528,21 @@ __global__ void __launch_bounds__(kExchThreads, 3)
     }
     __syncthreads();
     const int p = p0 + tx, pt = q0 + tx;
-    const float tp = __ldg(a.t1a + min(p, m - 1));
+    const R tp = __ldg(a.t1a + min(p, m - 1));
     grid_wait();
     grid_release();
     for (int vec = blockIdx.y; vec < a.nvec; vec += gridDim.y) {
-        const float2 *x = reinterpret_cast<const float2 *>(a.x) + vec * a.vstride;
-        float2 *y = reinterpret_cast<float2 *>(a.y) + vec * a.vstride;
-        float2 za[E], zb[E], xa[E];
-        float v[E];
+        const G *x = reinterpret_cast<const G *>(a.x) + vec * a.vstride;
+        G *y = reinterpret_cast<G *>(a.y) + vec * a.vstride;
+        G za[E], zb[E], xa[E];
+        R v[E];
 #pragma unroll
         for (int u = 0; u < E; ++u) {
             const int c = ty + RY * u;
             const bool oka = p < m && q0 + c < m, okb = pt < m && p0 + c < m;
-            zb[u] = okb ? y[pt + (int64_t)m * (p0 + c)] : make_float2(0.f, 0.f);
-            za[u] = oka ? y[p + (int64_t)m * (q0 + c)] : make_float2(0.f, 0.f);
-            xa[u] = oka ? __ldg(x + p + (int64_t)m * (q0 + c)) : make_float2(0.f, 0.f);
+            zb[u] = okb ? y[pt + (int64_t)m * (p0 + c)] : G{R(0), R(0)};
+            za[u] = oka ? y[p + (int64_t)m * (q0 + c)] : G{R(0), R(0)};
+            xa[u] = oka ? __ldg(x + p + (int64_t)m * (q0 + c)) : G{R(0), R(0)};
             v[u] = (__ldg(a.t1a + min(q0 + c, m - 1)) + tp) + __ldg(a.v12 + bq[c] - bp[tx]);
         }
 #pragma unroll
@@ -549,21 +551,21 @@ __global__ void __launch_bounds__(kExchThreads, 3)
 #pragma unroll
         for (int u = 0; u < E; ++u) {
             const int c = ty + RY * u, q = q0 + c;
-            const float pr = fmaf(v[u], a.vsr, a.shr), pi = fmaf(v[u], a.vsi, a.shi);
-            const float2 zt = tb[c][tx];
-            float yr = za[u].x + s * zt.x, yi = za[u].y + s * zt.y;
+            const R pr = fma(v[u], a.vsr, a.shr), pi = fma(v[u], a.vsi, a.shi);
+            const G zt = tb[c][tx];
+            R yr = za[u].x + s * zt.x, yi = za[u].y + s * zt.y;
             yr += pr * xa[u].x - pi * xa[u].y;
             yi += pr * xa[u].y + pi * xa[u].x;
-            ta[tx][c] = make_float2(yr, yi);  // ta[r][c] = Y(p0 + r, q0 + c)
-            if (p < m && q < m) y[p + (int64_t)m * q] = make_float2(yr, yi);
+            ta[tx][c] = G{yr, yi};  // ta[r][c] = Y(p0 + r, q0 + c)
+            if (p < m && q < m) y[p + (int64_t)m * q] = G{yr, yi};
         }
         __syncthreads();
         if (bi != bj) {
 #pragma unroll
             for (int u = 0; u < E; ++u) {
                 const int c = ty + RY * u;
-                const float2 t = ta[c][tx];  // Y(p0 + c, q0 + tx)
-                if (pt < m && p0 + c < m) y[pt + (int64_t)m * (p0 + c)] = make_float2(s * t.x, s * t.y);
+                const G t = ta[c][tx];  // Y(p0 + c, q0 + tx)
+                if (pt < m && p0 + c < m) y[pt + (int64_t)m * (p0 + c)] = G{s * t.x, s * t.y};
             }
         }
     }
@@ -604,11 +606,9 @@ cudaError_t prepare()
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(cube_line_kernel<R, NN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)K::CSMEM);
-    if constexpr (sizeof(R) == 4) {
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(cube_line_kernel<R, NN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)K::CSMEM);
-    }
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(cube_line_kernel<R, NN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)K::CSMEM);
     if (e == cudaSuccess) done[dev].store(true, std::memory_order_release);
     return e;
 }
@@ -626,9 +626,8 @@ cudaError_t pass(const LineArgs<R> &a, int which, cudaStream_t st)
         return launch<R>(kline_kernel<R, NN>, dim3((K::M * K::P2 + K::KT - 1) / K::KT, ny), K::KT, K::KSMEM, a, st);
     }
     const unsigned units = (unsigned)std::min<int64_t>((int64_t)K::M * a.nvec, 0x7fffffff);
-    if (which == 1) return launch<R>(cube_line_kernel<R, NN, true>, dim3(units), K::CT, K::CSMEM, a, st);
-    if constexpr (sizeof(R) == 4) return launch<R>(cube_line_kernel<R, NN, false>, dim3(units), K::CT, K::CSMEM, a, st);
-    else return cudaErrorInvalidValue;
+    return launch<R>(which == 1 ? cube_line_kernel<R, NN, true> : cube_line_kernel<R, NN, false>, dim3(units), K::CT,
+                     K::CSMEM, a, st);
 }
 
 template <class R, class G>
@@ -688,12 +687,14 @@ cudaError_t hammult_line_pass_launch(const HamDev &h, const float2 *x, float2 *y
     return go<float>(h, line_args<float>(h, x, y, nvec, vstride, shift), pass, st);
 }
 
-cudaError_t hammult_exch_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride, int pass,
-                                     double sign, cudaStream_t st, double2 shift)
+template <class R, class G>
+static cudaError_t exch_pass(const HamDev &h, const G *x, G *y, int nvec, int64_t vstride, int pass, double sign,
+                             cudaStream_t st, double2 shift)
 {
-    if (h.nelec != 2 || nvec <= 0 || !h.t1af || !h.v12f) return cudaErrorInvalidValue;
-    const LineArgs<float> a = line_args<float>(h, x, y, nvec, vstride, shift);
-    if (pass == 0) return go<float>(h, a, 2, st);
+    if (h.nelec != 2 || nvec <= 0) return cudaErrorInvalidValue;
+    const LineArgs<R> a = line_args<R>(h, x, y, nvec, vstride, shift);
+    if (!a.t1a || !a.v12) return cudaErrorInvalidValue;
+    if (pass == 0) return go<R>(h, a, 2, st);
     const int tiles = (int)((h.m + 31) / 32);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(tiles * (tiles + 1) / 2), (unsigned)std::min(nvec, 65535));
@@ -704,9 +705,21 @@ cudaError_t hammult_exch_pass_launch(const HamDev &h, const float2 *x, float2 *y
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = programmatic_launch() ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, exch_add_kernel, a, h.nn, (float)sign);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, exch_add_kernel<R>, a, h.nn, (R)sign);
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+cudaError_t hammult_exch_pass_launch(const HamDev &h, const float2 *x, float2 *y, int nvec, int64_t vstride, int pass,
+                                     double sign, cudaStream_t st, double2 shift)
+{
+    return exch_pass<float>(h, x, y, nvec, vstride, pass, sign, st, shift);
+}
+
+cudaError_t hammult_exch_pass_launch(const HamDev &h, const double2 *x, double2 *y, int nvec, int64_t vstride, int pass,
+                                     double sign, cudaStream_t st, double2 shift)
+{
+    return exch_pass<double>(h, x, y, nvec, vstride, pass, sign, st, shift);
 }
 
 }  // namespace de
