@@ -17,6 +17,7 @@
 // most 40 columns) computes in FP32.
 #include "de_internal.h"
 #include "de_kernels.h"
+#include "tri.h"
 
 #include <cuda.h>
 
@@ -321,7 +322,8 @@ __global__ void scale_kernel(const __grid_constant__ PtrPack P, const double2 *c
         P.out[j][r] = cmul(P.out[j][r], c);
 }
 
-__global__ void dotdiag_partial(const __grid_constant__ PtrPack P, int64_t len, int herm,
+template <bool TRI>
+__global__ void dotdiag_partial(const __grid_constant__ PtrPack P, int64_t len, unsigned m, int herm,
                                 double2 *__restrict__ work)
 {
     const int j = blockIdx.y;
@@ -329,7 +331,17 @@ __global__ void dotdiag_partial(const __grid_constant__ PtrPack P, int64_t len, 
     const double sg = herm ? -1.0 : 1.0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < len; r += stride) {
-        const double2 a = P.a[j][r], b = P.b[j][r];
+        int64_t row = r;
+        double w = 1.0;
+        if constexpr (TRI) {
+            if (!tri_row((unsigned)r, m, row, w)) continue;
+        }
+        double2 a = P.a[j][row];
+        const double2 b = P.b[j][row];
+        if constexpr (TRI) {
+            a.x *= w;
+            a.y *= w;
+        }
         const double ay = sg * a.y;
         sr = fma(a.x, b.x, sr);
         sr = fma(-ay, b.y, sr);
@@ -592,9 +604,9 @@ __global__ void __launch_bounds__(256)
 // the last of the NC, as in orthogonalise-and-normalise, and is read once.
 // HBM-bound; inside the mixed solve at 4.8 M rows, us before -> now (HBM time):
 // 3-4 columns 79 -> 44-56 (35-47), 5-8 columns 133 -> 70-108 (59-94).
-template <int NC, bool SELF>
+template <int NC, bool SELF, bool TRI>
 __global__ void __launch_bounds__(256, 2)
-    gram_col(const __grid_constant__ ColListT<double2> L, const double2 *__restrict__ b, int64_t len, int herm,
+    gram_col(const __grid_constant__ ColListT<double2> L, const double2 *__restrict__ b, int64_t len, unsigned m, int herm,
              double2 *__restrict__ work, double2 *__restrict__ out)
 {
     constexpr int U = 2;
@@ -608,10 +620,13 @@ __global__ void __launch_bounds__(256, 2)
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < len; r += U * stride) {
         double2 l[U][NC], x[U];
+        double wt[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int64_t ru = r + u * stride;
-            const bool in = ru < len;
+            wt[u] = 1.0;
+            int64_t ru = r + u * stride;
+            bool in = ru < len;
+            if constexpr (TRI) in = in && tri_row((unsigned)ru, m, ru, wt[u]);
 #pragma unroll
             for (int i = 0; i < NC; ++i) l[u][i] = in ? __ldg(col[i] + ru) : make_double2(0.0, 0.0);
             if constexpr (!SELF) x[u] = in ? __ldg(b + ru) : make_double2(0.0, 0.0);
@@ -619,6 +634,10 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if constexpr (SELF) x[u] = l[u][NC - 1];
+            if constexpr (TRI) {
+                x[u].x *= wt[u];
+                x[u].y *= wt[u];
+            }
 #pragma unroll
             for (int i = 0; i < NC; ++i) {
                 const double ly = sg * l[u][i].y;
@@ -1302,10 +1321,10 @@ __device__ __forceinline__ void dmma_g(double &d0, double &d1, double a, double 
 // columns are b_c = a_c - sigma v_c (c < 8) and R is [b_0..b_7, v_0..v_7],
 // so a lane's two loads (a_c, v_c of its column c) give its L fragment and
 // both R fragments.
-template <class S, int MTW, int NTW, bool KM8 = false>
+template <class S, int MTW, int NTW, bool KM8, bool TRI>
 __global__ void __launch_bounds__(512)
     gram_tc(const __grid_constant__ ColListT<S> L, const __grid_constant__ ColListT<S> R, int64_t len, int64_t chunk,
-            int herm, int wm, int wn, int rg, double2 *__restrict__ work)
+            unsigned m, int herm, int wm, int wn, int rg, double2 *__restrict__ work)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per = wm * wn;
@@ -1353,15 +1372,17 @@ __global__ void __launch_bounds__(512)
         double2 lv[US][MTW], rv[US][NTW];
 #pragma unroll
         for (int u = 0; u < US; ++u) {
-            const int64_t r = rb + 4 * (int64_t)rg * u + q4;
-            const bool rok = r < r1;
+            int64_t r = rb + 4 * (int64_t)rg * u + q4;
+            bool rok = r < r1;
+            double wt = 1.0;
+            if constexpr (TRI) rok = rok && tri_row((unsigned)r, m, r, wt);
             if constexpr (KM8) {
                 const double2 av = rok ? ld2(la[0] + r) : make_double2(0.0, 0.0);
                 const double2 v = rok ? ld2(lb[0] + r) : make_double2(0.0, 0.0);
                 const double2 sgm = L.sigma;
                 lv[u][0] = make_double2(av.x - (sgm.x * v.x - sgm.y * v.y), av.y - (sgm.x * v.y + sgm.y * v.x));
                 rv[u][0] = lv[u][0];
-                rv[u][1] = v;
+                rv[u][NTW - 1] = v;
             } else {
 #pragma unroll
                 for (int a = 0; a < MTW; ++a)
@@ -1369,6 +1390,13 @@ __global__ void __launch_bounds__(512)
 #pragma unroll
                 for (int b = 0; b < NTW; ++b)
                     rv[u][b] = (rok && ra[b]) ? elem(ra[b], rbp[b], R.sigma, r) : make_double2(0.0, 0.0);
+            }
+            if constexpr (TRI) {
+#pragma unroll
+                for (int b = 0; b < NTW; ++b) {
+                    rv[u][b].x *= wt;
+                    rv[u][b].y *= wt;
+                }
             }
         }
 #pragma unroll
@@ -1415,10 +1443,13 @@ __global__ void __launch_bounds__(512)
     }
 }
 
-template <class S, int MTW, int NTW, bool KM8 = false>
+template <class S, int MTW, int NTW, bool KM8 = false, bool TRI = false>
 static cudaError_t gram_tc_go(const ColListT<S> &L, const ColListT<S> &R, int64_t len, int herm, double2 *out, int ldo,
-                              double2 *work, cudaStream_t st)
+                              double2 *work, cudaStream_t st, int64_t tri)
 {
+    if constexpr (!TRI) {
+        if (tri) return gram_tc_go<S, MTW, NTW, KM8, true>(L, R, tri_slots(tri), herm, out, ldo, work, st, tri);
+    }
     const int mt = (L.n + 7) / 8, nt = (R.n + 7) / 8;
     const int wm = (mt + MTW - 1) / MTW, wn = (nt + NTW - 1) / NTW;
     const int per = wm * wn;
@@ -1431,7 +1462,7 @@ static cudaError_t gram_tc_go(const ColListT<S> &L, const ColListT<S> &R, int64_
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gram_tc<S, MTW, NTW, KM8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gram_tc<S, MTW, NTW, KM8, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              512 * MTW * NTW * 2 * (int)sizeof(double2));
         if (e != cudaSuccess) return e;
         attr[dev] = true;
@@ -1442,7 +1473,7 @@ static cudaError_t gram_tc_go(const ColListT<S> &L, const ColListT<S> &R, int64_
     int64_t chunk = (len + nblk - 1) / nblk;
     chunk = (chunk + 3) / 4 * 4;
     work += 1;
-    gram_tc<S, MTW, NTW, KM8><<<nblk, threads, smem, st>>>(L, R, len, chunk, herm, wm, wn, rg, work);
+    gram_tc<S, MTW, NTW, KM8, TRI><<<nblk, threads, smem, st>>>(L, R, len, chunk, (unsigned)tri, herm, wm, wn, rg, work);
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -1454,10 +1485,16 @@ static cudaError_t gram_tc_go(const ColListT<S> &L, const ColListT<S> &R, int64_
 
 template <int NC, bool SELF>
 static cudaError_t gram_col_go(const ColList &L, const double2 *b, int64_t len, int herm, double2 *out, double2 *work,
-                               cudaStream_t st)
+                               cudaStream_t st, int64_t tri)
 {
-    const int blocks = fused_blocks<gram_col<NC, SELF>>((len + 1) / 2, NC);
-    gram_col<NC, SELF><<<blocks, 256, 0, st>>>(L, b, len, herm, work, out);
+    if (tri) {
+        len = tri_slots(tri);
+        const int blocks = fused_blocks<gram_col<NC, SELF, true>>((len + 1) / 2, NC);
+        gram_col<NC, SELF, true><<<blocks, 256, 0, st>>>(L, b, len, (unsigned)tri, herm, work, out);
+    } else {
+        const int blocks = fused_blocks<gram_col<NC, SELF, false>>((len + 1) / 2, NC);
+        gram_col<NC, SELF, false><<<blocks, 256, 0, st>>>(L, b, len, 0u, herm, work, out);
+    }
     count_launch();
     return cudaGetLastError();
 }
@@ -1465,32 +1502,32 @@ static cudaError_t gram_col_go(const ColList &L, const double2 *b, int64_t len, 
 // L unshifted, 2 <= L.n <= 9, one unshifted column in R
 template <bool SELF>
 static cudaError_t gram_col_any(const ColList &L, const double2 *b, int64_t len, int herm, double2 *out, double2 *work,
-                                cudaStream_t st)
+                                cudaStream_t st, int64_t tri)
 {
     switch (L.n) {
-    case 2: return gram_col_go<2, SELF>(L, b, len, herm, out, work, st);
-    case 3: return gram_col_go<3, SELF>(L, b, len, herm, out, work, st);
-    case 4: return gram_col_go<4, SELF>(L, b, len, herm, out, work, st);
-    case 5: return gram_col_go<5, SELF>(L, b, len, herm, out, work, st);
-    case 6: return gram_col_go<6, SELF>(L, b, len, herm, out, work, st);
-    case 7: return gram_col_go<7, SELF>(L, b, len, herm, out, work, st);
-    case 8: return gram_col_go<8, SELF>(L, b, len, herm, out, work, st);
-    case 9: return gram_col_go<9, SELF>(L, b, len, herm, out, work, st);
+    case 2: return gram_col_go<2, SELF>(L, b, len, herm, out, work, st, tri);
+    case 3: return gram_col_go<3, SELF>(L, b, len, herm, out, work, st, tri);
+    case 4: return gram_col_go<4, SELF>(L, b, len, herm, out, work, st, tri);
+    case 5: return gram_col_go<5, SELF>(L, b, len, herm, out, work, st, tri);
+    case 6: return gram_col_go<6, SELF>(L, b, len, herm, out, work, st, tri);
+    case 7: return gram_col_go<7, SELF>(L, b, len, herm, out, work, st, tri);
+    case 8: return gram_col_go<8, SELF>(L, b, len, herm, out, work, st, tri);
+    case 9: return gram_col_go<9, SELF>(L, b, len, herm, out, work, st, tri);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <class S>
 static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t len, int herm, double2 *out, int ldo,
-                            double2 *work, cudaStream_t st)
+                            double2 *work, cudaStream_t st, int64_t tri)
 {
     if (L.n < 1 || L.n > 64 || R.n < 1 || R.n > 128 || len < 1) return cudaErrorInvalidValue;
     if constexpr (sizeof(S) == 16) {
         bool plain = R.n == 1 && L.n >= 2 && L.n <= 9 && !R.b[0];
         for (int i = 0; i < L.n && plain; ++i) plain = !L.b[i];
         if (plain)
-            return L.a[L.n - 1] == R.a[0] ? gram_col_any<true>(L, R.a[0], len, herm, out, work, st)
-                                          : gram_col_any<false>(L, R.a[0], len, herm, out, work, st);
+            return L.a[L.n - 1] == R.a[0] ? gram_col_any<true>(L, R.a[0], len, herm, out, work, st, tri)
+                                          : gram_col_any<false>(L, R.a[0], len, herm, out, work, st, tri);
     }
     if (R.n == 1 && L.n <= 32) {
         if (L.n <= 1) return gram_small_go<1, 1>(L, R, len, herm, out, ldo, work, st);
@@ -1511,30 +1548,30 @@ static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t 
         bool km8 = R.sigma.x == L.sigma.x && R.sigma.y == L.sigma.y;
         for (int c = 0; c < 8 && km8; ++c)
             km8 = L.b[c] && R.a[c] == L.a[c] && R.b[c] == L.b[c] && R.a[8 + c] == L.b[c] && !R.b[8 + c];
-        if (km8) return gram_tc_go<S, 1, 2, true>(L, R, len, herm, out, ldo, work, st);
+        if (km8) return gram_tc_go<S, 1, 2, true>(L, R, len, herm, out, ldo, work, st, tri);
     }
     // the tiles keep one shift; no caller has two
     bool one_shift = true;
     if (R.sigma.x != L.sigma.x || R.sigma.y != L.sigma.y)
         for (int j = 0; j < R.n; ++j) one_shift = one_shift && !R.b[j];
-    if (one_shift && gram_tile_supported(L.n, R.n)) return gram_tile_launch(L, R, len, herm, out, ldo, work, st);
+    if (one_shift && gram_tile_supported(L.n, R.n)) return gram_tile_launch(L, R, len, herm, out, ldo, work, st, tri);
     // everything else on the FP64 tensor cores, warp tiles sized to the output
     const int mt = (L.n + 7) / 8, nt = (R.n + 7) / 8;
-    if (mt == 1) return gram_tc_go<S, 1, 4>(L, R, len, herm, out, ldo, work, st);
-    if (nt <= 4) return gram_tc_go<S, 2, 2>(L, R, len, herm, out, ldo, work, st);
-    return gram_tc_go<S, 2, 4>(L, R, len, herm, out, ldo, work, st);
+    if (mt == 1) return gram_tc_go<S, 1, 4>(L, R, len, herm, out, ldo, work, st, tri);
+    if (nt <= 4) return gram_tc_go<S, 2, 2>(L, R, len, herm, out, ldo, work, st, tri);
+    return gram_tc_go<S, 2, 4>(L, R, len, herm, out, ldo, work, st, tri);
 }
 
 cudaError_t gram_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out, int ldo,
-                        double2 *work, cudaStream_t st)
+                        double2 *work, cudaStream_t st, int64_t tri)
 {
-    return gram_any(L, R, len, herm, out, ldo, work, st);
+    return gram_any(L, R, len, herm, out, ldo, work, st, tri);
 }
 
 cudaError_t gram_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,
-                        double2 *work, cudaStream_t st)
+                        double2 *work, cudaStream_t st, int64_t tri)
 {
-    return gram_any(L, R, len, herm, out, ldo, work, st);
+    return gram_any(L, R, len, herm, out, ldo, work, st, tri);
 }
 
 namespace {
@@ -1585,9 +1622,9 @@ __device__ __forceinline__ void herm_acc(double (&ar)[NZ * (NZ + 1) / 2], double
 // G = Z^H Z (n = NZ complex64 columns, FP64 sums) in one read: each thread
 // adds all NZ (NZ + 1) / 2 packed sums of two rows per step; warps, blocks
 // and the last block's fixed-order tree reduce them.
-template <int NZ>
+template <int NZ, bool TRI>
 __global__ void __launch_bounds__(256, 2)
-    gram_herm_kernel(const __grid_constant__ ColListT<float2> Z, int64_t len, double2 *__restrict__ work,
+    gram_herm_kernel(const __grid_constant__ ColListT<float2> Z, int64_t len, unsigned m, double2 *__restrict__ work,
                      double2 *__restrict__ out, int ldo)
 {
     constexpr int NP = NZ * (NZ + 1) / 2;
@@ -1598,14 +1635,27 @@ __global__ void __launch_bounds__(256, 2)
     const float2 *zc[NZ];
 #pragma unroll
     for (int j = 0; j < NZ; ++j) zc[j] = Z.a[j];
+    // upper half: the sums are doubled at the end, so a diagonal row enters by half
+    auto halve = [](double(&xr)[NZ], double(&xi)[NZ]) {
+#pragma unroll
+        for (int j = 0; j < NZ; ++j) {
+            xr[j] *= 0.70710678118654752440;
+            xi[j] *= 0.70710678118654752440;
+        }
+    };
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < len; r0 += 2 * stride) {
-        const int64_t r1 = r0 + stride;
-        const bool has1 = r1 < len;
+        int64_t ra = r0, r1 = r0 + stride;
+        bool has0 = true, has1 = r1 < len;
+        double w0 = 1.0, w1 = 1.0;
+        if constexpr (TRI) {
+            has0 = tri_row((unsigned)r0, m, ra, w0);
+            has1 = has1 && tri_row((unsigned)r1, m, r1, w1);
+        }
         float2 z0[NZ], z1[NZ];
 #pragma unroll
         for (int j = 0; j < NZ; ++j) {
-            z0[j] = __ldg(zc[j] + r0);
+            z0[j] = has0 ? __ldg(zc[j] + ra) : make_float2(0.f, 0.f);
             z1[j] = has1 ? __ldg(zc[j] + r1) : make_float2(0.f, 0.f);
         }
         double xr[NZ], xi[NZ];
@@ -1614,12 +1664,14 @@ __global__ void __launch_bounds__(256, 2)
             xr[j] = z0[j].x;
             xi[j] = z0[j].y;
         }
+        if (TRI && w0 == 1.0) halve(xr, xi);
         herm_acc<NZ, 0>(ar, ai, xr, xi);
 #pragma unroll
         for (int j = 0; j < NZ; ++j) {
             xr[j] = z1[j].x;
             xi[j] = z1[j].y;
         }
+        if (TRI && w1 == 1.0) halve(xr, xi);
         herm_acc<NZ, 0>(ar, ai, xr, xi);
     }
     __shared__ double2 wsum[8][NP];
@@ -1652,6 +1704,7 @@ __global__ void __launch_bounds__(256, 2)
             const int a = i < j ? i : j, b = i < j ? j : i;
             const int kk = a * NZ - a * (a - 1) / 2 + (b - a);  // packed index of (a, b)
             double2 v = res[kk];
+            if constexpr (TRI) v = make_double2(2.0 * v.x, 2.0 * v.y);
             if (i > j) v.y = -v.y;
             out[i + (int64_t)ldo * j] = v;
         }
@@ -1659,29 +1712,40 @@ __global__ void __launch_bounds__(256, 2)
     }
 }
 
-template <int NZ>
-cudaError_t gram_herm_go(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st)
+template <int NZ, bool TRI>
+cudaError_t gram_herm_go(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
+                         int64_t tri)
 {
     // partials: NZ (NZ + 1) / 2 per block must fit the reduction scratch (kSmallBlocks * 32)
+    if constexpr (TRI) len = tri_slots(tri);
     const int64_t want = (len + 511) / 512;
     const int blocks = (int)std::max<int64_t>(
-        1, std::min<int64_t>(want, std::min(wave_blocks<gram_herm_kernel<NZ>>(), kSmallBlocks)));
-    gram_herm_kernel<NZ><<<blocks, 256, 0, st>>>(Z, len, work, out, ldo);
+        1, std::min<int64_t>(want, std::min(wave_blocks<gram_herm_kernel<NZ, TRI>>(), kSmallBlocks)));
+    gram_herm_kernel<NZ, TRI><<<blocks, 256, 0, st>>>(Z, len, (unsigned)tri, work, out, ldo);
     count_launch();
     return cudaGetLastError();
 }
+
+template <int NZ>
+cudaError_t gram_herm_go(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
+                         int64_t tri)
+{
+    return tri ? gram_herm_go<NZ, true>(Z, len, out, ldo, work, st, tri)
+               : gram_herm_go<NZ, false>(Z, len, out, ldo, work, st, 0);
+}
 }  // namespace
 
-cudaError_t gram_herm_launch(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st)
+cudaError_t gram_herm_launch(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
+                             int64_t tri)
 {
     if (len < 1) return cudaErrorInvalidValue;
     switch (Z.n) {
-    case 2: return gram_herm_go<2>(Z, len, out, ldo, work, st);
-    case 3: return gram_herm_go<3>(Z, len, out, ldo, work, st);
-    case 4: return gram_herm_go<4>(Z, len, out, ldo, work, st);
-    case 5: return gram_herm_go<5>(Z, len, out, ldo, work, st);
-    case 6: return gram_herm_go<6>(Z, len, out, ldo, work, st);
-    case 7: return gram_herm_go<7>(Z, len, out, ldo, work, st);
+    case 2: return gram_herm_go<2>(Z, len, out, ldo, work, st, tri);
+    case 3: return gram_herm_go<3>(Z, len, out, ldo, work, st, tri);
+    case 4: return gram_herm_go<4>(Z, len, out, ldo, work, st, tri);
+    case 5: return gram_herm_go<5>(Z, len, out, ldo, work, st, tri);
+    case 6: return gram_herm_go<6>(Z, len, out, ldo, work, st, tri);
+    case 7: return gram_herm_go<7>(Z, len, out, ldo, work, st, tri);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -1794,9 +1858,10 @@ int64_t dotdiag_work_elems(int n, int64_t len)
 }
 
 cudaError_t dotdiag_launch(const double2 *const *a, const double2 *const *b, int n, int64_t len,
-                           int herm, double2 *out, double2 *work, cudaStream_t st)
+                           int herm, double2 *out, double2 *work, cudaStream_t st, int64_t tri)
 {
     if (n < 1 || n > 64) return cudaErrorInvalidValue;
+    if (tri) len = tri_slots(tri);
     PtrPack P{};
     for (int j = 0; j < n; ++j) {
         P.a[j] = a[j];
@@ -1804,7 +1869,8 @@ cudaError_t dotdiag_launch(const double2 *const *a, const double2 *const *b, int
     }
     work += 1;
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((len + 255) / 256, std::max(1, 296 / n)));
-    dotdiag_partial<<<dim3(nblk, n), 256, 0, st>>>(P, len, herm, work);
+    if (tri) dotdiag_partial<true><<<dim3(nblk, n), 256, 0, st>>>(P, len, (unsigned)tri, herm, work);
+    else dotdiag_partial<false><<<dim3(nblk, n), 256, 0, st>>>(P, len, 0u, herm, work);
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

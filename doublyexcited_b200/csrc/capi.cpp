@@ -258,7 +258,6 @@ int de_problem::matblock(const double2 *x, double2 *y, int nvec, double2 shift, 
         if (e != cudaSuccess) return cuda_error(e, "hammult1");
         return DE_OK;
     }
-    if (ham.fam[0][0] != DE_MATVEC_FMA || ham.fam[0][1] != DE_MATVEC_FMA) exch = 0.0;
     Rec r{{nullptr, nullptr, nullptr}, nvec, 0};
     DE_TRY(prof_begin(r));
     cudaError_t e = exch != 0.0 ? hammult_exch_pass_launch(ham, x, y, nvec, dim, 0, exch, stream, shift)
@@ -299,7 +298,6 @@ int de_problem::prof_end(Rec &r)
 int de_problem::matblock32(const float2 *x, float2 *y, int nvec, double2 shift, double exch)
 {
     if (p.nelec != 2) return set_error(DE_E_INVALID, "the FP32 matvec is built for the two-electron operator");
-    if (ham.fam[1][0] != DE_MATVEC_FMA || ham.fam[1][1] != DE_MATVEC_FMA) exch = 0.0;
     Rec r{{nullptr, nullptr, nullptr}, nvec, 1};
     DE_TRY(prof_begin(r));
     cudaError_t e = exch != 0.0 ? hammult_exch_pass_launch(ham, x, y, nvec, dim, 0, exch, stream, shift)

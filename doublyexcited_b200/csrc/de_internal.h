@@ -120,8 +120,8 @@ struct de_problem {
     int ensure_stage(int64_t elems);
     int ensure_work(int64_t elems);
     // device pointers; y = (H + shift) x (exch: 1 or -1 when every vector has
-    // X^T = exch X, which halves the kinetic work where the default kernels
-    // run; 0 otherwise)
+    // X^T = exch X and the default kernels serve the storage: half the kinetic
+    // work; 0 otherwise)
     int matblock(const double2 *x, double2 *y, int nvec, double2 shift = double2{0.0, 0.0}, double exch = 0.0);
     // the same in FP32 on complex64 vectors (the mixed form's inner solve)
     int matblock32(const float2 *x, float2 *y, int nvec, double2 shift = double2{0.0, 0.0}, double exch = 0.0);

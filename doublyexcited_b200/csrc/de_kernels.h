@@ -133,22 +133,25 @@ using ColListF = ColListT<float2>;
 // identity (herm=0).  out is device memory, column-major with leading
 // dimension ldo; nl <= 64, nr <= 128.  work must hold gram_work_elems().
 int64_t gram_work_elems(int nl, int nr, int64_t len);
+// tri = M: every column is an M x M vector with X^T = s X for one s (len = M^2),
+// and the sums run over its upper half (tri.h); 0: over all rows.
 cudaError_t gram_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out,
-                        int ldo, double2 *work, cudaStream_t st);
+                        int ldo, double2 *work, cudaStream_t st, int64_t tri = 0);
 cudaError_t gram_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,
-                        double2 *work, cudaStream_t st);
+                        double2 *work, cudaStream_t st, int64_t tri = 0);
 
 // The same on output tiles fed through shared memory (gram_tile.cu), for the
 // shapes gram_tile_supported accepts; L and R share one shift (L.sigma).
 bool gram_tile_supported(int nl, int nr);
 cudaError_t gram_tile_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out, int ldo,
-                             double2 *work, cudaStream_t st);
+                             double2 *work, cudaStream_t st, int64_t tri);
 cudaError_t gram_tile_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,
-                             double2 *work, cudaStream_t st);
+                             double2 *work, cudaStream_t st, int64_t tri);
 
 // Hermitian Gram G = Z^H Z of n <= 7 complex64 vectors (FP64 sums), all n x n
 // entries written to DEVICE out (column-major, ldo); work as for gram.
-cudaError_t gram_herm_launch(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st);
+cudaError_t gram_herm_launch(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
+                             int64_t tri = 0);
 
 // Y_j = beta_j * Y_j + alpha * sum_i X_i C(i,j) for j < nout (nout <= 16,
 // nin <= kMaxCols); C is DEVICE memory (complex, column-major, ldc).  Each
@@ -169,6 +172,18 @@ cudaError_t update_launch(const UpdListT<float2, float2> &U, const double2 *c_de
 cudaError_t update_launch(const UpdListT<float2, double2> &U, const double2 *c_dev, int ldc, int64_t len,
                           cudaStream_t st);
 
+// The same on M x M vectors that all have X^T = s X (symops.cu), for M and
+// nout that update_sym_supported accepts; sym_rows_supported(M): grids whose
+// sums and updates take the upper half.
+bool sym_rows_supported(int64_t m);
+bool update_sym_supported(int64_t m, int nout);
+cudaError_t update_sym_launch(const UpdList &U, const double2 *c_dev, int ldc, int64_t m, double s, cudaStream_t st);
+cudaError_t update_sym_launch(const UpdListT<float2, double2> &U, const double2 *c_dev, int ldc, int64_t m, double s,
+                              cudaStream_t st);
+// axpc_f32_launch on such vectors (c_dev not null)
+cudaError_t axpc_f32_sym_launch(float2 *out, const double2 *a, const double2 *b, double2 s0, const double2 *c_dev,
+                                int64_t m, double s, cudaStream_t st);
+
 // out_j = a_j + s * c_j * b_j, c_j from DEVICE memory (j < n, n <= 64).
 // c_dev may be null (c_j = 1).  out may alias a.
 cudaError_t axpc_launch(double2 *const *out, const double2 *const *a, const double2 *const *b,
@@ -180,7 +195,7 @@ cudaError_t axpc_f32_launch(float2 *out, const double2 *a, const double2 *b, dou
 // d_j = sum_r conj(A_j[r]) B_j[r] (herm) for j < n (n <= 64) into DEVICE out.
 int64_t dotdiag_work_elems(int n, int64_t len);
 cudaError_t dotdiag_launch(const double2 *const *a, const double2 *const *b, int n, int64_t len,
-                           int herm, double2 *out, double2 *work, cudaStream_t st);
+                           int herm, double2 *out, double2 *work, cudaStream_t st, int64_t tri = 0);
 
 // Gram-Schmidt step of the inner solve: q -= sum_i qp_i d_i, v -= sum_i
 // vp_i d_i (d: m values in DEVICE memory), then q, v *= 1/sqrt(|<q,q>|); the

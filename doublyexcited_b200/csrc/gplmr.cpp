@@ -208,6 +208,17 @@ struct Solver {
         return h->matblock(x, y, k, make_double2(ms.real(), ms.imag()), exch_mult);
     }
 
+    // M where every vector is exactly (anti)symmetric and the grid's sums and
+    // updates then take the upper half; 0: all rows
+    int64_t tri() const { return exch_mult != 0.0 && sym_rows_supported(h->m) ? h->m : 0; }
+    template <class SI>
+    cudaError_t update_any(const UpdListT<SI, double2> &U, const double2 *c, int ldc)
+    {
+        if (exch_mult != 0.0 && update_sym_supported(h->m, U.nout))
+            return update_sym_launch(U, c, ldc, h->m, exch_mult, st);
+        return update_launch(U, c, ldc, D, st);
+    }
+
     static ColList cols(double2 *base, int k, int64_t D, double2 *sub = nullptr, cplx sg = 0.0)
     {
         ColList L{};
@@ -222,7 +233,7 @@ struct Solver {
 
     int gram_dev(const ColList &L, const ColList &R, double2 *out, int ldo, int herm = 1)
     {
-        cudaError_t e = gram_launch(L, R, D, herm, out, ldo, h->d_work, st);
+        cudaError_t e = gram_launch(L, R, D, herm, out, ldo, h->d_work, st, tri());
         if (e != cudaSuccess) return cuda_error(e, "gram");
         return DE_OK;
     }
@@ -267,7 +278,7 @@ struct Solver {
             U.beta[j] = make_double2(beta.real(), beta.imag());
         }
         U.alpha = make_double2(alpha.real(), alpha.imag());
-        cudaError_t e = update_launch(U, c, ldc, D, st);
+        cudaError_t e = update_any(U, c, ldc);
         if (e != cudaSuccess) return cuda_error(e, "update");
         return DE_OK;
     }
@@ -378,7 +389,7 @@ struct Solver {
     int normalize(double2 *x, int k, double2 *ax = nullptr)
     {
         std::vector<const double2 *> a = cl(x, k);
-        cudaError_t e = dotdiag_launch(a.data(), a.data(), k, D, 1, dR, h->d_work, st);
+        cudaError_t e = dotdiag_launch(a.data(), a.data(), k, D, 1, dR, h->d_work, st, tri());
         if (e != cudaSuccess) return cuda_error(e, "dotdiag");
         if ((e = inv_sqrt_abs_launch(dR, dT, k, st)) != cudaSuccess) return cuda_error(e, "inv_sqrt");
         std::vector<double2 *> w = clw(x, k);
@@ -408,7 +419,8 @@ struct Solver {
     {
         if (nev == 1 && !compat && mixed && order > 1 && order <= 6 && gm.usepetscflag != 0 &&
             gm.max_inner_iter > 0) {
-            cudaError_t e = axpc_f32_launch(Z32, a, b, make_double2(-1.0, 0.0), dE, D, st);
+            cudaError_t e = tri() ? axpc_f32_sym_launch(Z32, a, b, make_double2(-1.0, 0.0), dE, h->m, exch_mult, st)
+                                  : axpc_f32_launch(Z32, a, b, make_double2(-1.0, 0.0), dE, D, st);
             if (e != cudaSuccess) return cuda_error(e, "axpc_f32");
             z0_staged = true;
             return DE_OK;
@@ -420,10 +432,10 @@ struct Solver {
     int residuals(std::vector<cplx> &e_host, std::vector<double> &res)
     {
         std::vector<const double2 *> xx = cl(X, nev), aa = cl(AX, nev), ww = cl(W, nev);
-        cudaError_t e = dotdiag_launch(xx.data(), aa.data(), nev, D, 1, dE, h->d_work, st);
+        cudaError_t e = dotdiag_launch(xx.data(), aa.data(), nev, D, 1, dE, h->d_work, st, tri());
         if (e != cudaSuccess) return cuda_error(e, "dotdiag");
         DE_TRY(minus_e(W, AX, X, nev));
-        if ((e = dotdiag_launch(ww.data(), ww.data(), nev, D, 1, dR, h->d_work, st)) != cudaSuccess)
+        if ((e = dotdiag_launch(ww.data(), ww.data(), nev, D, 1, dR, h->d_work, st, tri())) != cudaSuccess)
             return cuda_error(e, "dotdiag");
         DE_CUDA(cudaMemcpyAsync(hbuf, dE, nev * sizeof(double2), cudaMemcpyDeviceToHost, st));
         DE_CUDA(cudaMemcpyAsync(hbuf + 64, dR, nev * sizeof(double2), cudaMemcpyDeviceToHost, st));
@@ -466,7 +478,7 @@ struct Solver {
     template <class S>
     int gramT(const ColListT<S> &L, const ColListT<S> &R, double2 *out, int ldo)
     {
-        cudaError_t e = gram_launch(L, R, D, 1, out, ldo, h->d_work, st);
+        cudaError_t e = gram_launch(L, R, D, 1, out, ldo, h->d_work, st, tri());
         if (e != cudaSuccess) return cuda_error(e, "gram");
         return DE_OK;
     }
@@ -497,7 +509,9 @@ struct Solver {
             U.beta[j] = make_double2(0.0, 0.0);
         }
         U.alpha = make_double2(1.0, 0.0);
-        cudaError_t e = update_launch(U, c, ldc, D, st);
+        cudaError_t e;
+        if constexpr (std::is_same_v<SO, double2>) e = update_any(U, c, ldc);
+        else e = update_launch(U, c, ldc, D, st);
         if (e != cudaSuccess) return cuda_error(e, "update");
         return DE_OK;
     }
@@ -515,7 +529,9 @@ struct Solver {
             U.beta[j] = make_double2(1.0, 0.0);
         }
         U.alpha = make_double2(-1.0, 0.0);
-        cudaError_t e = update_launch(U, c, ldc, D, st);
+        cudaError_t e;
+        if constexpr (std::is_same_v<S, double2>) e = update_any(U, c, ldc);
+        else e = update_launch(U, c, ldc, D, st);
         if (e != cudaSuccess) return cuda_error(e, "update");
         return DE_OK;
     }
@@ -898,11 +914,11 @@ struct Solver {
         if (k == 1 && nz <= 7) {
             // one column: the Hermitian Gram of the nz basis vectors (read
             // once) and the normal equations on the device -- no host trip
-            cudaError_t e = gram_herm_launch(colsT(Z32, nz, D), D, dG, nz, h->d_work, st);
+            cudaError_t e = gram_herm_launch(colsT(Z32, nz, D), D, dG, nz, h->d_work, st, tri());
             if (e != cudaSuccess) return cuda_error(e, "gram_herm");
             if ((e = small_sstep_solve_launch(dG, nz, dSV, dFlags, st)) != cudaSuccess)
                 return cuda_error(e, "small_sstep_solve");
-            if (exch_sign != 0.0) {  // the combination and the exchange projection in one pass
+            if (exch_sign != 0.0 && !tri()) {  // the combination and the exchange projection in one pass
                 const float2 *zs[8];
                 for (int i = 0; i < nq; ++i) zs[i] = Z32 + (int64_t)i * D;
                 if ((e = update_exch_launch(zs, nq, dSV, b, h->m, exch_sign, st)) != cudaSuccess)
@@ -1040,7 +1056,11 @@ struct Solver {
         // is rounding, the start is put into the sector exactly; every step
         // then keeps X^T = sign X bit for bit (the products write it, the
         // blocks are projected, and all else acts element by element).
-        exch_mult = worst < 2e-14 ? sign : 0.0;
+        // Only the default products write it.
+        bool exact = true;
+        for (int sto = 0; sto <= (mixed ? 1 : 0); ++sto)
+            for (int pass = 0; pass < 2; ++pass) exact = exact && h->ham.fam[sto][pass] == DE_MATVEC_FMA;
+        exch_mult = exact && worst < 2e-14 ? sign : 0.0;
         if (exch_mult != 0.0) {
             for (int j = 0; j < nev; ++j) {
                 cudaError_t e = exch_project_launch(col(X, j), h->m, exch_mult, st);
@@ -1057,7 +1077,8 @@ struct Solver {
     // applied it).
     int symmetry_project(double2 *b, int k)
     {
-        const bool skip_exch = exch_done;
+        // exact by construction with exch_mult, else done by the combination
+        const bool skip_exch = exch_done || exch_mult != 0.0;
         exch_done = false;
         for (int j = 0; j < k; ++j) {
             if (exch_sign != 0.0 && !skip_exch) {

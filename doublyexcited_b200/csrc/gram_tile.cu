@@ -22,6 +22,7 @@
 // complex64 (1.8 M rows): 10 x 12 502 -> 196, 20 x 24 1259 -> 737.  The shifted
 // 8 x 16 projection stays on gram_tc's one-load form (294 us against 446).
 #include "de_kernels.h"
+#include "tri.h"
 
 #include <algorithm>
 #include <atomic>
@@ -41,6 +42,7 @@ struct GramTileArgs {
     unsigned char lslot[kTile * kWarps], rslot[kTile * kWarps];
     double2 sigma;
     int64_t len;
+    unsigned m;  // TRI: rows are the slots of an M x M upper half
     int nslots, nshift, nl, nr, tl, tr, stages;
     double sign;  // -1: conj(L)
     double2 *work, *out;  // work[0]: the fused reductions' ticket, zero between launches
@@ -77,7 +79,7 @@ __device__ __forceinline__ void sum_partials(const double2 *work, int nblk, int 
 
 // RT rows a stage.  Warp w: tile
 // w % (tl tr), row group w / (tl tr).
-template <class S, int RT>
+template <class S, int RT, bool TRI>
 __global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_constant__ GramTileArgs<S> a)
 {
     extern __shared__ __align__(16) unsigned char gt_smem[];
@@ -98,8 +100,13 @@ __global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_con
             const int64_t r0 = tl * RT;
             for (int e = t; e < elems; e += nt) {
                 const int s = e / RT, r = e % RT;
-                const bool in = r0 + r < a.len;
-                copy_async<S>(ring + st * stride + e, a.col[s] + (in ? r0 + r : 0), in);
+                bool in = r0 + r < a.len;
+                int64_t row = r0 + r;
+                if constexpr (TRI) {
+                    double w;
+                    in = in && tri_row((unsigned)row, a.m, row, w);
+                }
+                copy_async<S>(ring + st * stride + e, a.col[s] + (in ? row : 0), in);
             }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -139,6 +146,16 @@ __global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_con
                 const S lv = xs[ls[i] + r], xv = xs[rs[i] + r];
                 l[i] = make_double2(lv.x, a.sign * lv.y);
                 x[i] = make_double2(xv.x, xv.y);
+            }
+            if constexpr (TRI) {
+                int64_t row;
+                double w;
+                tri_row((unsigned)(tl * RT + r), a.m, row, w);
+#pragma unroll
+                for (int i = 0; i < kTile; ++i) {
+                    x[i].x *= w;
+                    x[i].y *= w;
+                }
             }
 #pragma unroll
             for (int i = 0; i < kTile; ++i)
@@ -202,7 +219,7 @@ __global__ void __launch_bounds__(256)
     if (o < nl * nr) sum_partials(work, nblk, nl, nl * nr, o, threadIdx.x & 31, out, ldo);
 }
 
-template <class S, int RT>
+template <class S, int RT, bool TRI>
 cudaError_t tile_launch(const GramTileArgs<S> &a, int threads, size_t smem, cudaStream_t st)
 {
     static std::atomic<int> sms[64] = {};
@@ -211,7 +228,7 @@ cudaError_t tile_launch(const GramTileArgs<S> &a, int threads, size_t smem, cuda
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     int n = sms[dev].load(std::memory_order_relaxed);
     if (!n) {
-        cudaError_t e = cudaFuncSetAttribute(gram_tile_kernel<S, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(gram_tile_kernel<S, RT, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
         if (e != cudaSuccess) return e;
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         if (n <= 0) n = 148;
@@ -219,7 +236,7 @@ cudaError_t tile_launch(const GramTileArgs<S> &a, int threads, size_t smem, cuda
     }
     // two CTAs per SM: 112 KB of shared memory and 128 registers a thread
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((a.len + RT - 1) / RT, std::min(2 * n, 296)));
-    gram_tile_kernel<S, RT><<<nblk, threads, smem, st>>>(a);
+    gram_tile_kernel<S, RT, TRI><<<nblk, threads, smem, st>>>(a);
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || a.nl * a.nr <= kFusedOut) return e;
@@ -232,7 +249,7 @@ cudaError_t tile_launch(const GramTileArgs<S> &a, int threads, size_t smem, cuda
 // most kWarps tiles.
 template <class S>
 cudaError_t tile_go(const ColListT<S> &L, const ColListT<S> &R, int l0, int nl, int r0, int nr, int64_t len, int herm,
-                    double2 *out, int ldo, double2 *work, cudaStream_t st)
+                    double2 *out, int ldo, double2 *work, cudaStream_t st, int64_t tri)
 {
     GramTileArgs<S> a{};
     a.sigma = L.sigma;
@@ -257,7 +274,8 @@ cudaError_t tile_go(const ColListT<S> &L, const ColListT<S> &R, int l0, int nl, 
     a.tr = (nr + kTile - 1) / kTile;
     for (int i = nl; i < a.tl * kTile; ++i) a.lslot[i] = a.lslot[0];  // padding, dropped
     for (int j = nr; j < a.tr * kTile; ++j) a.rslot[j] = a.rslot[0];
-    a.len = len;
+    a.len = tri ? tri_slots(tri) : len;
+    a.m = (unsigned)tri;
     a.nl = nl;
     a.nr = nr;
     a.sign = herm ? -1.0 : 1.0;
@@ -269,14 +287,19 @@ cudaError_t tile_go(const ColListT<S> &L, const ColListT<S> &R, int l0, int nl, 
     const size_t stage = (size_t)a.nslots * rt * sizeof(S);
     a.stages = (int)std::max<size_t>(2, std::min<size_t>(4, 111 * 1024 / stage));
     const size_t smem = std::max<size_t>(stage * a.stages, kWarps * 16 * sizeof(double2));
-    if (rt == 256) return tile_launch<S, 256>(a, threads, smem, st);
-    if (rt == 128) return tile_launch<S, 128>(a, threads, smem, st);
-    return tile_launch<S, 64>(a, threads, smem, st);
+    if (tri) {
+        if (rt == 256) return tile_launch<S, 256, true>(a, threads, smem, st);
+        if (rt == 128) return tile_launch<S, 128, true>(a, threads, smem, st);
+        return tile_launch<S, 64, true>(a, threads, smem, st);
+    }
+    if (rt == 256) return tile_launch<S, 256, false>(a, threads, smem, st);
+    if (rt == 128) return tile_launch<S, 128, false>(a, threads, smem, st);
+    return tile_launch<S, 64, false>(a, threads, smem, st);
 }
 
 template <class S>
 cudaError_t tiles_go(const ColListT<S> &L, const ColListT<S> &R, int64_t len, int herm, double2 *out, int ldo,
-                     double2 *work, cudaStream_t st)
+                     double2 *work, cudaStream_t st, int64_t tri)
 {
     if (!gram_tile_supported(L.n, R.n)) return cudaErrorInvalidValue;
     const int tl = (L.n + kTile - 1) / kTile, tr = (R.n + kTile - 1) / kTile;
@@ -285,7 +308,7 @@ cudaError_t tiles_go(const ColListT<S> &L, const ColListT<S> &R, int64_t len, in
     for (int i = 0; i < L.n; i += bl * kTile)
         for (int j = 0; j < R.n; j += br * kTile) {
             cudaError_t e = tile_go(L, R, i, std::min(bl * kTile, L.n - i), j, std::min(br * kTile, R.n - j), len, herm,
-                                    out, ldo, work, st);
+                                    out, ldo, work, st, tri);
             if (e != cudaSuccess) return e;
         }
     return cudaSuccess;
@@ -302,15 +325,15 @@ bool gram_tile_supported(int nl, int nr)
 }
 
 cudaError_t gram_tile_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out, int ldo,
-                             double2 *work, cudaStream_t st)
+                             double2 *work, cudaStream_t st, int64_t tri)
 {
-    return tiles_go(L, R, len, herm, out, ldo, work, st);
+    return tiles_go(L, R, len, herm, out, ldo, work, st, tri);
 }
 
 cudaError_t gram_tile_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,
-                             double2 *work, cudaStream_t st)
+                             double2 *work, cudaStream_t st, int64_t tri)
 {
-    return tiles_go(L, R, len, herm, out, ldo, work, st);
+    return tiles_go(L, R, len, herm, out, ldo, work, st, tri);
 }
 
 }  // namespace de

@@ -543,7 +543,10 @@ __global__ void __launch_bounds__(kExchThreads, 3)
             zb[u] = okb ? y[pt + (int64_t)m * (p0 + c)] : G{R(0), R(0)};
             za[u] = oka ? y[p + (int64_t)m * (q0 + c)] : G{R(0), R(0)};
             xa[u] = oka ? __ldg(x + p + (int64_t)m * (q0 + c)) : G{R(0), R(0)};
-            v[u] = (__ldg(a.t1a + min(q0 + c, m - 1)) + tp) + __ldg(a.v12 + bq[c] - bp[tx]);
+            // in a diagonal tile both orders of a pair take the same table entry
+            // (TINV's two halves agree to rounding only)
+            const int lo = bi == bj ? min(c, tx) : tx, hi = bi == bj ? max(c, tx) : c;
+            v[u] = (__ldg(a.t1a + min(q0 + c, m - 1)) + tp) + __ldg(a.v12 + bq[hi] - bp[lo]);
         }
 #pragma unroll
         for (int u = 0; u < E; ++u) tb[tx][ty + RY * u] = zb[u];  // tb[r][c] = Z(q0 + r, p0 + c)

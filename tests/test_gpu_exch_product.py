@@ -41,3 +41,20 @@ def test_nearly_symmetric_starts(de, oracle, eps):
     # a part of size eps outside the sector enters the Ritz value squared, but
     # the mixed form drops it from the new directions where it keeps the sector
     assert np.abs(r64.e - r32.e).max() < TOL + 10 * eps
+
+
+@pytest.mark.parametrize("precision,n,nev", [("mixed", 3, 1), ("mixed", 5, 1), ("mixed", 4, 2), ("fp64", 3, 4),
+                                             ("fp64", 5, 2), ("fp64", 5, 5)])
+@pytest.mark.parametrize("spin", ["singlet", "triplet"])
+def test_iteration_keeps_the_sector_bit_for_bit(de, oracle, precision, n, nev, spin):
+    """Nothing in the iteration may leave X^T = +-X by a single bit: sums and
+    updates take the upper half of the vectors for granted (N >= 5), and no
+    projection follows the preconditioner."""
+    p = oracle.Params(n=n, delta=2.0, theta=0.3)
+    x0 = oracle.seeded_start(p, nev, 21, spin)
+    with de.Problem(n=n, delta=2.0, theta=0.3, precision=precision) as h:
+        r = h.gplmr_eig(x0, -0.78, ns=2, maxit=3, tol=1e-14, max_inner_iter=3)
+    s = 1.0 if spin == "singlet" else -1.0
+    for j in range(nev):
+        x = r.x[:, j].reshape(p.m, p.m)
+        assert np.array_equal(x, s * x.T)
