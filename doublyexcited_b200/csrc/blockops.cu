@@ -923,6 +923,37 @@ __global__ void small_cholinv(const double2 *__restrict__ G, int k, double2 *__r
         for (int i = j + 1; i < k; ++i) Rinv[i + k * j] = make_double2(0.0, 0.0);
 }
 
+// C = [-(G1 + G2) W; W] with W = R1^-1 R2^-1: G1, G2 m x k (ld m), the rest k x
+// k, C (m + k) x k (ld m + k), k <= 16.
+__global__ void __launch_bounds__(256)
+    small_block_coef(const double2 *__restrict__ g1, const double2 *__restrict__ g2, int m, int k,
+                     const double2 *__restrict__ r1, const double2 *__restrict__ r2, double2 *__restrict__ c)
+{
+    __shared__ double2 w[16 * 16];
+    if ((int)threadIdx.x < k * k) {
+        const int i = threadIdx.x % k, j = threadIdx.x / k;
+        double2 s = make_double2(0.0, 0.0);
+        for (int l = 0; l < k; ++l) {
+            const double2 p = cmul(r1[i + k * l], r2[l + k * j]);
+            s.x += p.x;
+            s.y += p.y;
+        }
+        w[threadIdx.x] = s;
+    }
+    __syncthreads();
+    for (int o = threadIdx.x; o < (m + k) * k; o += blockDim.x) {
+        const int i = o % (m + k), j = o / (m + k);
+        double2 s = i >= m ? w[i - m + k * j] : make_double2(0.0, 0.0);
+        for (int l = 0; i < m && l < k; ++l) {
+            const double2 a = g1[i + m * l], b = g2[i + m * l];
+            const double2 p = cmul(make_double2(a.x + b.x, a.y + b.y), w[l + k * j]);
+            s.x -= p.x;
+            s.y -= p.y;
+        }
+        c[o] = s;
+    }
+}
+
 // 1 x 1 case of gen_cmatsub flag 2 (hr_eigen.f90:223-291): g > 0 real.
 __global__ void small_hsqrt1(const double2 *__restrict__ g, double2 *__restrict__ ginvh, double2 *__restrict__ gsq,
                              int *flag)
@@ -2033,6 +2064,15 @@ cudaError_t small_cholinv_launch(const double2 *g, int k, double2 *rinv, int *fl
 {
     if (k < 1 || k > 16) return cudaErrorInvalidValue;
     small_cholinv<<<1, 32, 0, st>>>(g, k, rinv, flag);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t small_block_coef_launch(const double2 *g1, const double2 *g2, int m, int k, const double2 *r1,
+                                    const double2 *r2, double2 *c, cudaStream_t st)
+{
+    if (m < 0 || k < 1 || k > 16) return cudaErrorInvalidValue;
+    small_block_coef<<<1, 256, 0, st>>>(g1, g2, m, k, r1, r2, c);
     count_launch();
     return cudaGetLastError();
 }

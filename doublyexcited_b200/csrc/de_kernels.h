@@ -257,6 +257,10 @@ cudaError_t small_cholinv_launch(const double2 *g, int k, double2 *rinv, int *fl
 // The mixed inner solve's normal equations for one column (Gram g of the
 // nz <= 9 power-basis vectors): the nz - 1 coefficients into DEVICE a.
 cudaError_t small_sstep_solve_launch(const double2 *g, int nz, double2 *a, int *flag, cudaStream_t st);
+// c = [-(g1 + g2) r1 r2; r1 r2], the coefficients of a pair block's V
+// (Solver::block_orthonormalize): g m x k, r k x k, c (m + k) x k.
+cudaError_t small_block_coef_launch(const double2 *g1, const double2 *g2, int m, int k, const double2 *r1,
+                                    const double2 *r2, double2 *c, cudaStream_t st);
 cudaError_t small_hsqrt1_launch(const double2 *g, double2 *ginvh, double2 *gsq, int *flag, cudaStream_t st);
 // |T - I| <= tol elementwise (the reference's self-check uses 1e-10).
 cudaError_t small_ortho_check_launch(const double2 *t, int k, int *flag, cudaStream_t st, double tol = 1e-10);

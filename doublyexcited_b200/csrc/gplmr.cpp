@@ -87,6 +87,7 @@ struct Solver {
     static constexpr double kOrthoTolMixed = 1e-3;
     double2 *dG = nullptr, *dC = nullptr, *dE = nullptr, *dR = nullptr, *dT = nullptr, *dT2 = nullptr;
     double2 *dOC = nullptr;  // orth_normalize's coefficients
+    double2 *dB1 = nullptr, *dB2 = nullptr, *dRinv2 = nullptr, *dVC = nullptr;  // block_orthonormalize
     double2 *dRinv = nullptr, *dGinvh = nullptr, *dGsq = nullptr, *dG1 = nullptr, *dSV = nullptr;
     int *dFlags = nullptr;
     double2 *hbuf = nullptr;  // pinned staging for k x k results (>= 64 x 128 + 64)
@@ -148,6 +149,10 @@ struct Solver {
         DE_TRY(alloc(&dE, 64));
         DE_TRY(alloc(&dR, 64));
         DE_TRY(alloc(&dOC, 130));
+        DE_TRY(alloc(&dB1, 64 * 16));
+        DE_TRY(alloc(&dB2, 64 * 16));
+        DE_TRY(alloc(&dRinv2, 16 * 16));
+        DE_TRY(alloc(&dVC, 80 * 16));
         DE_TRY(alloc(&dT, 64));
         DE_TRY(alloc(&dT2, 65));
         DE_TRY(alloc(&dRinv, 16 * 16));
@@ -597,23 +602,34 @@ struct Solver {
         return DE_OK;
     }
 
-    // Orthonormalise the k pairs (q_i, v_i) of one Krylov block among
-    // themselves in the q inner product: CholQR twice (G = Q^H Q = R^H R,
-    // Q <- Q R^-1, V <- V R^-1).  The QR factor with a positive real diagonal
-    // is unique, so this is the reference's column-by-column two-pass
-    // Gram-Schmidt (myhgramschmidt_many) to rounding, in 3 passes over the
-    // block instead of k.
+    // The k new pairs (q_i, v_i) of a Krylov block, the m0 earlier ones being
+    // columns [0, m0) of Q and V and the new ones [m0, m0 + k): two classical
+    // passes of the block Gram-Schmidt Q_new -= Q C (none for m0 = 0), then
+    // CholQR twice (G = Q_new^H Q_new = R^H R, Q_new <- Q_new R^-1).  The QR
+    // factor with a positive real diagonal is unique, so this is the
+    // reference's column-by-column two-pass Gram-Schmidt (myhgramschmidt_many)
+    // to rounding.  V only follows Q: its four updates have one product,
+    // V_new <- (V_new - V (C_1 + C_2)) R_1^-1 R_2^-1, which is formed at the
+    // end (5 m0 + 48 vector passes a block of k = 4 became 3.5 m0 + 30 in the
+    // exchange-symmetric case).
     template <class S>
-    int block_cholqr2(S *qb, S *vb, int k)
+    int block_orthonormalize(S *Q, S *V, int m0, int k)
     {
+        S *qb = Q + (int64_t)m0 * D;
+        double2 *gs[2] = {dB1, dB2}, *rs[2] = {dRinv, dRinv2};
+        for (int pass = 0; m0 > 0 && pass < 2; ++pass) {
+            DE_TRY(gramT(colsT(Q, m0, D), colsT(qb, k, D), gs[pass], m0));
+            DE_TRY(update_sub(Q, m0, qb, k, gs[pass], m0));
+        }
         for (int pass = 0; pass < 2; ++pass) {
             DE_TRY(gramT(colsT(qb, k, D), colsT(qb, k, D), dG, k));
-            cudaError_t e = small_cholinv_launch(dG, k, dRinv, dFlags, st);
+            cudaError_t e = small_cholinv_launch(dG, k, rs[pass], dFlags, st);
             if (e != cudaSuccess) return cuda_error(e, "small_cholinv");
-            DE_TRY(updateT(qb, k, qb, k, dRinv, k));
-            DE_TRY(updateT(vb, k, vb, k, dRinv, k));
+            DE_TRY(updateT(qb, k, qb, k, rs[pass], k));
         }
-        return DE_OK;
+        cudaError_t e = small_block_coef_launch(dB1, dB2, m0, k, dRinv, dRinv2, dVC, st);
+        if (e != cudaSuccess) return cuda_error(e, "small_block_coef");
+        return updateT(V, m0 + k, V + (int64_t)m0 * D, k, dVC, m0 + k);
     }
 
     int shift_sub(double2 *q, const double2 *v, int k)  // q <- q - sigma v
@@ -698,24 +714,10 @@ struct Solver {
                 mv_ref += compat ? 1 : k;  // the reference recomputes the product checked above
             }
             const int m0 = io * k;
-            if (k > 1 && m0 == 0 && !compat) {
-                DE_TRY(block_cholqr2(qb, vb, k));
-            } else if (k == 1 || m0 == 0) {
+            if (k == 1 || (m0 == 0 && compat)) {
                 for (int i = 0; i < k; ++i) DE_TRY(hgram(m0 + i, qb + (int64_t)i * D, vb + (int64_t)i * D));
             } else {
-                // Block form of the same two-pass classical Gram-Schmidt: the
-                // k new pairs are projected against the m0 earlier pairs as a
-                // block, twice (Q_new -= Q C, V_new -= V C with C = Q^H Q_new),
-                // then orthonormalised among themselves column by column.  In
-                // exact arithmetic this is the reference's column-by-column
-                // result; it reads each earlier vector 6 times per block
-                // instead of 5 times per column.
-                for (int pass = 0; pass < 2; ++pass) {
-                    DE_TRY(gramT(colsT(Q, m0, D), colsT(qb, k, D), dG, m0));
-                    DE_TRY(update_sub(Q, m0, qb, k, dG, m0));
-                    DE_TRY(update_sub(V, m0, vb, k, dG, m0));
-                }
-                DE_TRY(block_cholqr2(qb, vb, k));
+                DE_TRY(block_orthonormalize(Q, V, m0, k));
             }
         }
         // solution: V (lanham rhs), rhs(:,1,:) = G^{1/2} (:309-316)
