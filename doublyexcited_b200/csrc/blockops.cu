@@ -91,32 +91,37 @@ __device__ __forceinline__ double2 col_elem(const ColListT<S> &L, int c, int64_t
     return v;
 }
 
-// One 256-thread block per 32 outputs; warp g sums blocks b = g (mod 8).
+// One 256-thread block per 8 outputs: 32 groups take the partials of every
+// 32nd block, 16 loads in flight, then a fixed tree (29 us with 8 groups of one
+// warp and 1184 partials, 18 us so).
 __global__ void __launch_bounds__(256)
     gram_reduce(const double2 *__restrict__ work, int nblk, int nl, int nr, double2 *__restrict__ out, int ldo)
 {
-    __shared__ double2 acc[8][32];
-    const int g = threadIdx.x >> 5, lane = threadIdx.x & 31, o = blockIdx.x * 32 + lane;
+    __shared__ double2 acc[32][8];
+    const int k = threadIdx.x & 7, g = threadIdx.x >> 3, o = blockIdx.x * 8 + k;
     const int nout = nl * nr;
     double sx = 0.0, sy = 0.0;
-    if (o < nout) {
-#pragma unroll 8
-        for (int b = g; b < nblk; b += 8) {
-            const double2 v = work[(int64_t)b * nout + o];
-            sx += v.x;
-            sy += v.y;
+    for (int b = g; b < nblk && o < nout; b += 16 * 32) {
+        double2 v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            v[u] = b + 32 * u < nblk ? __ldg(work + (int64_t)(b + 32 * u) * nout + o) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            sx += v[u].x;
+            sy += v[u].y;
         }
     }
-    acc[g][lane] = make_double2(sx, sy);
+    acc[g][k] = make_double2(sx, sy);
     __syncthreads();
-    if (threadIdx.x < 32 && o < nout) {
-        double x = 0.0, y = 0.0;
-        for (int k = 0; k < 8; ++k) {
-            x += acc[k][threadIdx.x].x;
-            y += acc[k][threadIdx.x].y;
+    for (int half = 16; half > 0; half >>= 1) {
+        if (g < half) {
+            acc[g][k].x += acc[g + half][k].x;
+            acc[g][k].y += acc[g + half][k].y;
         }
-        out[o % nl + (int64_t)ldo * (o / nl)] = make_double2(x, y);
+        __syncthreads();
     }
+    if (g == 0 && o < nout) out[o % nl + (int64_t)ldo * (o / nl)] = acc[0][k];
 }
 
 int gram_blocks(int nl, int nr, int64_t len)
@@ -495,11 +500,18 @@ __device__ __forceinline__ void reduce_partials(const double2 *__restrict__ part
     const int o = threadIdx.x % np, g = threadIdx.x / np;
     double sx = 0.0, sy = 0.0;
     if (o < nout) {
-#pragma unroll 4
-        for (unsigned b = g; b < nblk; b += groups) {
-            const double2 v = __ldcg(part + (int64_t)b * stride + o);
-            sx += v.x;
-            sy += v.y;
+        // 16 loads in flight: this tail is latency, paid by every reduction
+        for (unsigned b = g; b < nblk; b += 16 * groups) {
+            double2 v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u)
+                v[u] = b + u * groups < nblk ? __ldcg(part + (int64_t)(b + u * groups) * stride + o)
+                                             : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                sx += v[u].x;
+                sy += v[u].y;
+            }
         }
     }
     acc[threadIdx.x] = make_double2(sx, sy);
@@ -877,50 +889,70 @@ __global__ void orth_norm_coef(const double2 *__restrict__ g, int n, double2 *__
     coef[n] = make_double2(r, 0.0);
 }
 
-__global__ void small_cholinv(const double2 *__restrict__ G, int k, double2 *__restrict__ Rinv, int *flag)
+// Right-looking Cholesky of the k x k matrix A in shared memory by the whole
+// block: A's upper triangle becomes R, inv its reciprocal diagonal; false on
+// breakdown.  The entries of a step are independent; one thread walking them
+// (and waiting for global memory at each) took 10 us at k = 4, 14 us for the 5
+// x 5 system of the power basis, against 4-5 us.
+__device__ __forceinline__ bool block_cholesky(double2 *A, double *inv, int k)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double2 R[16 * 16];
-    double rsum = 0.0;
-    for (int j = 0; j < k; ++j)
-        for (int i = 0; i < k; ++i) rsum += hypot(G[i + k * j].x, G[i + k * j].y);
-    if (rsum == 0.0) {
-        raise_flag(flag, 2);
+    for (int j = 0; j < k; ++j) {
+        const double dj = A[j + k * j].x;  // the same for every thread
+        if (!(dj > 0.0) || !isfinite(dj)) return false;
+        const double rjj = sqrt(dj), r = 1.0 / rjj;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            A[j + k * j] = make_double2(rjj, 0.0);
+            inv[j] = r;
+        }
+        for (int l = j + 1 + threadIdx.x; l < k; l += blockDim.x) {
+            A[j + k * l].x *= r;
+            A[j + k * l].y *= r;
+        }
+        __syncthreads();
+        const int n = k - j - 1;
+        for (int o = threadIdx.x; o < n * n; o += blockDim.x) {
+            const int i = j + 1 + o % n, l = j + 1 + o / n;
+            if (i > l) continue;
+            const double2 p = A[j + k * i], q = A[j + k * l];  // A(i,l) -= conj(R(j,i)) R(j,l)
+            A[i + k * l].x -= p.x * q.x + p.y * q.y;
+            A[i + k * l].y -= p.x * q.y - p.y * q.x;
+        }
+        __syncthreads();
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(64)
+    small_cholinv(const double2 *__restrict__ G, int k, double2 *__restrict__ Rinv, int *flag)
+{
+    __shared__ double2 R[16 * 16], X[16 * 16];
+    __shared__ double inv[16];
+    bool nonzero = false;
+    for (int o = threadIdx.x; o < k * k; o += blockDim.x) {
+        R[o] = G[o];
+        X[o] = make_double2(0.0, 0.0);
+        nonzero = nonzero || !(R[o].x == 0.0 && R[o].y == 0.0);
+    }
+    const bool any = __syncthreads_or(nonzero);
+    if (!any || !block_cholesky(R, inv, k)) {
+        if (threadIdx.x == 0) raise_flag(flag, any ? 1 : 2);
         return;
     }
-    for (int j = 0; j < k; ++j) {
-        double dj = G[j + k * j].x;
-        for (int i = 0; i < j; ++i) dj -= R[i + k * j].x * R[i + k * j].x + R[i + k * j].y * R[i + k * j].y;
-        if (!(dj > 0.0)) {
-            raise_flag(flag, 1);
-            return;
-        }
-        const double rjj = sqrt(dj);
-        R[j + k * j] = make_double2(rjj, 0.0);
-        for (int l = j + 1; l < k; ++l) {
-            double2 s = G[j + k * l];
-            for (int i = 0; i < j; ++i) {  // s -= conj(R(i,j)) R(i,l)
-                const double2 a = R[i + k * j], b = R[i + k * l];
-                s.x -= a.x * b.x + a.y * b.y;
-                s.y -= a.x * b.y - a.y * b.x;
-            }
-            R[j + k * l] = make_double2(s.x / rjj, s.y / rjj);
-        }
-        for (int l = 0; l < j; ++l) R[j + k * l] = make_double2(0.0, 0.0);
-    }
-    for (int j = 0; j < k; ++j)  // R x = e_j by back substitution
+    if ((int)threadIdx.x < k) {  // R x = e_j by back substitution, a column per thread
+        const int j = threadIdx.x;
         for (int i = j; i >= 0; --i) {
             double2 s = make_double2(i == j ? 1.0 : 0.0, 0.0);
             for (int l = i + 1; l <= j; ++l) {
-                const double2 a = R[i + k * l], b = Rinv[l + k * j];
+                const double2 a = R[i + k * l], b = X[l + k * j];
                 s.x -= a.x * b.x - a.y * b.y;
                 s.y -= a.x * b.y + a.y * b.x;
             }
-            const double rii = R[i + k * i].x;
-            Rinv[i + k * j] = make_double2(s.x / rii, s.y / rii);
+            X[i + k * j] = make_double2(s.x * inv[i], s.y * inv[i]);
         }
-    for (int j = 0; j < k; ++j)
-        for (int i = j + 1; i < k; ++i) Rinv[i + k * j] = make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    for (int o = threadIdx.x; o < k * k; o += blockDim.x) Rinv[o] = X[o];
 }
 
 // C = [-(G1 + G2) W; W] with W = R1^-1 R2^-1: G1, G2 m x k (ld m), the rest k x
@@ -1509,7 +1541,7 @@ static cudaError_t gram_tc_go(const ColListT<S> &L, const ColListT<S> &R, int64_
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int nout = L.n * R.n;
-    gram_reduce<<<(nout + 31) / 32, 256, 0, st>>>(work, nblk, L.n, R.n, out, ldo);
+    gram_reduce<<<(nout + 7) / 8, 256, 0, st>>>(work, nblk, L.n, R.n, out, ldo);
     count_launch();
     return cudaGetLastError();
 }
@@ -1567,6 +1599,13 @@ static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t 
         if (L.n <= 8) return gram_small_go<8, 1>(L, R, len, herm, out, ldo, work, st);
         if (L.n <= 16) return gram_small_go<16, 1>(L, R, len, herm, out, ldo, work, st);
         return gram_small_go<32, 1>(L, R, len, herm, out, ldo, work, st);
+    }
+    // a block against itself: half the sums, one read of each column (4 x 4 at
+    // 1.8 M rows 24 us against 32 on the tiles)
+    if constexpr (sizeof(S) == 16) {
+        bool self = herm && L.n == R.n && L.n >= 2 && L.n <= 7;
+        for (int i = 0; i < L.n && self; ++i) self = L.a[i] == R.a[i] && !L.b[i] && !R.b[i];
+        if (self) return gram_herm_launch(L, len, out, ldo, work, st, tri);
     }
     // up to 4 x 4 of a short vector in one fused launch, all operands straight
     // into registers: 13 us against 15 for the tiles at 118 K rows, 70 against
@@ -1653,9 +1692,9 @@ __device__ __forceinline__ void herm_acc(double (&ar)[NZ * (NZ + 1) / 2], double
 // G = Z^H Z (n = NZ complex64 columns, FP64 sums) in one read: each thread
 // adds all NZ (NZ + 1) / 2 packed sums of two rows per step; warps, blocks
 // and the last block's fixed-order tree reduce them.
-template <int NZ, bool TRI>
+template <class S, int NZ, bool TRI>
 __global__ void __launch_bounds__(256, 2)
-    gram_herm_kernel(const __grid_constant__ ColListT<float2> Z, int64_t len, unsigned m, double2 *__restrict__ work,
+    gram_herm_kernel(const __grid_constant__ ColListT<S> Z, int64_t len, unsigned m, double2 *__restrict__ work,
                      double2 *__restrict__ out, int ldo)
 {
     constexpr int NP = NZ * (NZ + 1) / 2;
@@ -1663,7 +1702,7 @@ __global__ void __launch_bounds__(256, 2)
     double ar[NP], ai[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) ar[k] = ai[k] = 0.0;
-    const float2 *zc[NZ];
+    const S *zc[NZ];
 #pragma unroll
     for (int j = 0; j < NZ; ++j) zc[j] = Z.a[j];
     // upper half: the sums are doubled at the end, so a diagonal row enters by half
@@ -1683,11 +1722,11 @@ __global__ void __launch_bounds__(256, 2)
             has0 = tri_row((unsigned)r0, m, ra, w0);
             has1 = has1 && tri_row((unsigned)r1, m, r1, w1);
         }
-        float2 z0[NZ], z1[NZ];
+        S z0[NZ], z1[NZ];
 #pragma unroll
         for (int j = 0; j < NZ; ++j) {
-            z0[j] = has0 ? __ldg(zc[j] + ra) : make_float2(0.f, 0.f);
-            z1[j] = has1 ? __ldg(zc[j] + r1) : make_float2(0.f, 0.f);
+            z0[j] = has0 ? __ldg(zc[j] + ra) : S{0, 0};
+            z1[j] = has1 ? __ldg(zc[j] + r1) : S{0, 0};
         }
         double xr[NZ], xi[NZ];
 #pragma unroll
@@ -1743,42 +1782,55 @@ __global__ void __launch_bounds__(256, 2)
     }
 }
 
-template <int NZ, bool TRI>
-cudaError_t gram_herm_go(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
+template <class S, int NZ, bool TRI>
+cudaError_t gram_herm_go(const ColListT<S> &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
                          int64_t tri)
 {
     // partials: NZ (NZ + 1) / 2 per block must fit the reduction scratch (kSmallBlocks * 32)
     if constexpr (TRI) len = tri_slots(tri);
     const int64_t want = (len + 511) / 512;
     const int blocks = (int)std::max<int64_t>(
-        1, std::min<int64_t>(want, std::min(wave_blocks<gram_herm_kernel<NZ, TRI>>(), kSmallBlocks)));
-    gram_herm_kernel<NZ, TRI><<<blocks, 256, 0, st>>>(Z, len, (unsigned)tri, work, out, ldo);
+        1, std::min<int64_t>(want, std::min(wave_blocks<gram_herm_kernel<S, NZ, TRI>>(), kSmallBlocks)));
+    gram_herm_kernel<S, NZ, TRI><<<blocks, 256, 0, st>>>(Z, len, (unsigned)tri, work, out, ldo);
     count_launch();
     return cudaGetLastError();
 }
 
-template <int NZ>
-cudaError_t gram_herm_go(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
+template <class S, int NZ>
+cudaError_t gram_herm_go(const ColListT<S> &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
                          int64_t tri)
 {
-    return tri ? gram_herm_go<NZ, true>(Z, len, out, ldo, work, st, tri)
-               : gram_herm_go<NZ, false>(Z, len, out, ldo, work, st, 0);
+    return tri ? gram_herm_go<S, NZ, true>(Z, len, out, ldo, work, st, tri)
+               : gram_herm_go<S, NZ, false>(Z, len, out, ldo, work, st, 0);
 }
 }  // namespace
+
+template <class S>
+static cudaError_t gram_herm_any(const ColListT<S> &Z, int64_t len, double2 *out, int ldo, double2 *work,
+                                 cudaStream_t st, int64_t tri)
+{
+    if (len < 1) return cudaErrorInvalidValue;
+    switch (Z.n) {
+    case 2: return gram_herm_go<S, 2>(Z, len, out, ldo, work, st, tri);
+    case 3: return gram_herm_go<S, 3>(Z, len, out, ldo, work, st, tri);
+    case 4: return gram_herm_go<S, 4>(Z, len, out, ldo, work, st, tri);
+    case 5: return gram_herm_go<S, 5>(Z, len, out, ldo, work, st, tri);
+    case 6: return gram_herm_go<S, 6>(Z, len, out, ldo, work, st, tri);
+    case 7: return gram_herm_go<S, 7>(Z, len, out, ldo, work, st, tri);
+    default: return cudaErrorInvalidValue;
+    }
+}
 
 cudaError_t gram_herm_launch(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
                              int64_t tri)
 {
-    if (len < 1) return cudaErrorInvalidValue;
-    switch (Z.n) {
-    case 2: return gram_herm_go<2>(Z, len, out, ldo, work, st, tri);
-    case 3: return gram_herm_go<3>(Z, len, out, ldo, work, st, tri);
-    case 4: return gram_herm_go<4>(Z, len, out, ldo, work, st, tri);
-    case 5: return gram_herm_go<5>(Z, len, out, ldo, work, st, tri);
-    case 6: return gram_herm_go<6>(Z, len, out, ldo, work, st, tri);
-    case 7: return gram_herm_go<7>(Z, len, out, ldo, work, st, tri);
-    default: return cudaErrorInvalidValue;
-    }
+    return gram_herm_any(Z, len, out, ldo, work, st, tri);
+}
+
+cudaError_t gram_herm_launch(const ColList &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
+                             int64_t tri)
+{
+    return gram_herm_any(Z, len, out, ldo, work, st, tri);
 }
 
 template <int NC>
@@ -1984,70 +2036,65 @@ cudaError_t gs_pass2_launch(const float2 *const *qp, const float2 *const *vp, in
 // column-major, ld nz), with D = sqrt(diag(G[1:,1:])), solves
 // (D^-1 G[1:,1:] D^-1 + 1e-13 I) y = D^-1 G[1:,0] by Cholesky and returns
 // a = D^-1 y (nq values).  Flag 8 if the system is not positive definite.
-__global__ void small_sstep_solve(const double2 *__restrict__ G, int nz, double2 *__restrict__ a, int *flag)
+__global__ void __launch_bounds__(64)
+    small_sstep_solve(const double2 *__restrict__ G, int nz, double2 *__restrict__ a, int *flag)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int n = nz - 1;
-    double d[8];
-    double2 R[8 * 8], y[8];
-    for (int i = 0; i < n; ++i) {
-        const double v = G[(i + 1) + nz * (i + 1)].x;
-        if (!(v > 0.0) || !isfinite(v)) {
-            raise_flag(flag, 8);
-            return;
-        }
-        d[i] = sqrt(v);
+    __shared__ double2 R[8 * 8], y[8];
+    __shared__ double d[8], inv[8];
+    const int n = nz - 1, t = threadIdx.x;
+    double v = 1.0;
+    if (t < n) {
+        v = G[(t + 1) + nz * (t + 1)].x;
+        d[t] = 1.0 / sqrt(v);
     }
-    // Cholesky of the scaled, regularised Gram: Gs = R^H R (R upper)
-    for (int j = 0; j < n; ++j) {
-        double dj = G[(j + 1) + nz * (j + 1)].x / (d[j] * d[j]) + 1e-13;
-        for (int i = 0; i < j; ++i) dj -= R[i + 8 * j].x * R[i + 8 * j].x + R[i + 8 * j].y * R[i + 8 * j].y;
-        if (!(dj > 0.0) || !isfinite(dj)) {
-            raise_flag(flag, 8);
-            return;
-        }
-        const double rjj = sqrt(dj);
-        R[j + 8 * j] = make_double2(rjj, 0.0);
-        for (int l = j + 1; l < n; ++l) {
-            const double2 g = G[(j + 1) + nz * (l + 1)];
-            double2 t = make_double2(g.x / (d[j] * d[l]), g.y / (d[j] * d[l]));
-            for (int i = 0; i < j; ++i) {  // t -= conj(R(i,j)) R(i,l)
-                const double2 p = R[i + 8 * j], q = R[i + 8 * l];
-                t.x -= p.x * q.x + p.y * q.y;
-                t.y -= p.x * q.y - p.y * q.x;
-            }
-            R[j + 8 * l] = make_double2(t.x / rjj, t.y / rjj);
-        }
+    if (__syncthreads_or(!(v > 0.0) || !isfinite(v))) {
+        if (t == 0) raise_flag(flag, 8);
+        return;
     }
-    // R^H y = D^-1 G[1:, 0] (forward), then R x = y (back)
-    for (int i = 0; i < n; ++i) {
-        const double2 g = G[(i + 1) + nz * 0];
-        double2 t = make_double2(g.x / d[i], g.y / d[i]);
-        for (int l = 0; l < i; ++l) {  // t -= conj(R(l,i)) y(l)
-            const double2 p = R[l + 8 * i], q = y[l];
-            t.x -= p.x * q.x + p.y * q.y;
-            t.y -= p.x * q.y - p.y * q.x;
-        }
-        const double rii = R[i + 8 * i].x;
-        y[i] = make_double2(t.x / rii, t.y / rii);
+    if (t < n * n) {
+        const int i = t % n, j = t / n;
+        const double2 g = G[(i + 1) + nz * (j + 1)];
+        const double s = d[i] * d[j];
+        R[t] = make_double2(i == j ? g.x * s + 1e-13 : g.x * s, g.y * s);
     }
-    for (int i = n - 1; i >= 0; --i) {
-        double2 t = y[i];
-        for (int l = i + 1; l < n; ++l) {  // t -= R(i,l) x(l)
-            const double2 p = R[i + 8 * l], q = y[l];
-            t.x -= p.x * q.x - p.y * q.y;
-            t.y -= p.x * q.y + p.y * q.x;
-        }
-        const double rii = R[i + 8 * i].x;
-        y[i] = make_double2(t.x / rii, t.y / rii);
+    if (t < n) {
+        const double2 g = G[t + 1];
+        y[t] = make_double2(g.x * d[t], g.y * d[t]);
     }
-    for (int i = 0; i < n; ++i) a[i] = make_double2(y[i].x / d[i], y[i].y / d[i]);
+    __syncthreads();
+    if (!block_cholesky(R, inv, n)) {
+        if (t == 0) raise_flag(flag, 8);
+        return;
+    }
+    for (int i = 0; i < n; ++i) {  // R^H y = D^-1 G[1:, 0]
+        const double2 yi = make_double2(y[i].x * inv[i], y[i].y * inv[i]);
+        __syncthreads();
+        if (t == i) y[i] = yi;
+        if (t > i && t < n) {  // y(t) -= conj(R(i,t)) y(i)
+            const double2 p = R[i + n * t];
+            y[t].x -= p.x * yi.x + p.y * yi.y;
+            y[t].y -= p.x * yi.y - p.y * yi.x;
+        }
+        __syncthreads();
+    }
+    for (int i = n - 1; i >= 0; --i) {  // R x = y
+        const double2 xi = make_double2(y[i].x * inv[i], y[i].y * inv[i]);
+        __syncthreads();
+        if (t == i) y[i] = xi;
+        if (t < i) {  // y(t) -= R(t,i) x(i)
+            const double2 p = R[t + n * i];
+            y[t].x -= p.x * xi.x - p.y * xi.y;
+            y[t].y -= p.x * xi.y + p.y * xi.x;
+        }
+        __syncthreads();
+    }
+    if (t < n) a[t] = make_double2(y[t].x * d[t], y[t].y * d[t]);
 }
 
 cudaError_t small_sstep_solve_launch(const double2 *g, int nz, double2 *a, int *flag, cudaStream_t st)
 {
     if (nz < 2 || nz > 9) return cudaErrorInvalidValue;
-    small_sstep_solve<<<1, 32, 0, st>>>(g, nz, a, flag);
+    small_sstep_solve<<<1, 64, 0, st>>>(g, nz, a, flag);
     count_launch();
     return cudaGetLastError();
 }
@@ -2063,7 +2110,7 @@ cudaError_t orth_norm_coef_launch(const double2 *g, int n, double2 *coef, int *f
 cudaError_t small_cholinv_launch(const double2 *g, int k, double2 *rinv, int *flag, cudaStream_t st)
 {
     if (k < 1 || k > 16) return cudaErrorInvalidValue;
-    small_cholinv<<<1, 32, 0, st>>>(g, k, rinv, flag);
+    small_cholinv<<<1, 64, 0, st>>>(g, k, rinv, flag);
     count_launch();
     return cudaGetLastError();
 }

@@ -148,9 +148,11 @@ cudaError_t gram_tile_launch(const ColList &L, const ColList &R, int64_t len, in
 cudaError_t gram_tile_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,
                              double2 *work, cudaStream_t st, int64_t tri);
 
-// Hermitian Gram G = Z^H Z of n <= 7 complex64 vectors (FP64 sums), all n x n
+// Hermitian Gram G = Z^H Z of 2 <= n <= 7 vectors (FP64 sums), all n x n
 // entries written to DEVICE out (column-major, ldo); work as for gram.
 cudaError_t gram_herm_launch(const ColListF &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
+                             int64_t tri = 0);
+cudaError_t gram_herm_launch(const ColList &Z, int64_t len, double2 *out, int ldo, double2 *work, cudaStream_t st,
                              int64_t tri = 0);
 
 // Y_j = beta_j * Y_j + alpha * sum_i X_i C(i,j) for j < nout (nout <= 16,

@@ -63,11 +63,16 @@ __device__ __forceinline__ void sum_partials(const double2 *work, int nblk, int 
                                              double2 *out, int ldo)
 {
     double x = 0.0, y = 0.0;
-#pragma unroll 4
-    for (int b = lane; b < nblk; b += 32) {
-        const double2 v = __ldcg(work + (int64_t)b * nout + o);
-        x += v.x;
-        y += v.y;
+    for (int b = lane; b < nblk; b += 32 * 10) {  // all of 296 CTAs' partials in flight
+        double2 v[10];
+#pragma unroll
+        for (int u = 0; u < 10; ++u)
+            v[u] = b + 32 * u < nblk ? __ldcg(work + (int64_t)(b + 32 * u) * nout + o) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 10; ++u) {
+            x += v[u].x;
+            y += v[u].y;
+        }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
