@@ -17,6 +17,7 @@
 // most 40 columns) computes in FP32.
 #include "de_internal.h"
 #include "de_kernels.h"
+#include "pdl.h"
 #include "tri.h"
 
 #include <cuda.h>
@@ -97,6 +98,7 @@ __device__ __forceinline__ double2 col_elem(const ColListT<S> &L, int c, int64_t
 __global__ void __launch_bounds__(256)
     gram_reduce(const double2 *__restrict__ work, int nblk, int nl, int nr, double2 *__restrict__ out, int ldo)
 {
+    pdl_enter();
     __shared__ double2 acc[32][8];
     const int k = threadIdx.x & 7, g = threadIdx.x >> 3, o = blockIdx.x * 8 + k;
     const int nout = nl * nr;
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(256)
     update_kernel(const __grid_constant__ UpdListT<SI, SO> U, const double2 *__restrict__ C, int ldc,
                   int64_t len)
 {
+    pdl_enter();
     using T = typename UpdArith<SI, SO>::T;
     using T2 = typename UpdArith<SI, SO>::T2;
     extern __shared__ __align__(16) unsigned char upd_sm[];
@@ -223,6 +226,7 @@ template <int NC>
 __global__ void __launch_bounds__(256, 3)
     update_col(const __grid_constant__ UpdListT<double2, double2> U, const double2 *__restrict__ C, int64_t len)
 {
+    pdl_enter();
     __shared__ double2 cs[NC];
     if (threadIdx.x < NC) cs[threadIdx.x] = cmul(U.alpha, C[threadIdx.x]);
     __syncthreads();
@@ -267,9 +271,7 @@ cudaError_t update_go(const UpdListT<SI, SO> &U, const double2 *c, int ldc, int6
     const size_t smem = (size_t)U.nin * NOUT * sizeof(typename UpdArith<SI, SO>::T2);
     const int64_t want = (len + 255) / 256;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, 148 * 8));
-    update_kernel<SI, SO, NOUT><<<blocks, 256, smem, st>>>(U, c, ldc, len);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(update_kernel<SI, SO, NOUT>, blocks, 256, smem, st, U, c, ldc, len);
 }
 
 // ---------------------------------------------------------------- small
@@ -283,6 +285,7 @@ struct PtrPack {
 __global__ void axpc_kernel(const __grid_constant__ PtrPack P, double2 s, const double2 *c_dev,
                             int64_t len)
 {
+    pdl_enter();
     const int j = blockIdx.y;
     double2 c = c_dev ? c_dev[j] : make_double2(1.0, 0.0);
     const double2 sc = cmul(s, c);
@@ -297,6 +300,7 @@ __global__ void axpc_kernel(const __grid_constant__ PtrPack P, double2 s, const 
 __global__ void axpc_f32_kernel(float2 *__restrict__ out, const double2 *__restrict__ a,
                                 const double2 *__restrict__ b, double2 s, const double2 *c_dev, int64_t len)
 {
+    pdl_enter();
     const double2 c = c_dev ? c_dev[0] : make_double2(1.0, 0.0);
     const double2 sc = cmul(s, c);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -311,6 +315,7 @@ template <class S>
 __global__ void axpy_kernel(S *__restrict__ out, const S *__restrict__ a, const S *__restrict__ b, double2 s,
                             int64_t n)
 {
+    pdl_enter();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
         const double2 av = ldp(a + r), bv = ldp(b + r);
@@ -320,6 +325,7 @@ __global__ void axpy_kernel(S *__restrict__ out, const S *__restrict__ a, const 
 
 __global__ void scale_kernel(const __grid_constant__ PtrPack P, const double2 *c_dev, int64_t len)
 {
+    pdl_enter();
     const int j = blockIdx.y;
     const double2 c = c_dev[j];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -331,6 +337,7 @@ template <bool TRI>
 __global__ void dotdiag_partial(const __grid_constant__ PtrPack P, int64_t len, unsigned m, int herm,
                                 double2 *__restrict__ work)
 {
+    pdl_enter();
     const int j = blockIdx.y;
     double sr = 0.0, si = 0.0;
     const double sg = herm ? -1.0 : 1.0;
@@ -380,6 +387,7 @@ __global__ void dotdiag_partial(const __grid_constant__ PtrPack P, int64_t len, 
 __global__ void __launch_bounds__(256)
     dotdiag_reduce(const double2 *__restrict__ work, int nblk, int n, double2 *__restrict__ out)
 {
+    pdl_enter();
     __shared__ double2 acc[8];
     const int j = blockIdx.x;
     double sr = 0.0, si = 0.0;
@@ -407,6 +415,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void inv_sqrt_abs_kernel(const double2 *d, double2 *c, int n)
 {
+    pdl_enter();
     const int j = threadIdx.x;
     if (j < n) {
         const double a = sqrt(hypot(d[j].x, d[j].y));
@@ -621,6 +630,7 @@ __global__ void __launch_bounds__(256, 2)
     gram_col(const __grid_constant__ ColListT<double2> L, const double2 *__restrict__ b, int64_t len, unsigned m, int herm,
              double2 *__restrict__ work, double2 *__restrict__ out)
 {
+    pdl_enter();
     constexpr int U = 2;
     const double2 *col[NC];
 #pragma unroll
@@ -865,8 +875,6 @@ __device__ __forceinline__ void raise_flag(int *flag, int bit)
     atomicCAS(flag + 1, 0, bit);
 }
 
-// Upper Cholesky R of the Hermitian G (upper triangle read, as zpotrf 'U')
-// and R^{-1}.  flag |= 1 on breakdown, 2 when G is all zero.
 // Coefficients that orthogonalise one column b against orthonormal columns
 // Q (n of them) and normalise it, from g = [Q^H b; b^H b]: with |w|^2 =
 // b^H b - |Q^H b|^2 (Pythagoras), coef = [-(Q^H b)/|w|; 1/|w|], so that
@@ -874,6 +882,7 @@ __device__ __forceinline__ void raise_flag(int *flag, int bit)
 // a cholQR breakdown does, and leaves b unchanged.
 __global__ void orth_norm_coef(const double2 *__restrict__ g, int n, double2 *__restrict__ coef, int *flag)
 {
+    pdl_enter();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const double bb = g[n].x;
     double w2 = bb;
@@ -923,9 +932,12 @@ __device__ __forceinline__ bool block_cholesky(double2 *A, double *inv, int k)
     return true;
 }
 
+// Upper Cholesky R of the Hermitian G (upper triangle read, as zpotrf 'U')
+// and R^{-1}.  flag |= 1 on breakdown, 2 when G is all zero.
 __global__ void __launch_bounds__(64)
     small_cholinv(const double2 *__restrict__ G, int k, double2 *__restrict__ Rinv, int *flag)
 {
+    pdl_enter();
     __shared__ double2 R[16 * 16], X[16 * 16];
     __shared__ double inv[16];
     bool nonzero = false;
@@ -961,6 +973,7 @@ __global__ void __launch_bounds__(256)
     small_block_coef(const double2 *__restrict__ g1, const double2 *__restrict__ g2, int m, int k,
                      const double2 *__restrict__ r1, const double2 *__restrict__ r2, double2 *__restrict__ c)
 {
+    pdl_enter();
     __shared__ double2 w[16 * 16];
     if ((int)threadIdx.x < k * k) {
         const int i = threadIdx.x % k, j = threadIdx.x / k;
@@ -1004,6 +1017,7 @@ __global__ void small_hsqrt1(const double2 *__restrict__ g, double2 *__restrict_
 // flag |= 4 when any |T - I| > 1e-10.
 __global__ void small_ortho_check(const double2 *__restrict__ t, int k, double tol, int *flag)
 {
+    pdl_enter();
     const int o = threadIdx.x;
     if (o < k * k) {
         const int i = o % k, j = o / k;
@@ -1094,6 +1108,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void cvt_c2f_kernel(const double2 *__restrict__ x, float2 *__restrict__ y, int64_t n)
 {
+    pdl_enter();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const double2 v = x[i];
@@ -1389,6 +1404,7 @@ __global__ void __launch_bounds__(512)
     gram_tc(const __grid_constant__ ColListT<S> L, const __grid_constant__ ColListT<S> R, int64_t len, int64_t chunk,
             unsigned m, int herm, int wm, int wn, int rg, double2 *__restrict__ work)
 {
+    pdl_enter();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per = wm * wn;
     const int g = warp / per, wt = warp - g * per;
@@ -1536,14 +1552,11 @@ static cudaError_t gram_tc_go(const ColListT<S> &L, const ColListT<S> &R, int64_
     int64_t chunk = (len + nblk - 1) / nblk;
     chunk = (chunk + 3) / 4 * 4;
     work += 1;
-    gram_tc<S, MTW, NTW, KM8, TRI><<<nblk, threads, smem, st>>>(L, R, len, chunk, (unsigned)tri, herm, wm, wn, rg, work);
-    count_launch();
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = pdl_launch(gram_tc<S, MTW, NTW, KM8, TRI>, nblk, threads, smem, st,
+                      L, R, len, chunk, (unsigned)tri, herm, wm, wn, rg, work);
     if (e != cudaSuccess) return e;
     const int nout = L.n * R.n;
-    gram_reduce<<<(nout + 7) / 8, 256, 0, st>>>(work, nblk, L.n, R.n, out, ldo);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(gram_reduce, (nout + 7) / 8, 256, 0, st, work, nblk, L.n, R.n, out, ldo);
 }
 
 template <int NC, bool SELF>
@@ -1553,13 +1566,10 @@ static cudaError_t gram_col_go(const ColList &L, const double2 *b, int64_t len, 
     if (tri) {
         len = tri_slots(tri);
         const int blocks = fused_blocks<gram_col<NC, SELF, true>>((len + 1) / 2, NC);
-        gram_col<NC, SELF, true><<<blocks, 256, 0, st>>>(L, b, len, (unsigned)tri, herm, work, out);
-    } else {
-        const int blocks = fused_blocks<gram_col<NC, SELF, false>>((len + 1) / 2, NC);
-        gram_col<NC, SELF, false><<<blocks, 256, 0, st>>>(L, b, len, 0u, herm, work, out);
+        return pdl_launch(gram_col<NC, SELF, true>, blocks, 256, 0, st, L, b, len, (unsigned)tri, herm, work, out);
     }
-    count_launch();
-    return cudaGetLastError();
+    const int blocks = fused_blocks<gram_col<NC, SELF, false>>((len + 1) / 2, NC);
+    return pdl_launch(gram_col<NC, SELF, false>, blocks, 256, 0, st, L, b, len, 0u, herm, work, out);
 }
 
 // L unshifted, 2 <= L.n <= 9, one unshifted column in R
@@ -1697,6 +1707,7 @@ __global__ void __launch_bounds__(256, 2)
     gram_herm_kernel(const __grid_constant__ ColListT<S> Z, int64_t len, unsigned m, double2 *__restrict__ work,
                      double2 *__restrict__ out, int ldo)
 {
+    pdl_enter();
     constexpr int NP = NZ * (NZ + 1) / 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double ar[NP], ai[NP];
@@ -1791,9 +1802,7 @@ cudaError_t gram_herm_go(const ColListT<S> &Z, int64_t len, double2 *out, int ld
     const int64_t want = (len + 511) / 512;
     const int blocks = (int)std::max<int64_t>(
         1, std::min<int64_t>(want, std::min(wave_blocks<gram_herm_kernel<S, NZ, TRI>>(), kSmallBlocks)));
-    gram_herm_kernel<S, NZ, TRI><<<blocks, 256, 0, st>>>(Z, len, (unsigned)tri, work, out, ldo);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(gram_herm_kernel<S, NZ, TRI>, blocks, 256, 0, st, Z, len, (unsigned)tri, work, out, ldo);
 }
 
 template <class S, int NZ>
@@ -1837,9 +1846,7 @@ template <int NC>
 static cudaError_t update_col_go(const UpdList &U, const double2 *c_dev, int64_t len, cudaStream_t st)
 {
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((len + 511) / 512, wave_blocks<update_col<NC>>()));
-    update_col<NC><<<blocks, 256, 0, st>>>(U, c_dev, len);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(update_col<NC>, blocks, 256, 0, st, U, c_dev, len);
 }
 
 template <class SI, class SO>
@@ -1893,34 +1900,26 @@ cudaError_t axpc_launch(double2 *const *out, const double2 *const *a, const doub
         P.a[j] = a[j];
         P.b[j] = b[j];
     }
-    axpc_kernel<<<dim3(stream_blocks(len) / n + 1, n), 256, 0, st>>>(P, s, c_dev, len);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(axpc_kernel, dim3(stream_blocks(len) / n + 1, n), 256, 0, st, P, s, c_dev, len);
 }
 
 cudaError_t axpc_f32_launch(float2 *out, const double2 *a, const double2 *b, double2 s, const double2 *c_dev,
                             int64_t len, cudaStream_t st)
 {
     if (len < 1) return cudaErrorInvalidValue;
-    axpc_f32_kernel<<<stream_blocks(len) * 2, 256, 0, st>>>(out, a, b, s, c_dev, len);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(axpc_f32_kernel, stream_blocks(len) * 2, 256, 0, st, out, a, b, s, c_dev, len);
 }
 
 cudaError_t axpy_launch(double2 *out, const double2 *a, const double2 *b, double2 s, int64_t n, cudaStream_t st)
 {
     if (n < 1) return cudaErrorInvalidValue;
-    axpy_kernel<double2><<<stream_blocks(n) * 2, 256, 0, st>>>(out, a, b, s, n);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(axpy_kernel<double2>, stream_blocks(n) * 2, 256, 0, st, out, a, b, s, n);
 }
 
 cudaError_t axpy_launch(float2 *out, const float2 *a, const float2 *b, double2 s, int64_t n, cudaStream_t st)
 {
     if (n < 1) return cudaErrorInvalidValue;
-    axpy_kernel<float2><<<stream_blocks(n) * 2, 256, 0, st>>>(out, a, b, s, n);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(axpy_kernel<float2>, stream_blocks(n) * 2, 256, 0, st, out, a, b, s, n);
 }
 
 cudaError_t scale_cols_launch(double2 *const *x, int n, const double2 *c_dev, int64_t len,
@@ -1929,9 +1928,7 @@ cudaError_t scale_cols_launch(double2 *const *x, int n, const double2 *c_dev, in
     if (n < 1 || n > 64) return cudaErrorInvalidValue;
     PtrPack P{};
     for (int j = 0; j < n; ++j) P.out[j] = x[j];
-    scale_kernel<<<dim3(stream_blocks(len) / n + 1, n), 256, 0, st>>>(P, c_dev, len);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(scale_kernel, dim3(stream_blocks(len) / n + 1, n), 256, 0, st, P, c_dev, len);
 }
 
 int64_t dotdiag_work_elems(int n, int64_t len)
@@ -1952,14 +1949,10 @@ cudaError_t dotdiag_launch(const double2 *const *a, const double2 *const *b, int
     }
     work += 1;
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((len + 255) / 256, std::max(1, 296 / n)));
-    if (tri) dotdiag_partial<true><<<dim3(nblk, n), 256, 0, st>>>(P, len, (unsigned)tri, herm, work);
-    else dotdiag_partial<false><<<dim3(nblk, n), 256, 0, st>>>(P, len, 0u, herm, work);
-    count_launch();
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = tri ? pdl_launch(dotdiag_partial<true>, dim3(nblk, n), 256, 0, st, P, len, (unsigned)tri, herm, work)
+                        : pdl_launch(dotdiag_partial<false>, dim3(nblk, n), 256, 0, st, P, len, 0u, herm, work);
     if (e != cudaSuccess) return e;
-    dotdiag_reduce<<<n, 256, 0, st>>>(work, nblk, n, out);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(dotdiag_reduce, n, 256, 0, st, work, nblk, n, out);
 }
 
 template <class S>
@@ -2039,6 +2032,7 @@ cudaError_t gs_pass2_launch(const float2 *const *qp, const float2 *const *vp, in
 __global__ void __launch_bounds__(64)
     small_sstep_solve(const double2 *__restrict__ G, int nz, double2 *__restrict__ a, int *flag)
 {
+    pdl_enter();
     __shared__ double2 R[8 * 8], y[8];
     __shared__ double d[8], inv[8];
     const int n = nz - 1, t = threadIdx.x;
@@ -2094,34 +2088,26 @@ __global__ void __launch_bounds__(64)
 cudaError_t small_sstep_solve_launch(const double2 *g, int nz, double2 *a, int *flag, cudaStream_t st)
 {
     if (nz < 2 || nz > 9) return cudaErrorInvalidValue;
-    small_sstep_solve<<<1, 64, 0, st>>>(g, nz, a, flag);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(small_sstep_solve, 1, 64, 0, st, g, nz, a, flag);
 }
 
 cudaError_t orth_norm_coef_launch(const double2 *g, int n, double2 *coef, int *flag, cudaStream_t st)
 {
     if (n < 0 || n > 127) return cudaErrorInvalidValue;
-    orth_norm_coef<<<1, 32, 0, st>>>(g, n, coef, flag);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(orth_norm_coef, 1, 32, 0, st, g, n, coef, flag);
 }
 
 cudaError_t small_cholinv_launch(const double2 *g, int k, double2 *rinv, int *flag, cudaStream_t st)
 {
     if (k < 1 || k > 16) return cudaErrorInvalidValue;
-    small_cholinv<<<1, 64, 0, st>>>(g, k, rinv, flag);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(small_cholinv, 1, 64, 0, st, g, k, rinv, flag);
 }
 
 cudaError_t small_block_coef_launch(const double2 *g1, const double2 *g2, int m, int k, const double2 *r1,
                                     const double2 *r2, double2 *c, cudaStream_t st)
 {
     if (m < 0 || k < 1 || k > 16) return cudaErrorInvalidValue;
-    small_block_coef<<<1, 256, 0, st>>>(g1, g2, m, k, r1, r2, c);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(small_block_coef, 1, 256, 0, st, g1, g2, m, k, r1, r2, c);
 }
 
 cudaError_t small_hsqrt1_launch(const double2 *g, double2 *ginvh, double2 *gsq, int *flag, cudaStream_t st)
@@ -2134,9 +2120,7 @@ cudaError_t small_hsqrt1_launch(const double2 *g, double2 *ginvh, double2 *gsq, 
 cudaError_t small_ortho_check_launch(const double2 *t, int k, int *flag, cudaStream_t st, double tol)
 {
     if (k < 1 || k > 16) return cudaErrorInvalidValue;
-    small_ortho_check<<<1, 256, 0, st>>>(t, k, tol, flag);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(small_ortho_check, 1, 256, 0, st, t, k, tol, flag);
 }
 
 cudaError_t small_gemm_launch(const double2 *a, const double2 *b, double2 *c, int m, int k, int n, cudaStream_t st)
@@ -2150,9 +2134,7 @@ cudaError_t small_gemm_launch(const double2 *a, const double2 *b, double2 *c, in
 cudaError_t inv_sqrt_abs_launch(const double2 *d, double2 *c, int n, cudaStream_t st)
 {
     if (n < 1 || n > 64) return cudaErrorInvalidValue;
-    inv_sqrt_abs_kernel<<<1, 64, 0, st>>>(d, c, n);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(inv_sqrt_abs_kernel, 1, 64, 0, st, d, c, n);
 }
 
 cudaError_t update_exch_launch(const float2 *const *z, int nz, const double2 *coef, double2 *y, int64_t m, double s,
@@ -2182,9 +2164,7 @@ cudaError_t exch_dot_launch(const double2 *x, int64_t m, double2 *out, double2 *
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    dotdiag_reduce<<<1, 256, 0, st>>>(work + 1, (int)(t * t), 1, out);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(dotdiag_reduce, 1, 256, 0, st, work + 1, (int)(t * t), 1, out);
 }
 
 cudaError_t exch_project_launch(double2 *x, int64_t m, double s, cudaStream_t st)
@@ -2206,9 +2186,7 @@ cudaError_t refl_corr_launch(const double2 *x, int nn, double2 *out, double2 *wo
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    dotdiag_reduce<<<8, 256, 0, st>>>(work + 1, blocks, 8, out);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(dotdiag_reduce, 8, 256, 0, st, work + 1, blocks, 8, out);
 }
 
 cudaError_t refl_project_launch(double2 *x, int nn, unsigned keep, cudaStream_t st)
@@ -2223,9 +2201,7 @@ cudaError_t refl_project_launch(double2 *x, int nn, unsigned keep, cudaStream_t 
 cudaError_t to_f32_launch(const double2 *x, float2 *y, int64_t n, cudaStream_t st)
 {
     if (n < 1) return cudaErrorInvalidValue;
-    cvt_c2f_kernel<<<stream_blocks(n) * 2, 256, 0, st>>>(x, y, n);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(cvt_c2f_kernel, stream_blocks(n) * 2, 256, 0, st, x, y, n);
 }
 
 cudaError_t to_f32_launch(const double *x, float *y, int64_t n, cudaStream_t st)

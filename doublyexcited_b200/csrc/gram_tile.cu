@@ -22,6 +22,7 @@
 // complex64 (1.8 M rows): 10 x 12 502 -> 196, 20 x 24 1259 -> 737.  The shifted
 // 8 x 16 projection stays on gram_tc's one-load form (294 us against 446).
 #include "de_kernels.h"
+#include "pdl.h"
 #include "tri.h"
 
 #include <algorithm>
@@ -87,6 +88,7 @@ __device__ __forceinline__ void sum_partials(const double2 *work, int nblk, int 
 template <class S, int RT, bool TRI>
 __global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_constant__ GramTileArgs<S> a)
 {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char gt_smem[];
     S *ring = reinterpret_cast<S *>(gt_smem);  // [stage][slot][RT]
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nt = blockDim.x;
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_con
 __global__ void __launch_bounds__(256)
     gram_tile_reduce(const double2 *__restrict__ work, int nblk, int nl, int nr, double2 *__restrict__ out, int ldo)
 {
+    pdl_enter();
     const int o = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (o < nl * nr) sum_partials(work, nblk, nl, nl * nr, o, threadIdx.x & 31, out, ldo);
 }
@@ -241,13 +244,9 @@ cudaError_t tile_launch(const GramTileArgs<S> &a, int threads, size_t smem, cuda
     }
     // two CTAs per SM: 112 KB of shared memory and 128 registers a thread
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((a.len + RT - 1) / RT, std::min(2 * n, 296)));
-    gram_tile_kernel<S, RT, TRI><<<nblk, threads, smem, st>>>(a);
-    count_launch();
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = pdl_launch(gram_tile_kernel<S, RT, TRI>, nblk, threads, smem, st, a);
     if (e != cudaSuccess || a.nl * a.nr <= kFusedOut) return e;
-    gram_tile_reduce<<<(a.nl * a.nr + 7) / 8, 256, 0, st>>>(a.work + 1, nblk, a.nl, a.nr, a.out, a.ldo);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(gram_tile_reduce, (a.nl * a.nr + 7) / 8, 256, 0, st, a.work + 1, nblk, a.nl, a.nr, a.out, a.ldo);
 }
 
 // One launch: L columns [l0, l0 + nl) against R columns [r0, r0 + nr), at

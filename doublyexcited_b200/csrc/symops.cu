@@ -8,6 +8,7 @@
 // and writes it and s times its transpose: n/2 + 1 vectors.  The results are
 // (anti)symmetric bit for bit, as the general update's are.
 #include "de_kernels.h"
+#include "pdl.h"
 
 #include <algorithm>
 
@@ -33,6 +34,7 @@ __global__ void __launch_bounds__(1024 / E, E == 4 ? 2 : 1)
     update_sym_kernel(const __grid_constant__ UpdListT<SI, double2> U, const double2 *__restrict__ C, int ldc, int64_t m,
                       double s)
 {
+    pdl_enter();
     constexpr int RY = 32 / E;
     extern __shared__ __align__(16) unsigned char us_smem[];
     double2 *cs = reinterpret_cast<double2 *>(us_smem);  // [nin][NOUT]
@@ -122,6 +124,7 @@ __global__ void __launch_bounds__(512)
     axpc_f32_sym_kernel(float2 *__restrict__ out, const double2 *__restrict__ a, const double2 *__restrict__ b,
                         double2 s0, const double2 *__restrict__ c_dev, int64_t m, float s)
 {
+    pdl_enter();
     constexpr int E = 2, RY = 16;
     __shared__ float2 tile[32][33];
     int bi, bj;
@@ -160,10 +163,8 @@ template <class SI, int NOUT, int E, int IC>
 cudaError_t go(const UpdListT<SI, double2> &U, const double2 *c, int ldc, int64_t m, double s, cudaStream_t st)
 {
     const int64_t t = (m + 31) / 32;
-    update_sym_kernel<SI, NOUT, E, IC><<<(unsigned)(t * (t + 1) / 2), 1024 / E, (size_t)U.nin * NOUT * sizeof(double2),
-                                         st>>>(U, c, ldc, m, s);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(update_sym_kernel<SI, NOUT, E, IC>, (unsigned)(t * (t + 1) / 2), 1024 / E,
+                      (size_t)U.nin * NOUT * sizeof(double2), st, U, c, ldc, m, s);
 }
 
 template <class SI>
@@ -199,9 +200,7 @@ cudaError_t axpc_f32_sym_launch(float2 *out, const double2 *a, const double2 *b,
 {
     if (!sym_rows_supported(m) || !c_dev) return cudaErrorInvalidValue;
     const int64_t t = (m + 31) / 32;
-    axpc_f32_sym_kernel<<<(unsigned)(t * (t + 1) / 2), 512, 0, st>>>(out, a, b, s0, c_dev, m, (float)s);
-    count_launch();
-    return cudaGetLastError();
+    return pdl_launch(axpc_f32_sym_kernel, (unsigned)(t * (t + 1) / 2), 512, 0, st, out, a, b, s0, c_dev, m, (float)s);
 }
 
 }  // namespace de
