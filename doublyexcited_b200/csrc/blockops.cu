@@ -932,6 +932,24 @@ __device__ __forceinline__ bool block_cholesky(double2 *A, double *inv, int k)
     return true;
 }
 
+// X = R^-1 of the upper factor of block_cholesky, a column per thread by back
+// substitution; X is zero below the diagonal on entry.
+__device__ __forceinline__ void block_upper_inverse(const double2 *R, const double *inv, double2 *X, int k)
+{
+    if ((int)threadIdx.x < k) {
+        const int j = threadIdx.x;
+        for (int i = j; i >= 0; --i) {
+            double2 s = make_double2(i == j ? 1.0 : 0.0, 0.0);
+            for (int l = i + 1; l <= j; ++l) {
+                const double2 a = R[i + k * l], b = X[l + k * j];
+                s.x -= a.x * b.x - a.y * b.y;
+                s.y -= a.x * b.y + a.y * b.x;
+            }
+            X[i + k * j] = make_double2(s.x * inv[i], s.y * inv[i]);
+        }
+    }
+}
+
 // Upper Cholesky R of the Hermitian G (upper triangle read, as zpotrf 'U')
 // and R^{-1}.  flag |= 1 on breakdown, 2 when G is all zero.
 __global__ void __launch_bounds__(64)
@@ -951,26 +969,72 @@ __global__ void __launch_bounds__(64)
         if (threadIdx.x == 0) raise_flag(flag, any ? 1 : 2);
         return;
     }
-    if ((int)threadIdx.x < k) {  // R x = e_j by back substitution, a column per thread
-        const int j = threadIdx.x;
-        for (int i = j; i >= 0; --i) {
-            double2 s = make_double2(i == j ? 1.0 : 0.0, 0.0);
-            for (int l = i + 1; l <= j; ++l) {
-                const double2 a = R[i + k * l], b = X[l + k * j];
-                s.x -= a.x * b.x - a.y * b.y;
-                s.y -= a.x * b.y + a.y * b.x;
-            }
-            X[i + k * j] = make_double2(s.x * inv[i], s.y * inv[i]);
-        }
-    }
+    block_upper_inverse(R, inv, X, k);
     __syncthreads();
     for (int o = threadIdx.x; o < k * k; o += blockDim.x) Rinv[o] = X[o];
 }
 
-// C = [-(G1 + G2) W; W] with W = R1^-1 R2^-1: G1, G2 m x k (ld m), the rest k x
-// k, C (m + k) x k (ld m + k), k <= 16.
+// The second Gram-Schmidt pass and the first CholQR of a block in one update:
+// with B = Q^H W (g's first m rows), |W - Q B|^2 = W^H W - B^H B (Pythagoras), so
+// the factor R needs no further Gram.  W has been through the first pass, so B is
+// of the order of its rounding and nothing cancels -- unless all of W is
+// rounding, when half of a column or more may go: then the pass is done alone (R
+// = 1) and the CholQR that follows normalises.
 __global__ void __launch_bounds__(256)
-    small_block_coef(const double2 *__restrict__ g1, const double2 *__restrict__ g2, int m, int k,
+    small_orth_chol(const double2 *__restrict__ g, int m, int k, double2 *__restrict__ rinv, double2 *__restrict__ c,
+                    int *flag)
+{
+    pdl_enter();
+    __shared__ double2 B[64 * 16], R[16 * 16], X[16 * 16];
+    __shared__ double inv[16];
+    const int ld = m + k;
+    for (int o = threadIdx.x; o < ld * k; o += blockDim.x) {
+        const int i = o % ld, j = o / ld;
+        if (i < m) B[i + m * j] = g[o];
+        else R[i - m + k * j] = g[o];
+    }
+    for (int o = threadIdx.x; o < k * k; o += blockDim.x) X[o] = make_double2(0.0, 0.0);
+    __syncthreads();
+    bool lost = false;
+    if ((int)threadIdx.x < k * k) {
+        const int i = threadIdx.x % k, j = threadIdx.x / k;
+        double2 s = R[threadIdx.x];
+        const double before = s.x;
+        for (int l = 0; l < m; ++l) {
+            const double2 p = B[l + m * i], q = B[l + m * j];
+            s.x -= p.x * q.x + p.y * q.y;
+            s.y -= p.x * q.y - p.y * q.x;
+        }
+        R[threadIdx.x] = s;
+        lost = i == j && !(s.x > 0.5 * before);
+    }
+    if (__syncthreads_or(lost)) {
+        for (int j = threadIdx.x; j < k; j += blockDim.x) X[j + k * j] = make_double2(1.0, 0.0);
+    } else {
+        if (!block_cholesky(R, inv, k)) {
+            if (threadIdx.x == 0) raise_flag(flag, 1);
+            return;
+        }
+        block_upper_inverse(R, inv, X, k);
+    }
+    __syncthreads();
+    for (int o = threadIdx.x; o < k * k; o += blockDim.x) rinv[o] = X[o];
+    for (int o = threadIdx.x; o < ld * k; o += blockDim.x) {
+        const int i = o % ld, j = o / ld;
+        double2 s = i >= m ? X[i - m + k * j] : make_double2(0.0, 0.0);
+        for (int l = 0; i < m && l <= j; ++l) {
+            const double2 p = cmul(B[i + m * l], X[l + k * j]);
+            s.x -= p.x;
+            s.y -= p.y;
+        }
+        c[o] = s;
+    }
+}
+
+// C = [-(G1 + G2) W; W] with W = R1^-1 R2^-1: G1, G2 m x k (ld m and ld2), the
+// rest k x k, C (m + k) x k (ld m + k), k <= 16.
+__global__ void __launch_bounds__(256)
+    small_block_coef(const double2 *__restrict__ g1, const double2 *__restrict__ g2, int ld2, int m, int k,
                      const double2 *__restrict__ r1, const double2 *__restrict__ r2, double2 *__restrict__ c)
 {
     pdl_enter();
@@ -990,7 +1054,7 @@ __global__ void __launch_bounds__(256)
         const int i = o % (m + k), j = o / (m + k);
         double2 s = i >= m ? w[i - m + k * j] : make_double2(0.0, 0.0);
         for (int l = 0; i < m && l < k; ++l) {
-            const double2 a = g1[i + m * l], b = g2[i + m * l];
+            const double2 a = g1[i + m * l], b = g2[i + ld2 * l];
             const double2 p = cmul(make_double2(a.x + b.x, a.y + b.y), w[l + k * j]);
             s.x -= p.x;
             s.y -= p.y;
@@ -2103,11 +2167,18 @@ cudaError_t small_cholinv_launch(const double2 *g, int k, double2 *rinv, int *fl
     return pdl_launch(small_cholinv, 1, 64, 0, st, g, k, rinv, flag);
 }
 
-cudaError_t small_block_coef_launch(const double2 *g1, const double2 *g2, int m, int k, const double2 *r1,
+cudaError_t small_orth_chol_launch(const double2 *g, int m, int k, double2 *rinv, double2 *c, int *flag,
+                                   cudaStream_t st)
+{
+    if (m < 1 || k < 1 || k > 16 || m > 64) return cudaErrorInvalidValue;
+    return pdl_launch(small_orth_chol, 1, 256, 0, st, g, m, k, rinv, c, flag);
+}
+
+cudaError_t small_block_coef_launch(const double2 *g1, const double2 *g2, int ld2, int m, int k, const double2 *r1,
                                     const double2 *r2, double2 *c, cudaStream_t st)
 {
     if (m < 0 || k < 1 || k > 16) return cudaErrorInvalidValue;
-    return pdl_launch(small_block_coef, 1, 256, 0, st, g1, g2, m, k, r1, r2, c);
+    return pdl_launch(small_block_coef, 1, 256, 0, st, g1, g2, ld2, m, k, r1, r2, c);
 }
 
 cudaError_t small_hsqrt1_launch(const double2 *g, double2 *ginvh, double2 *gsq, int *flag, cudaStream_t st)

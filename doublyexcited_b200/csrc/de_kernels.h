@@ -179,7 +179,9 @@ cudaError_t update_launch(const UpdListT<float2, double2> &U, const double2 *c_d
 // sums and updates take the upper half.
 bool sym_rows_supported(int64_t m);
 bool update_sym_supported(int64_t m, int nout);
-cudaError_t update_sym_launch(const UpdList &U, const double2 *c_dev, int ldc, int64_t m, double s, cudaStream_t st);
+// upper: leave Y's tiles below the diagonal unwritten
+cudaError_t update_sym_launch(const UpdList &U, const double2 *c_dev, int ldc, int64_t m, double s, cudaStream_t st,
+                              bool upper = false);
 cudaError_t update_sym_launch(const UpdListT<float2, double2> &U, const double2 *c_dev, int ldc, int64_t m, double s,
                               cudaStream_t st);
 // axpc_f32_launch on such vectors (c_dev not null)
@@ -256,12 +258,17 @@ cudaError_t orth_norm_coef_launch(const double2 *g, int n, double2 *coef, int *f
 // flag bits: 1 Cholesky breakdown, 2 all-zero block, 4 orthonormality
 // self-check failed, 8 singular 1 x 1 Gram.
 cudaError_t small_cholinv_launch(const double2 *g, int k, double2 *rinv, int *flag, cudaStream_t st);
+// From g = [Q W]^H W ((m + k) x k, ld m + k; Q orthonormal, W all but orthogonal
+// to it): rinv = R^-1 of W - Q (Q^H W) = (its orthonormal factor) R, and c = [-(Q^H
+// W) R^-1; R^-1] (ld m + k), which forms that factor from [Q W].
+cudaError_t small_orth_chol_launch(const double2 *g, int m, int k, double2 *rinv, double2 *c, int *flag,
+                                   cudaStream_t st);
 // The mixed inner solve's normal equations for one column (Gram g of the
 // nz <= 9 power-basis vectors): the nz - 1 coefficients into DEVICE a.
 cudaError_t small_sstep_solve_launch(const double2 *g, int nz, double2 *a, int *flag, cudaStream_t st);
 // c = [-(g1 + g2) r1 r2; r1 r2], the coefficients of a pair block's V
 // (Solver::block_orthonormalize): g m x k, r k x k, c (m + k) x k.
-cudaError_t small_block_coef_launch(const double2 *g1, const double2 *g2, int m, int k, const double2 *r1,
+cudaError_t small_block_coef_launch(const double2 *g1, const double2 *g2, int ld2, int m, int k, const double2 *r1,
                                     const double2 *r2, double2 *c, cudaStream_t st);
 cudaError_t small_hsqrt1_launch(const double2 *g, double2 *ginvh, double2 *gsq, int *flag, cudaStream_t st);
 // |T - I| <= tol elementwise (the reference's self-check uses 1e-10).

@@ -140,7 +140,7 @@ struct Solver {
                 const int64_t nz = D * (int64_t)(order + 1) * nev;
                 DE_TRY(alloc(reinterpret_cast<double2 **>(&Z32), (nz + 1) / 2));
             } else {
-                DE_TRY(alloc(&LV, n));
+                if (nev == 1 || compat) DE_TRY(alloc(&LV, n));  // blocks keep Q alone (basic_block)
                 DE_TRY(alloc(&LQ, n));
             }
         }
@@ -152,7 +152,7 @@ struct Solver {
         DE_TRY(alloc(&dB1, 64 * 16));
         DE_TRY(alloc(&dB2, 64 * 16));
         DE_TRY(alloc(&dRinv2, 16 * 16));
-        DE_TRY(alloc(&dVC, 80 * 16));
+        DE_TRY(alloc(&dVC, 64 * 80 / 2));  // 64 columns: nq (nq + k) / 2 for nq <= 64, k <= 16
         DE_TRY(alloc(&dT, 64));
         DE_TRY(alloc(&dT2, 65));
         DE_TRY(alloc(&dRinv, 16 * 16));
@@ -221,6 +221,15 @@ struct Solver {
     {
         if (exch_mult != 0.0 && update_sym_supported(h->m, U.nout))
             return update_sym_launch(U, c, ldc, h->m, exch_mult, st);
+        return update_launch(U, c, ldc, D, st);
+    }
+    // An update whose result only Grams and updates of this kind read next:
+    // where those take the upper half, the lower one is not written.  The
+    // result's columns must be rewritten in full (update_any) before a product.
+    cudaError_t update_part(const UpdList &U, const double2 *c, int ldc)
+    {
+        if (exch_mult != 0.0 && update_sym_supported(h->m, U.nout))
+            return update_sym_launch(U, c, ldc, h->m, exch_mult, st, true);
         return update_launch(U, c, ldc, D, st);
     }
 
@@ -610,8 +619,8 @@ struct Solver {
     // reference's column-by-column two-pass Gram-Schmidt (myhgramschmidt_many)
     // to rounding.  V only follows Q: its four updates have one product,
     // V_new <- (V_new - V (C_1 + C_2)) R_1^-1 R_2^-1, which is formed at the
-    // end (5 m0 + 48 vector passes a block of k = 4 became 3.5 m0 + 30 in the
-    // exchange-symmetric case).
+    // end.  For the compatibility mode, whose pairs are not q = (H - sigma) v;
+    // basic_block needs no V.
     template <class S>
     int block_orthonormalize(S *Q, S *V, int m0, int k)
     {
@@ -627,7 +636,7 @@ struct Solver {
             if (e != cudaSuccess) return cuda_error(e, "small_cholinv");
             DE_TRY(updateT(qb, k, qb, k, rs[pass], k));
         }
-        cudaError_t e = small_block_coef_launch(dB1, dB2, m0, k, dRinv, dRinv2, dVC, st);
+        cudaError_t e = small_block_coef_launch(dB1, dB2, m0, m0, k, dRinv, dRinv2, dVC, st);
         if (e != cudaSuccess) return cuda_error(e, "small_block_coef");
         return updateT(V, m0 + k, V + (int64_t)m0 * D, k, dVC, m0 + k);
     }
@@ -642,9 +651,128 @@ struct Solver {
         return DE_OK;
     }
 
+    // Y[0..nout) = beta Y + alpha sum_i X_i C(i, j) over columns of one buffer,
+    // the result's upper half at least (update_part)
+    int part(double2 *xb, int nin, double2 *yb, int nout, const double2 *c, int ldc, double alpha, double beta)
+    {
+        UpdList U{};
+        U.nin = nin;
+        U.nout = nout;
+        for (int i = 0; i < nin; ++i) U.x[i] = col(xb, i);
+        for (int j = 0; j < nout; ++j) {
+            U.y[j] = col(yb, j);
+            U.beta[j] = make_double2(beta, 0.0);
+        }
+        U.alpha = make_double2(alpha, 0.0);
+        cudaError_t e = update_part(U, c, ldc);
+        if (e != cudaSuccess) return cuda_error(e, "update");
+        return DE_OK;
+    }
+
+    // basicblocklansolve harmonic_ritz_small.F90:258-324 on a block b of k > 1
+    // columns, in place: b <- V (Q^H V_0) G^{1/2}, Q = (H - sigma) V.
+    //
+    // The reference continues each Krylov block from the vectors v: the next
+    // pair is ((H - sigma) w, w) with w = H v_i = q_i + sigma v_i.  Its sigma v_i
+    // part maps to sigma q_i, which the Gram-Schmidt against Q takes out again,
+    // so the pair ((H - sigma) q_i, q_i) gives the same block.  Then
+    // V = [V_0, Q_0, .., Q_{n-2}] times a block upper triangular matrix of the
+    // Gram-Schmidt coefficients, and V is never formed: the solution
+    // V y = b-part + sum Q_{i-1} z_i follows from y by back substitution, in
+    // the update that wrote V y before.
+    //
+    // Each new block takes the two classical passes and the two CholQRs of
+    // block_orthonormalize, pass 2 and CholQR 1 in one update
+    // (small_orth_chol): 2 m0 + 20 vector passes at k = 4 against 2.5 m0 + 50
+    // with V.  Two outer iterations at N = 5, NEV = 4: 47.8 -> 37.0 ms.
+    int basic_block(double2 *b, int k)
+    {
+        const int nq = order * k;
+        auto kmat = [&](int i) { return col(LQ, i * k); };
+        DE_TRY(inner_mult_shifted(b, LQ, k));
+        std::vector<cplx> g, ginv, gsq;
+        DE_TRY(gram_hostT(colsT(LQ, k, D), colsT(LQ, k, D), g));
+        auto t0 = clk::now();
+        DE_TRY(herm_sqrt_pair(k, g, ginv, gsq));
+        t_dense += secs(t0, clk::now());
+        std::vector<cplx> ginvh((size_t)k * k);
+        for (int j = 0; j < k; ++j)
+            for (int i = 0; i < k; ++i) ginvh[i + (size_t)k * j] = std::conj(ginv[j + (size_t)k * i]);
+        DE_TRY(upload(ginvh, dC));
+        DE_TRY(part(LQ, k, LQ, k, dC, k, 1.0, 0.0));
+        mv_ref += k;  // the self-check's product (harmonic_ritz_small.F90:221-242)
+        DE_TRY(gramT(colsT(LQ, k, D), colsT(LQ, k, D), dG, k));
+        cudaError_t e = small_ortho_check_launch(dG, k, dFlags, st, 1e-10);
+        if (e != cudaSuccess) return cuda_error(e, "small_ortho_check");
+        double2 *cf = dVC;  // the blocks' coefficients, one after the other
+        for (int io = 0; io < order; ++io) {
+            const int m0 = io * k;
+            double2 *qb = kmat(io);
+            mv_ref += k;  // H v_{io-1}, or the product checked above
+            if (io == 0) {
+                e = small_cholinv_launch(dG, k, dRinv, dFlags, st);
+                if (e != cudaSuccess) return cuda_error(e, "small_cholinv");
+                DE_TRY(part(qb, k, qb, k, dRinv, k, 1.0, 0.0));
+            } else {
+                DE_TRY(inner_mult_shifted(kmat(io - 1), qb, k));
+                DE_TRY(gramT(colsT(LQ, m0, D), colsT(qb, k, D), dB1, m0));
+                DE_TRY(part(LQ, m0, qb, k, dB1, m0, -1.0, 1.0));
+                DE_TRY(gramT(colsT(LQ, m0 + k, D), colsT(qb, k, D), dB2, m0 + k));
+                e = small_orth_chol_launch(dB2, m0, k, dRinv, dSV, dFlags, st);
+                if (e != cudaSuccess) return cuda_error(e, "small_orth_chol");
+                DE_TRY(part(LQ, m0 + k, qb, k, dSV, m0 + k, 1.0, 0.0));
+            }
+            DE_TRY(gramT(colsT(qb, k, D), colsT(qb, k, D), dG, k));
+            e = small_cholinv_launch(dG, k, dRinv2, dFlags, st);
+            if (e != cudaSuccess) return cuda_error(e, "small_cholinv");
+            // in full where a product reads it
+            if (io + 1 < order) DE_TRY(updateT(qb, k, qb, k, dRinv2, k));
+            else DE_TRY(part(qb, k, qb, k, dRinv2, k, 1.0, 0.0));
+            e = small_block_coef_launch(dB1, dB2, m0 + k, m0, k, dRinv, dRinv2, cf, st);
+            if (e != cudaSuccess) return cuda_error(e, "small_block_coef");
+            cf += (m0 + k) * k;
+        }
+        // with g1 = Q^H b and V_0 = b F, F = G^{-1/2 H} R_1^-1 R_2^-1 of block 0:
+        // y = (g1 F) G^{1/2}
+        const size_t nc = cf - dVC;
+        double2 *hc = hbuf + 2048;
+        DE_CUDA(cudaMemcpyAsync(hc, dVC, nc * sizeof(double2), cudaMemcpyDeviceToHost, st));
+        std::vector<cplx> g1;
+        DE_TRY(gram_hostT(colsT(LQ, nq, D), colsT(b, k, D), g1));
+        t0 = clk::now();
+        const cplx *cc = reinterpret_cast<const cplx *>(hc);
+        std::vector<cplx> f((size_t)k * k), fs((size_t)k * k), y((size_t)nq * k), a((size_t)nq * k), w(k);
+        for (int j = 0; j < k; ++j)
+            for (int i = 0; i < k; ++i)
+                for (int l = 0; l < k; ++l) f[i + k * j] += ginvh[i + k * l] * cc[l + k * j];
+        for (int j = 0; j < k; ++j)
+            for (int i = 0; i < k; ++i)
+                for (int l = 0; l < k; ++l) fs[i + k * j] += f[i + k * l] * gsq[l + k * j];
+        for (int j = 0; j < k; ++j)
+            for (int l = 0; l < k; ++l)
+                for (int i = 0; i < nq; ++i) y[i + nq * j] += g1[i + nq * l] * fs[l + k * j];
+        // a: rows [0, k) on b, rows [io k, (io + 1) k) on Q_{io-1}
+        for (int io = order - 1; io >= 0; --io) {
+            const int m0 = io * k, ld = m0 + k;
+            const cplx *c = io == 0 ? f.data() : cc + k * (m0 * (io + 1) / 2);
+            for (int j = 0; j < k; ++j)
+                for (int l = 0; l < k; ++l) {
+                    const cplx yl = y[m0 + l + nq * j];
+                    for (int i = 0; i < m0; ++i) y[i + nq * j] += c[i + ld * l] * yl;
+                    for (int i = 0; i < k; ++i) a[m0 + i + nq * j] += c[m0 + i + ld * l] * yl;
+                }
+        }
+        t_dense += secs(t0, clk::now());
+        DE_TRY(upload(a, dC));
+        std::vector<const double2 *> xs = cl(b, k);
+        for (int i = 0; i < nq - k; ++i) xs.push_back(col(LQ, i));
+        return update(xs, clw(b, k), dC, nq, 1.0, 0.0);
+    }
+
     // basicblocklansolve harmonic_ritz_small.F90:258-324 on block b (k
-    // columns), in place: b <- V (Q^H V_1) G^{1/2}.  S is the storage of
-    // the Krylov blocks; b is always FP64.
+    // columns), in place: b <- V (Q^H V_1) G^{1/2}: one column, or the
+    // compatibility mode's blocks.  S is the storage of the Krylov blocks; b is
+    // always FP64.
     template <class S>
     int basic(double2 *b, int k)
     {
@@ -688,9 +816,9 @@ struct Solver {
         } else {
             mv_ref += k;
         }
-        DE_TRY(gramT(colsT(Q, k, D), colsT(Q, k, D), dT, k));
+        DE_TRY(gramT(colsT(Q, k, D), colsT(Q, k, D), dG, k));
         {
-            cudaError_t e = small_ortho_check_launch(dT, k, dFlags, st, ortho_tol);
+            cudaError_t e = small_ortho_check_launch(dG, k, dFlags, st, ortho_tol);
             if (e != cudaSuccess) return cuda_error(e, "small_ortho_check");
         }
         // fast_harmritz_setup :86-158 (maxiter = M^2 never truncates a block)
@@ -1005,7 +1133,7 @@ struct Solver {
             if (s == DE_OK) s = symmetry_project(b, k);
         } else {
             s = equilibrate(b, k);
-            if (s == DE_OK) s = basic<double2>(b, k);
+            if (s == DE_OK) s = k > 1 && !compat ? basic_block(b, k) : basic<double2>(b, k);
             // Block solves (NEV > 1) keep the start block's sectors too: in
             // exact arithmetic the iteration never leaves them, but FP64
             // rounding leaks into the others, and GPLMR then converges to

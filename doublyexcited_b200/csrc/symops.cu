@@ -6,7 +6,9 @@
 // HBM-bound: a combination of n columns moves n + 1 vectors.  Here a CTA forms
 // the 32 x 32 tile at (p0, q0), p0 <= q0, from the upper halves of its inputs
 // and writes it and s times its transpose: n/2 + 1 vectors.  The results are
-// (anti)symmetric bit for bit, as the general update's are.
+// (anti)symmetric bit for bit, as the general update's are.  A block that only
+// such sums and updates read next needs its upper tiles alone (`upper`): n/2 +
+// 1/2 vectors.
 #include "de_kernels.h"
 #include "pdl.h"
 
@@ -32,7 +34,7 @@ __device__ __forceinline__ void tile_pair(int b, int &bi, int &bj)
 template <class SI, int NOUT, int E, int IC>
 __global__ void __launch_bounds__(1024 / E, E == 4 ? 2 : 1)
     update_sym_kernel(const __grid_constant__ UpdListT<SI, double2> U, const double2 *__restrict__ C, int ldc, int64_t m,
-                      double s)
+                      double s, int upper)
 {
     pdl_enter();
     constexpr int RY = 32 / E;
@@ -105,7 +107,7 @@ __global__ void __launch_bounds__(1024 / E, E == 4 ? 2 : 1)
 #pragma unroll
         for (int u = 0; u < E; ++u)
             if (in[u]) y[row[u]] = make_double2(ar[u][j], ai[u][j]);
-        if (bi == bj) continue;
+        if (bi == bj || upper) continue;
         if (j > 0) __syncthreads();
 #pragma unroll
         for (int u = 0; u < E; ++u) tile[tx][ty + RY * u] = make_double2(s * ar[u][j], s * ai[u][j]);
@@ -160,21 +162,22 @@ __global__ void __launch_bounds__(512)
 }
 
 template <class SI, int NOUT, int E, int IC>
-cudaError_t go(const UpdListT<SI, double2> &U, const double2 *c, int ldc, int64_t m, double s, cudaStream_t st)
+cudaError_t go(const UpdListT<SI, double2> &U, const double2 *c, int ldc, int64_t m, double s, bool upper, cudaStream_t st)
 {
     const int64_t t = (m + 31) / 32;
     return pdl_launch(update_sym_kernel<SI, NOUT, E, IC>, (unsigned)(t * (t + 1) / 2), 1024 / E,
-                      (size_t)U.nin * NOUT * sizeof(double2), st, U, c, ldc, m, s);
+                      (size_t)U.nin * NOUT * sizeof(double2), st, U, c, ldc, m, s, (int)upper);
 }
 
 template <class SI>
-cudaError_t any(const UpdListT<SI, double2> &U, const double2 *c, int ldc, int64_t m, double s, cudaStream_t st)
+cudaError_t any(const UpdListT<SI, double2> &U, const double2 *c, int ldc, int64_t m, double s, bool upper,
+                cudaStream_t st)
 {
     if (!update_sym_supported(m, U.nout) || U.nin < 1 || U.nin > kMaxCols) return cudaErrorInvalidValue;
-    if (U.nout <= 1) return go<SI, 1, 4, 4>(U, c, ldc, m, s, st);
-    if (U.nout <= 2) return go<SI, 2, 4, 2>(U, c, ldc, m, s, st);
-    if (U.nout <= 4) return go<SI, 4, 4, 2>(U, c, ldc, m, s, st);
-    return go<SI, 8, 2, 2>(U, c, ldc, m, s, st);
+    if (U.nout <= 1) return go<SI, 1, 4, 4>(U, c, ldc, m, s, upper, st);
+    if (U.nout <= 2) return go<SI, 2, 4, 2>(U, c, ldc, m, s, upper, st);
+    if (U.nout <= 4) return go<SI, 4, 4, 2>(U, c, ldc, m, s, upper, st);
+    return go<SI, 8, 2, 2>(U, c, ldc, m, s, upper, st);
 }
 
 }  // namespace
@@ -184,15 +187,16 @@ cudaError_t any(const UpdListT<SI, double2> &U, const double2 *c, int ldc, int64
 bool sym_rows_supported(int64_t m) { return m >= 1000 && m <= 46000; }
 bool update_sym_supported(int64_t m, int nout) { return sym_rows_supported(m) && nout >= 1 && nout <= 8; }
 
-cudaError_t update_sym_launch(const UpdList &U, const double2 *c_dev, int ldc, int64_t m, double s, cudaStream_t st)
+cudaError_t update_sym_launch(const UpdList &U, const double2 *c_dev, int ldc, int64_t m, double s, cudaStream_t st,
+                              bool upper)
 {
-    return any(U, c_dev, ldc, m, s, st);
+    return any(U, c_dev, ldc, m, s, upper, st);
 }
 
 cudaError_t update_sym_launch(const UpdListT<float2, double2> &U, const double2 *c_dev, int ldc, int64_t m, double s,
                               cudaStream_t st)
 {
-    return any(U, c_dev, ldc, m, s, st);
+    return any(U, c_dev, ldc, m, s, false, st);
 }
 
 cudaError_t axpc_f32_sym_launch(float2 *out, const double2 *a, const double2 *b, double2 s0, const double2 *c_dev,

@@ -58,3 +58,36 @@ def test_iteration_keeps_the_sector_bit_for_bit(de, oracle, precision, n, nev, s
     for j in range(nev):
         x = r.x[:, j].reshape(p.m, p.m)
         assert np.array_equal(x, s * x.T)
+
+
+# nev 2, 5 and 9: the two widths of the upper-half update and, above 8 columns,
+# the general one.  Both sides are FP64; their rounding (1e-15) is amplified by
+# the conditioning of the k x k Grams, which the self-check holds below 1e5.
+@pytest.mark.parametrize("nev,order", [(2, 6), (5, 3), (9, 2)])
+def test_block_solve_on_upper_halves(de, oracle, nev, order):
+    p = oracle.Params(n=5, delta=2.0, theta=0.3)
+    x0 = oracle.seeded_start(p, nev, 31, "singlet")
+    e = []
+    for family in ("fma", "stream"):  # the latter's products keep no sector: whole vectors
+        with de.Problem(n=5, delta=2.0, theta=0.3) as h:
+            for pass_ in (0, 1):
+                h.set_matvec_launch("c128", pass_, family, 0)
+            e.append(h.gplmr_eig(x0, -0.78, ns=1, maxit=1, tol=1e-14, max_inner_iter=order).e)
+    assert np.abs(e[0] - e[1]).max() < 1e-9
+
+
+def test_block_solve_of_an_exhausted_space(de):
+    """On 27 points a spherical singlet start reaches 24 states (the
+    orbits of point pairs under the cube's symmetries and exchange), so Krylov
+    blocks of two columns run out of them by the 12th: what Gram-Schmidt leaves of
+    the next is rounding, and more blocks do not change the solution."""
+    c = np.arange(3) - 1.0
+    r2 = (c[:, None, None] ** 2 + c[None, :, None] ** 2 + c[None, None, :] ** 2).ravel()
+    x0 = np.stack([np.outer(np.exp(-a * r2), np.exp(-b * r2)).ravel() + np.outer(np.exp(-b * r2), np.exp(-a * r2)).ravel()
+                   for a, b in ((0.3, 0.3), (0.8, 0.1))], 1).astype(complex)
+    e = []
+    for order in (20, 30):
+        with de.Problem(n=1, delta=2.0, theta=0.3) as h:
+            e.append(h.gplmr_eig(x0, -0.78, ns=1, maxit=2, tol=1e-9, max_inner_iter=order).e)
+    # the solves are exact but for the rounding the last blocks add
+    assert np.abs(e[0] - e[1]).max() < 1e-9
