@@ -662,10 +662,13 @@ __global__ void __launch_bounds__(256, 2)
             }
 #pragma unroll
             for (int i = 0; i < NC; ++i) {
-                const double ly = sg * l[u][i].y;
                 ar[i] = fma(l[u][i].x, x[u].x, ar[i]);
-                ar[i] = fma(-ly, x[u].y, ar[i]);
                 ai[i] = fma(l[u][i].x, x[u].y, ai[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < NC; ++i) {
+                const double ly = sg * l[u][i].y;
+                ar[i] = fma(-ly, x[u].y, ar[i]);
                 ai[i] = fma(ly, x[u].x, ai[i]);
             }
         }
@@ -1749,18 +1752,33 @@ __host__ __device__ constexpr int herm_j(int k)
 
 // conj(z_i) z_j of one row added to the packed sums; K walks the pairs at
 // compile time.  Products of two floats are exact in double.
-template <int NZ, int K>
-__device__ __forceinline__ void herm_acc(double (&ar)[NZ * (NZ + 1) / 2], double (&ai)[NZ * (NZ + 1) / 2],
-                                         const double (&zr)[NZ], const double (&zi)[NZ])
+template <int NZ, int K, int HALF>
+__device__ __forceinline__ void herm_half(double (&ar)[NZ * (NZ + 1) / 2], double (&ai)[NZ * (NZ + 1) / 2],
+                                          const double (&zr)[NZ], const double (&zi)[NZ])
 {
     if constexpr (K < NZ * (NZ + 1) / 2) {
         constexpr int i = herm_i<NZ>(K), j = herm_j<NZ>(K);
-        ar[K] = fma(zr[i], zr[j], ar[K]);
-        ar[K] = fma(zi[i], zi[j], ar[K]);
-        ai[K] = fma(zr[i], zi[j], ai[K]);
-        ai[K] = fma(-zi[i], zr[j], ai[K]);
-        herm_acc<NZ, K + 1>(ar, ai, zr, zi);
+        if constexpr (HALF == 0) {
+            ar[K] = fma(zr[i], zr[j], ar[K]);
+            if constexpr (i != j) ai[K] = fma(zr[i], zi[j], ai[K]);
+        } else {
+            ar[K] = fma(zi[i], zi[j], ar[K]);
+            if constexpr (i != j) ai[K] = fma(-zi[i], zr[j], ai[K]);
+        }
+        herm_half<NZ, K + 1, HALF>(ar, ai, zr, zi);
     }
+}
+
+// The two halves of every sum are NZ (NZ + 1) multiply-adds apart, so that none
+// waits for the one before it (6 complex64 columns of the upper half at N = 6:
+// 45 -> 36 us; prefetched rows at one block per SM gained nothing); a diagonal
+// sum has no imaginary part.
+template <int NZ>
+__device__ __forceinline__ void herm_acc(double (&ar)[NZ * (NZ + 1) / 2], double (&ai)[NZ * (NZ + 1) / 2],
+                                         const double (&zr)[NZ], const double (&zi)[NZ])
+{
+    herm_half<NZ, 0, 0>(ar, ai, zr, zi);
+    herm_half<NZ, 0, 1>(ar, ai, zr, zi);
 }
 
 // G = Z^H Z (n = NZ complex64 columns, FP64 sums) in one read: each thread
@@ -1810,14 +1828,14 @@ __global__ void __launch_bounds__(256, 2)
             xi[j] = z0[j].y;
         }
         if (TRI && w0 == 1.0) halve(xr, xi);
-        herm_acc<NZ, 0>(ar, ai, xr, xi);
+        herm_acc<NZ>(ar, ai, xr, xi);
 #pragma unroll
         for (int j = 0; j < NZ; ++j) {
             xr[j] = z1[j].x;
             xi[j] = z1[j].y;
         }
         if (TRI && w1 == 1.0) halve(xr, xi);
-        herm_acc<NZ, 0>(ar, ai, xr, xi);
+        herm_acc<NZ>(ar, ai, xr, xi);
     }
     __shared__ double2 wsum[8][NP];
 #pragma unroll

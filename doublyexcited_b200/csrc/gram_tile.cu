@@ -164,13 +164,19 @@ __global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_con
                     x[i].y *= w;
                 }
             }
+            // the second terms 32 multiply-adds after the first: none waits for the one before it
 #pragma unroll
             for (int i = 0; i < kTile; ++i)
 #pragma unroll
                 for (int j = 0; j < kTile; ++j) {
                     gr[i][j] = fma(l[i].x, x[j].x, gr[i][j]);
-                    gr[i][j] = fma(-l[i].y, x[j].y, gr[i][j]);
                     gi[i][j] = fma(l[i].x, x[j].y, gi[i][j]);
+                }
+#pragma unroll
+            for (int i = 0; i < kTile; ++i)
+#pragma unroll
+                for (int j = 0; j < kTile; ++j) {
+                    gr[i][j] = fma(-l[i].y, x[j].y, gr[i][j]);
                     gi[i][j] = fma(l[i].y, x[j].x, gi[i][j]);
                 }
         }

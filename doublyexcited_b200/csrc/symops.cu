@@ -76,8 +76,11 @@ __global__ void __launch_bounds__(1024 / E, E == 4 ? 2 : 1)
 #pragma unroll
         for (int j = 0; j < NOUT; ++j) {
             ar[u][j] = fma(v.x, c[j].x, ar[u][j]);
-            ar[u][j] = fma(-v.y, c[j].y, ar[u][j]);
             ai[u][j] = fma(v.x, c[j].y, ai[u][j]);
+        }
+#pragma unroll
+        for (int j = 0; j < NOUT; ++j) {
+            ar[u][j] = fma(-v.y, c[j].y, ar[u][j]);
             ai[u][j] = fma(v.y, c[j].x, ai[u][j]);
         }
     };
