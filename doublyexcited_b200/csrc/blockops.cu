@@ -1669,7 +1669,7 @@ static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t 
             return L.a[L.n - 1] == R.a[0] ? gram_col_any<true>(L, R.a[0], len, herm, out, work, st, tri)
                                           : gram_col_any<false>(L, R.a[0], len, herm, out, work, st, tri);
     }
-    if (R.n == 1 && L.n <= 32) {
+    if (R.n == 1 && L.n <= 32 && !tri) {  // these read whole vectors
         if (L.n <= 1) return gram_small_go<1, 1>(L, R, len, herm, out, ldo, work, st);
         if (L.n <= 2) return gram_small_go<2, 1>(L, R, len, herm, out, ldo, work, st);
         if (L.n <= 4) return gram_small_go<4, 1>(L, R, len, herm, out, ldo, work, st);
@@ -2013,6 +2013,12 @@ cudaError_t scale_cols_launch(double2 *const *x, int n, const double2 *c_dev, in
     return pdl_launch(scale_kernel, dim3(stream_blocks(len) / n + 1, n), 256, 0, st, P, c_dev, len);
 }
 
+cudaError_t dotdiag_reduce_launch(const double2 *work, int nblk, int n, double2 *out, cudaStream_t st)
+{
+    if (n < 1 || nblk < 1) return cudaErrorInvalidValue;
+    return pdl_launch(dotdiag_reduce, n, 256, 0, st, work, nblk, n, out);
+}
+
 int64_t dotdiag_work_elems(int n, int64_t len)
 {
     (void)len;
@@ -2034,7 +2040,7 @@ cudaError_t dotdiag_launch(const double2 *const *a, const double2 *const *b, int
     cudaError_t e = tri ? pdl_launch(dotdiag_partial<true>, dim3(nblk, n), 256, 0, st, P, len, (unsigned)tri, herm, work)
                         : pdl_launch(dotdiag_partial<false>, dim3(nblk, n), 256, 0, st, P, len, 0u, herm, work);
     if (e != cudaSuccess) return e;
-    return pdl_launch(dotdiag_reduce, n, 256, 0, st, work, nblk, n, out);
+    return dotdiag_reduce_launch(work, nblk, n, out, st);
 }
 
 template <class S>

@@ -184,6 +184,16 @@ cudaError_t update_sym_launch(const UpdList &U, const double2 *c_dev, int ldc, i
                               bool upper = false);
 cudaError_t update_sym_launch(const UpdListT<float2, double2> &U, const double2 *c_dev, int ldc, int64_t m, double s,
                               cudaStream_t st);
+// Columns x, A x (upper tiles) scaled to |x| = 1 from n2 = <x, x>, e_out = E =
+// <x, A x>, w = A x - E x in full, r2 = |w|^2; e = <x, A x> before the scaling
+// (conj: <A x, x>).  work: residual_sym_work_elems + 1.
+int64_t residual_sym_work_elems(int n, int64_t m);
+cudaError_t residual_sym_launch(double2 *const *x, double2 *const *ax, double2 *const *w, int n, const double2 *n2,
+                                const double2 *e, int conj, double2 *e_out, double2 *r2, int64_t m, double s,
+                                double2 *work, cudaStream_t st);
+cudaError_t residual_sym_launch(double2 *const *x, double2 *const *ax, float2 *const *w, int n, const double2 *n2,
+                                const double2 *e, int conj, double2 *e_out, double2 *r2, int64_t m, double s,
+                                double2 *work, cudaStream_t st);
 // axpc_f32_launch on such vectors (c_dev not null)
 cudaError_t axpc_f32_sym_launch(float2 *out, const double2 *a, const double2 *b, double2 s0, const double2 *c_dev,
                                 int64_t m, double s, cudaStream_t st);
@@ -285,6 +295,8 @@ cudaError_t scale_cols_launch(double2 *const *x, int n, const double2 *c_dev, in
                               cudaStream_t st);
 
 // c_j = 1/sqrt(|d_j|) on device (myhgramschmidt_many normalisation).
+// out[j] = the sum of the nblk partials work[j nblk ..] of each of n outputs
+cudaError_t dotdiag_reduce_launch(const double2 *work, int nblk, int n, double2 *out, cudaStream_t st);
 cudaError_t inv_sqrt_abs_launch(const double2 *d, double2 *c, int n, cudaStream_t st);
 
 // Potential-table construction on device from the TINV table.

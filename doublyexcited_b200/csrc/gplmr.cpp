@@ -81,6 +81,7 @@ struct Solver {
     double exch_mult = 0.0;
     unsigned refl_keep = 0xFFu;  // reflection sectors the start block reaches (bit c: sector c)
     bool exch_done = false;      // the last inner solve's output is already exchange-projected
+    int64_t work_elems = 0;      // of h->d_work
     bool z0_staged = false;      // the next inner solve's complex64 start Z_0 is already in Z32
     // The mixed form's self-check: complex64 rounding amplified by the
     // conditioning of the k x k Gram (G^-1/2); a gross-failure detector.
@@ -170,6 +171,7 @@ struct Solver {
         for (cudaEvent_t &e : up_ev) DE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         const int64_t wk = std::max<int64_t>(gram_work_elems(64, 128, D), dotdiag_work_elems(64, D));
         DE_TRY(h->ensure_work(wk));
+        work_elems = wk;
         return DE_OK;
     }
 
@@ -223,6 +225,9 @@ struct Solver {
             return update_sym_launch(U, c, ldc, h->m, exch_mult, st);
         return update_launch(U, c, ldc, D, st);
     }
+    // No product reads X, AX, P and AP: where every update of nev columns takes
+    // the upper half, their lower halves are not written during the iteration.
+    bool half() const { return exch_mult != 0.0 && update_sym_supported(h->m, nev); }
     // An update whose result only Grams and updates of this kind read next:
     // where those take the upper half, the lower one is not written.  The
     // result's columns must be rewritten in full (update_any) before a product.
@@ -280,7 +285,7 @@ struct Solver {
 
     // Y = beta Y + alpha sum_i Xsrc_i C(i, j);  xs / ys are column pointers.
     int update(const std::vector<const double2 *> &xs, const std::vector<double2 *> &ys,
-               const double2 *c, int ldc, cplx alpha, cplx beta)
+               const double2 *c, int ldc, cplx alpha, cplx beta, bool whole = true)
     {
         UpdList U{};
         U.nin = (int)xs.size();
@@ -292,7 +297,7 @@ struct Solver {
             U.beta[j] = make_double2(beta.real(), beta.imag());
         }
         U.alpha = make_double2(alpha.real(), alpha.imag());
-        cudaError_t e = update_any(U, c, ldc);
+        cudaError_t e = whole || !half() ? update_any(U, c, ldc) : update_part(U, c, ldc);
         if (e != cudaSuccess) return cuda_error(e, "update");
         return DE_OK;
     }
@@ -351,6 +356,7 @@ struct Solver {
     // Gram also carries b^H b, so |b - Q Q^H b| follows by Pythagoras; the
     // reference's orthogonalisation followed by cholQR (gplmr.F90:112-196,
     // lamod.f90:128-180) reads every vector twice more for the same column.
+    // With ab, the product of b is known and neither is multiplied next.
     int orth_normalize(std::initializer_list<QBlk> qs, double2 *b, double2 *ab = nullptr)
     {
         ColList L{};
@@ -368,8 +374,8 @@ struct Solver {
         DE_TRY(gram_dev(L, cols(b, 1, D), dG, L.n));
         cudaError_t e = orth_norm_coef_launch(dG, n, dOC, dFlags, st);
         if (e != cudaSuccess) return cuda_error(e, "orth_norm_coef");
-        DE_TRY(update(xs, clw(b, 1), dOC, n + 1, 1.0, 0.0));
-        if (ab) DE_TRY(update(axs, clw(ab, 1), dOC, n + 1, 1.0, 0.0));
+        DE_TRY(update(xs, clw(b, 1), dOC, n + 1, 1.0, 0.0, !ab));
+        if (ab) DE_TRY(update(axs, clw(ab, 1), dOC, n + 1, 1.0, 0.0, false));
         return DE_OK;
     }
 
@@ -429,10 +435,13 @@ struct Solver {
     // When the mixed form's one-column inner solve takes it next, only its
     // complex64 copy is written, straight into the power basis' Z_0: the
     // inner solve overwrites out with its result without reading it.
+    bool stages_z0() const
+    {
+        return nev == 1 && !compat && mixed && order > 1 && order <= 6 && gm.usepetscflag != 0 && gm.max_inner_iter > 0;
+    }
     int seed(double2 *out, const double2 *a, const double2 *b)
     {
-        if (nev == 1 && !compat && mixed && order > 1 && order <= 6 && gm.usepetscflag != 0 &&
-            gm.max_inner_iter > 0) {
+        if (stages_z0()) {
             cudaError_t e = tri() ? axpc_f32_sym_launch(Z32, a, b, make_double2(-1.0, 0.0), dE, h->m, exch_mult, st)
                                   : axpc_f32_launch(Z32, a, b, make_double2(-1.0, 0.0), dE, D, st);
             if (e != cudaSuccess) return cuda_error(e, "axpc_f32");
@@ -451,6 +460,10 @@ struct Solver {
         DE_TRY(minus_e(W, AX, X, nev));
         if ((e = dotdiag_launch(ww.data(), ww.data(), nev, D, 1, dR, h->d_work, st, tri())) != cudaSuccess)
             return cuda_error(e, "dotdiag");
+        return residuals_host(e_host, res);
+    }
+    int residuals_host(std::vector<cplx> &e_host, std::vector<double> &res)
+    {
         DE_CUDA(cudaMemcpyAsync(hbuf, dE, nev * sizeof(double2), cudaMemcpyDeviceToHost, st));
         DE_CUDA(cudaMemcpyAsync(hbuf + 64, dR, nev * sizeof(double2), cudaMemcpyDeviceToHost, st));
         DE_CUDA(cudaMemcpyAsync(hbuf + 128, dFlags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -465,6 +478,39 @@ struct Solver {
                 return set_error(DE_E_NAN, "non-finite residual or eigenvalue in column %d", j);
         }
         return DE_OK;
+    }
+
+    // x <- x / |x|, AX likewise, then the residuals: at the end of an iteration
+    int normalize_residuals(std::vector<cplx> &e_host, std::vector<double> &res)
+    {
+        if (!half() || residual_sym_work_elems(nev, h->m) >= work_elems) {
+            DE_TRY(normalize(X, nev, AX));
+            return residuals(e_host, res);
+        }
+        const double2 *n2 = dR, *ee = dT;
+        if (nev == 1) {  // [AX X]^H X in one read
+            ColList L{};
+            L.n = 2;
+            L.a[0] = AX;
+            L.a[1] = X;
+            DE_TRY(gram_dev(L, cols(X, 1, D), dT, 2));
+            n2 = dT + 1;
+        } else {
+            std::vector<const double2 *> xx = cl(X, nev), aa = cl(AX, nev);
+            cudaError_t e = dotdiag_launch(xx.data(), xx.data(), nev, D, 1, dR, h->d_work, st, tri());
+            if (e == cudaSuccess) e = dotdiag_launch(xx.data(), aa.data(), nev, D, 1, dT, h->d_work, st, tri());
+            if (e != cudaSuccess) return cuda_error(e, "dotdiag");
+        }
+        std::vector<double2 *> xx = clw(X, nev), aa = clw(AX, nev), ww = clw(W, nev);
+        float2 *z[1] = {Z32};
+        cudaError_t e = stages_z0()
+                            ? residual_sym_launch(xx.data(), aa.data(), z, 1, n2, ee, 1, dE, dR, h->m, exch_mult,
+                                                  h->d_work, st)
+                            : residual_sym_launch(xx.data(), aa.data(), ww.data(), nev, n2, ee, nev == 1, dE, dR, h->m,
+                                                  exch_mult, h->d_work, st);
+        if (e != cudaSuccess) return cuda_error(e, "residual_sym");
+        z0_staged = stages_z0();
+        return residuals_host(e_host, res);
     }
 
     // ---- inner solve -------------------------------------------------------
@@ -1361,8 +1407,8 @@ struct Solver {
                     r0 += nr;
                 }
                 DE_TRY(upload(c, dC));
-                DE_TRY(update(xs, clw(P, nev), dC, nin, 1.0, 0.0));
-                DE_TRY(update(axs, clw(AP, nev), dC, nin, 1.0, 0.0));
+                DE_TRY(update(xs, clw(P, nev), dC, nin, 1.0, 0.0, false));
+                DE_TRY(update(axs, clw(AP, nev), dC, nin, 1.0, 0.0, false));
             }
             // X <- X CX + P; AX <- AX CX + AP
             {
@@ -1376,11 +1422,10 @@ struct Solver {
                 std::vector<const double2 *> ps = cl(P, nev), aps = cl(AP, nev);
                 xs.insert(xs.end(), ps.begin(), ps.end());
                 axs.insert(axs.end(), aps.begin(), aps.end());
-                DE_TRY(update(xs, clw(X, nev), dC, 2 * nev, 1.0, 0.0));
-                DE_TRY(update(axs, clw(AX, nev), dC, 2 * nev, 1.0, 0.0));
+                DE_TRY(update(xs, clw(X, nev), dC, 2 * nev, 1.0, 0.0, false));
+                DE_TRY(update(axs, clw(AX, nev), dC, 2 * nev, 1.0, 0.0, false));
             }
-            DE_TRY(normalize(X, nev, AX));
-            DE_TRY(residuals(E, res));
+            DE_TRY(normalize_residuals(E, res));
             maxres = *std::max_element(res.begin(), res.end());
             if (outmodulus > 0 && (maxres <= tol || it % outmodulus == 0)) {
                 printf("ITERATION %5d\n", it);
@@ -1389,6 +1434,12 @@ struct Solver {
                 fflush(stdout);
             }
             ++it;
+        }
+        if (half()) {  // X's lower half
+            std::vector<cplx> one((size_t)nev * nev, 0.0);
+            for (int j = 0; j < nev; ++j) one[j + (size_t)nev * j] = 1.0;
+            DE_TRY(upload(one, dC));
+            DE_TRY(update(cl(X, nev), clw(X, nev), dC, nev, 1.0, 0.0));
         }
         DE_CUDA(cudaStreamSynchronize(st));
         for (int j = 0; j < nev; ++j) e_out[j] = de_complex{E[j].real(), E[j].imag()};

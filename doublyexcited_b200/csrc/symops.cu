@@ -164,6 +164,117 @@ __global__ void __launch_bounds__(512)
     }
 }
 
+struct ResArgs {
+    double2 *x[16], *ax[16];
+    void *w[16];
+    const double2 *n2, *e;  // <x, x> and <x, A x> (conjugated: <A x, x>) of the columns as they come in
+    double2 *e_out;
+    int conj;
+};
+
+// The end of an outer iteration (lamod.f90:94-126, gplmr.F90:128-139) in one
+// pass: x and A x scaled to |x| = 1, E = <x, A x>, the residual w = A x - E x in
+// SW (complex64 where the inner solve takes it next) and the partial sums of
+// |w|^2.  x and A x are read and written in their upper tiles, w is written in
+// full: 3 vector passes (2.5 for complex64) against 9 in separate kernels.
+template <class SW>
+__global__ void __launch_bounds__(256, 2)
+    residual_sym_kernel(const __grid_constant__ ResArgs A, int64_t m, double s, double2 *__restrict__ partial)
+{
+    pdl_enter();
+    constexpr int E = 4, RY = 8;
+    __shared__ SW tile[32][33];
+    __shared__ double2 ec;
+    __shared__ double sc, red[8];
+    const int col = blockIdx.y;
+    if (threadIdx.x == 0) {
+        const double2 n = A.n2[col], e = A.e[col];
+        const double c = 1.0 / sqrt(hypot(n.x, n.y)), c2 = c * c;
+        sc = c;
+        ec = make_double2(c2 * e.x, A.conj ? -c2 * e.y : c2 * e.y);
+        if (blockIdx.x == 0) A.e_out[col] = ec;
+    }
+    int bi, bj;
+    tile_pair(blockIdx.x, bi, bj);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t p = bi * 32 + tx, pt = bj * 32 + tx;
+    double2 *x = A.x[col], *ax = A.ax[col];
+    SW *w = static_cast<SW *>(A.w[col]);
+    double2 xv[E], av[E];
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+        const int64_t q = bj * 32 + ty + RY * u;
+        const bool in = p < m && q < m;
+        xv[u] = in ? x[p + m * q] : make_double2(0.0, 0.0);
+        av[u] = in ? ax[p + m * q] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    const double c = sc;
+    const double2 e = ec;
+    double sum = 0.0;
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+        const int64_t q = bj * 32 + ty + RY * u;
+        xv[u].x *= c;
+        xv[u].y *= c;
+        av[u].x *= c;
+        av[u].y *= c;
+        const double2 v = make_double2(av[u].x - e.x * xv[u].x + e.y * xv[u].y, av[u].y - e.x * xv[u].y - e.y * xv[u].x);
+        SW o;
+        o.x = v.x;
+        o.y = v.y;
+        if (p < m && q < m) {
+            x[p + m * q] = xv[u];
+            ax[p + m * q] = av[u];
+            w[p + m * q] = o;
+        }
+        sum = fma(v.x, v.x, sum);
+        sum = fma(v.y, v.y, sum);
+        o.x = s * o.x;
+        o.y = s * o.y;
+        tile[tx][ty + RY * u] = o;
+    }
+    __syncthreads();
+    if (bi != bj) {
+        sum *= 2.0;  // the tile below the diagonal
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const int cc = ty + RY * u;
+            const int64_t q = bi * 32 + cc;
+            if (pt < m && q < m) w[pt + m * q] = tile[cc][tx];
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+    if (tx == 0) red[ty] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int k = 0; k < 8; ++k) t += red[k];
+        partial[(int64_t)col * gridDim.x + blockIdx.x] = make_double2(t, 0.0);
+    }
+}
+
+template <class SW>
+cudaError_t residual_go(double2 *const *x, double2 *const *ax, SW *const *w, int n, const double2 *n2, const double2 *e,
+                        int conj, double2 *e_out, double2 *r2, int64_t m, double s, double2 *work, cudaStream_t st)
+{
+    if (!sym_rows_supported(m) || n < 1 || n > 16) return cudaErrorInvalidValue;
+    ResArgs A{};
+    for (int j = 0; j < n; ++j) {
+        A.x[j] = x[j];
+        A.ax[j] = ax[j];
+        A.w[j] = w[j];
+    }
+    A.n2 = n2;
+    A.e = e;
+    A.e_out = e_out;
+    A.conj = conj;
+    const int64_t nblk = residual_sym_work_elems(1, m);
+    cudaError_t er = pdl_launch(residual_sym_kernel<SW>, dim3((unsigned)nblk, n), 256, 0, st, A, m, s, work + 1);
+    return er != cudaSuccess ? er : dotdiag_reduce_launch(work + 1, (int)nblk, n, r2, st);
+}
+
 template <class SI, int NOUT, int E, int IC>
 cudaError_t go(const UpdListT<SI, double2> &U, const double2 *c, int ldc, int64_t m, double s, bool upper, cudaStream_t st)
 {
@@ -208,6 +319,26 @@ cudaError_t axpc_f32_sym_launch(float2 *out, const double2 *a, const double2 *b,
     if (!sym_rows_supported(m) || !c_dev) return cudaErrorInvalidValue;
     const int64_t t = (m + 31) / 32;
     return pdl_launch(axpc_f32_sym_kernel, (unsigned)(t * (t + 1) / 2), 512, 0, st, out, a, b, s0, c_dev, m, (float)s);
+}
+
+int64_t residual_sym_work_elems(int n, int64_t m)
+{
+    const int64_t t = (m + 31) / 32;
+    return n * (t * (t + 1) / 2);
+}
+
+cudaError_t residual_sym_launch(double2 *const *x, double2 *const *ax, double2 *const *w, int n, const double2 *n2,
+                                const double2 *e, int conj, double2 *e_out, double2 *r2, int64_t m, double s,
+                                double2 *work, cudaStream_t st)
+{
+    return residual_go(x, ax, w, n, n2, e, conj, e_out, r2, m, s, work, st);
+}
+
+cudaError_t residual_sym_launch(double2 *const *x, double2 *const *ax, float2 *const *w, int n, const double2 *n2,
+                                const double2 *e, int conj, double2 *e_out, double2 *r2, int64_t m, double s,
+                                double2 *work, cudaStream_t st)
+{
+    return residual_go(x, ax, w, n, n2, e, conj, e_out, r2, m, s, work, st);
 }
 
 }  // namespace de

@@ -76,6 +76,25 @@ def test_block_solve_on_upper_halves(de, oracle, nev, order):
     assert np.abs(e[0] - e[1]).max() < 1e-9
 
 
+# The outer iteration's upper-half vectors, for one column with few and with
+# more than nine basis vectors and for blocks; two iterations, so that all of X,
+# AX, P and AP enter the second.  FP64 rounding as above; complex64 as TOL.
+@pytest.mark.parametrize("precision,nev,ns", [("mixed", 1, 2), ("mixed", 1, 9), ("fp64", 3, 2), ("fp64", 9, 1)])
+def test_outer_iteration_on_upper_halves(de, oracle, precision, nev, ns):
+    x0 = oracle.seeded_start(oracle.Params(n=5, delta=2.0, theta=0.3), nev, 51, "triplet")
+    e, res = [], []
+    for family in ("fma", "stream"):
+        with de.Problem(n=5, delta=2.0, theta=0.3, precision=precision) as h:
+            for pass_ in (0, 1):
+                h.set_matvec_launch("c128", pass_, family, 0)
+            r = h.gplmr_eig(x0, -0.78, ns=ns, maxit=2, tol=1e-14, max_inner_iter=3)
+            e.append(r.e)
+            res.append(r.max_residual)
+    tol = 1e-9 if precision == "fp64" else TOL
+    assert np.abs(e[0] - e[1]).max() < tol
+    assert abs(res[0] - res[1]) < tol
+
+
 def test_block_solve_of_an_exhausted_space(de):
     """On 27 points a spherical singlet start reaches 24 states (the
     orbits of point pairs under the cube's symmetries and exchange), so Krylov
