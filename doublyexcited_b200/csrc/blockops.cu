@@ -499,6 +499,7 @@ __device__ __forceinline__ void block_sum(double (&re)[N], double (&im)[N], doub
 // to a power of two, thread t sums output t % np over the blocks
 // b = t / np (mod 256 / np), then a pairwise tree in shared memory adds the
 // 256 / np group sums.  The result does not depend on block timing.
+template <bool DEEP = true>
 __device__ __forceinline__ void reduce_partials(const double2 *__restrict__ part, unsigned nblk, int stride,
                                                 int nout, double2 *res)
 {
@@ -508,8 +509,17 @@ __device__ __forceinline__ void reduce_partials(const double2 *__restrict__ part
     const int groups = 256 / np;
     const int o = threadIdx.x % np, g = threadIdx.x / np;
     double sx = 0.0, sy = 0.0;
-    if (o < nout) {
-        // 16 loads in flight: this tail is latency, paid by every reduction
+    if (!DEEP && o < nout) {
+#pragma unroll 4
+        for (unsigned b = g; b < nblk; b += groups) {
+            const double2 v = __ldcg(part + (int64_t)b * stride + o);
+            sx += v.x;
+            sy += v.y;
+        }
+    } else if (o < nout) {
+        // 16 loads in flight: this tail is latency, paid by every reduction.
+        // (Not in gram_small, whose main loop the compiler then schedules worse:
+        // 12 x 1 at 4.8 M rows 454 us with 4 loads, 487 with 16.)
         for (unsigned b = g; b < nblk; b += 16 * groups) {
             double2 v[16];
 #pragma unroll
@@ -611,7 +621,7 @@ __global__ void __launch_bounds__(256)
     block_sum<NLM * NRM>(ar, ai, part + (int64_t)blockIdx.x * nout, nout);
     if (last_block(ticket, gridDim.x)) {
         __shared__ double2 res[32];
-        reduce_partials(part, gridDim.x, nout, nout, res);
+        reduce_partials<false>(part, gridDim.x, nout, nout, res);
         for (int o = threadIdx.x; o < nl * nr; o += blockDim.x) {
             const int i = o / nr, j = o % nr;
             out[i + (int64_t)ldo * j] = res[i * NRM + j];
@@ -1669,7 +1679,10 @@ static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t 
             return L.a[L.n - 1] == R.a[0] ? gram_col_any<true>(L, R.a[0], len, herm, out, work, st, tri)
                                           : gram_col_any<false>(L, R.a[0], len, herm, out, work, st, tri);
     }
-    if (R.n == 1 && L.n <= 32 && !tri) {  // these read whole vectors
+    // one ket: a thread holds all sums, up to 8 of them, or up to 32 of a short
+    // vector; longer ones go to the tiles (4.8 M rows: 12 x 1 454 us against 215,
+    // 24 x 1 1645 against 351).  These read whole vectors.
+    if (R.n == 1 && (L.n <= 8 || (L.n <= 32 && len < (1 << 18))) && !tri) {
         if (L.n <= 1) return gram_small_go<1, 1>(L, R, len, herm, out, ldo, work, st);
         if (L.n <= 2) return gram_small_go<2, 1>(L, R, len, herm, out, ldo, work, st);
         if (L.n <= 4) return gram_small_go<4, 1>(L, R, len, herm, out, ldo, work, st);
@@ -1686,11 +1699,12 @@ static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t 
     }
     // up to 4 x 4 of a short vector in one fused launch, all operands straight
     // into registers: 13 us against 15 for the tiles at 118 K rows, 70 against
-    // 33 at 1.8 M
-    if (L.n <= 4 && R.n <= 4 && len < (1 << 18)) {
-        if (L.n <= 2 && R.n <= 2) return gram_small_go<2, 2>(L, R, len, herm, out, ldo, work, st);
-        return gram_small_go<4, 4>(L, R, len, herm, out, ldo, work, st);
-    }
+    // 33 at 1.8 M; 1 x 2 at any length, where the tiles pad one bra to four (44
+    // us against 32 at 1.8 M rows), and 2 x 2 up to 2^20 rows (36 against 31 at
+    // 531 K)
+    if (!tri && L.n <= 2 && R.n <= 2 && (L.n == 1 || len < (1 << 20)))
+        return gram_small_go<2, 2>(L, R, len, herm, out, ldo, work, st);
+    if (!tri && L.n <= 4 && R.n <= 4 && len < (1 << 18)) return gram_small_go<4, 4>(L, R, len, herm, out, ldo, work, st);
     if (L.n == 8 && R.n == 16 && herm) {  // the projection of one column with a P block
         bool km8 = R.sigma.x == L.sigma.x && R.sigma.y == L.sigma.y;
         for (int c = 0; c < 8 && km8; ++c)

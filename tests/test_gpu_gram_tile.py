@@ -10,9 +10,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("size", [1, 63, 64, 65, 257, 16384, 262144, 300007])
+@pytest.mark.parametrize("size", [1, 63, 64, 65, 257, 16384, 262144, 300007, 1048577])
 @pytest.mark.parametrize("nbra,nket,herm", [(4, 4, 1), (5, 4, 0), (1, 3, 1), (3, 2, 0), (8, 17, 1), (33, 4, 0),
-                                            (13, 29, 1), (2, 32, 0), (32, 16, 1), (64, 1, 0), (40, 17, 1)])
+                                            (13, 29, 1), (2, 32, 0), (32, 16, 1), (64, 1, 0), (40, 17, 1),
+                                            (24, 24, 1), (1, 2, 0), (2, 2, 1), (12, 1, 1), (32, 1, 0)])
 def test_dots_tiles(de, size, nbra, nket, herm):
     import torch
 
