@@ -171,9 +171,11 @@ def alg_bytes(nn):
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum, pass A + pass B)
 # per vector-matvec of the kernels the library picks, keyed by (NN,
 # storage): one ncu capture of the block-of-2 matvec at N=6 (`--workload
-# matvec-n6`), the three kernels' bytes over 2 vectors.  Kernels without a
-# capture report null.
-NCU_TRAFFIC_PER_VECTOR = {(13, "f32"): 237.0e6, (13, "f64"): 552.3e6}
+# matvec-n6`), the three kernels' bytes over 2 vectors; "-exch": the two
+# kernels of an exchange-symmetric product inside the mixed solve at N=6 (one
+# vector; part of it stays in L2).  Kernels without a capture report null.
+NCU_TRAFFIC_PER_VECTOR = {(13, "f32"): 237.0e6, (13, "f64"): 552.3e6, (13, "f32-exch"): 97.3e6,
+                          (13, "f64-exch"): 250.3e6}
 
 # The timed solves keep the library's matvec events on for the roofline
 # figures, on every 8th MATBLOCK call of each storage: all calls of one
@@ -321,10 +323,14 @@ def dist_setup():
     return rank, world, local
 
 
-def matvec_kernel_name(nn, fp32):
+def matvec_kernel_name(nn, fp32, exch=False):
     """The kernels the library picks (de_set_matvec_kernel's default): the
-    line kernels on every grid."""
+    line kernels on every grid; exch: the products of a solve whose vectors
+    keep the exchange symmetry of a singlet or triplet start (the mixed form
+    and blocks)."""
     r = "float" if fp32 else "double"
+    if exch:
+        return f"hammult cube_line_kernel + exch_add_kernel <{r}, {nn}>"
     return f"hammult plane_kernel + kline_kernel (pass A) + cube_line_kernel (pass B) <{r}, {nn}>"
 
 
@@ -803,6 +809,8 @@ def main():
     peak = fp64_peak_tflops(torch)
     peak32 = fp32_peak_tflops(torch)
 
+    exch = a.precision == "mixed" or w["nev"] > 1
+
     def roof(pr, fp32, pk, src):
         ms = pr["pass_a_ms"] + pr["pass_b_ms"]
         vecs = max(1, pr["vectors"])
@@ -810,8 +818,8 @@ def main():
         ebytes = 16 if fp32 else 32
         return {"bound": "tensor" if not fp32 else "fp32-fma", "achieved": ach, "peak": pk, "unit": "TFLOP/s",
                 "frac": ach / pk if pk else None,
-                "traffic": NCU_TRAFFIC_PER_VECTOR.get((nn, "f32" if fp32 else "f64")),
-                "kernel": matvec_kernel_name(nn, fp32) + ", per vector-matvec",
+                "traffic": NCU_TRAFFIC_PER_VECTOR.get((nn, ("f32" if fp32 else "f64") + ("-exch" if exch else ""))),
+                "kernel": matvec_kernel_name(nn, fp32, exch) + ", per vector-matvec",
                 "alg_flops_per_vector": alg_flops(nn), "alg_bytes_per_vector": ebytes * nn ** 6,
                 "achieved_gbs_alg": ebytes * nn ** 6 * vecs / (ms / 1e3) / 1e9 if ms > 0 else None,
                 "matvec_ms_per_vector": ms / vecs, "pass_a_ms": pr["pass_a_ms"] / vecs,

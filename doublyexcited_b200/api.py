@@ -101,8 +101,8 @@ class Problem:
 
     def set_matvec_kernel(self, kind: str) -> None:
         """'fma' (default): the CUDA-core kernels that contract whole lines
-        in registers, even/odd-split (every grid); 'tensor': the axis contractions on the FP64 tensor
-        cores where built (NN 9..19); 'stream': the earlier CUDA-core
+        in registers, even/odd-split (every grid); 'tensor': the axis
+        contractions on the FP64 tensor cores where built (NN 9..19); 'stream': the earlier CUDA-core
         streaming kernels (NN 13..19); 'tf32': the complex64 matvec's
         kinetic contractions on the TF32 tensor cores with head/tail split
         operands (NN 9..15)."""

@@ -3,7 +3,7 @@
 //
 // Reference: KEMULTS hammod.F90:264-286 inside KEMULT2 :138-187, and the
 // potential term Y = Y + V*X (:58-59).  The two passes are the CUDA-core
-// kernels' (hammult.cu, hammult_ev.cu): pass A contracts the electron-2
+// kernels' (hammult.cu, hammult_line.cu): pass A contracts the electron-2
 // axes of row cubes X(p, :) and adds the potential, writing Y; pass B
 // contracts the electron-1 axes of column cubes X(:, q) and folds pass A's
 // Y in.
