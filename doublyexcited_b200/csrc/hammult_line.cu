@@ -35,9 +35,11 @@
 // * The kernel that only writes runs first; the accumulating ones cost more
 //   (their old values are on the critical path).  complex64 adds into Y with
 //   red.global.add.v2.f32, one per element and kernel, so the order of the
-//   sums is fixed and no load of Y is waited for (kline at NN = 17: 89 us
-//   against 106 us).  complex128 would need two scalar adds per element and
-//   measured no faster; it prefetches Y two outputs ahead instead.
+//   sums is fixed and no load of Y is waited for (a product at NN = 17: 260 us
+//   against 314 with Y prefetched as below).  That add flushes subnormals, so
+//   tiny values take a load, an add and a store (add_to).  complex128 would
+//   need two scalar adds per element and measured no faster; it prefetches Y
+//   two outputs ahead instead.
 //
 // Measured on B200, us per vector, one vector per call, before (the even/odd
 // slab, streaming or cube kernels, whichever the grid had) and now, as plane +
@@ -143,6 +145,8 @@ struct Cx<double> {
 };
 template <class R>
 using CC = typename Cx<R>::C;
+template <class R>
+using G2 = std::conditional_t<sizeof(R) == 8, double2, float2>;
 
 template <int I, int E, class F>
 __device__ __forceinline__ void static_for(F f)
@@ -153,14 +157,16 @@ __device__ __forceinline__ void static_for(F f)
     }
 }
 
+struct Nothing {};
+
 // One line: v holds its NN values and is overwritten; emit(pos, value,
 // loaded) receives delta^2 T v at every point.  loaded = fetch(pos) is what
 // the caller adds there, fetched LA outputs ahead.  ORDER keeps the memory
 // operations in that order: without it the compiler gathers all of a line's
 // loads in front of the sums, and complex128 lines do not leave it the
 // registers.
-template <class R, int NN, int LA, bool ORDER, class Q, class F>
-__device__ __forceinline__ void line_transform(CC<R> (&v)[NN], Q fetch, F emit)
+template <class R, int NN, int LA, bool ORDER, class Q, class F, class P = Nothing>
+__device__ __forceinline__ void line_transform(CC<R> (&v)[NN], Q fetch, F emit, P emit_pair = P())
 {
     using X = Cx<R>;
     constexpr int N = NN / 2;
@@ -201,8 +207,12 @@ __device__ __forceinline__ void line_transform(CC<R> (&v)[NN], Q fetch, F emit)
                 constexpr R d = (R)ocoef(a, b);
                 o = X::fma(d, v[N - b], o);
             });
-            emit(N + a, X::add(e, o), lp[a]);
-            emit(N - a, X::sub(e, o), lm[a]);
+            if constexpr (std::is_same_v<P, Nothing>) {
+                emit(N + a, X::add(e, o), lp[a]);
+                emit(N - a, X::sub(e, o), lm[a]);
+            } else {
+                emit_pair(N + a, X::add(e, o), lp[a], N - a, X::sub(e, o), lm[a]);
+            }
         }
     });
 }
@@ -219,8 +229,6 @@ struct LineArgs {
     R shr, shi;  // diagonal shift
 };
 
-struct Nothing {};
-
 template <class R>
 __device__ __forceinline__ void times_s2(const LineArgs<R> &a, CC<R> z, R &yr, R &yi)
 {
@@ -230,10 +238,40 @@ __device__ __forceinline__ void times_s2(const LineArgs<R> &a, CC<R> z, R &yr, R
     yi = a.s2r * zi + a.s2i * zr;
 }
 
-// y += (yr, yi) without waiting for y; one add per element and kernel
-__device__ __forceinline__ void add_to(unsigned long long *y, float yr, float yi)
+// y += v of complex64 values, one add per element and kernel, without waiting
+// for y.  The add in L2 flushes subnormals, and a vector of values below 1e-36
+// lost 0.1 % of its norm, one below 1e-40 all of it; a value with a part below
+// 2^-100 is therefore added here.  At or above that nothing is lost: y's
+// subnormal part is below half an ulp of the sum, and a sum that cancels is
+// zero or at least 2^-123.  One test serves the two outputs of a step: us per
+// product without a test, with one per output, with one per pair: NN = 13
+// 47.3, 44.1, 43.6; NN = 17 256, 264, 260; NN = 19 665, 643, 632.
+__device__ __forceinline__ bool l2_add(float2 v, float2 w)
 {
-    asm volatile("red.global.add.v2.f32 [%0], {%1,%2};" ::"l"(y), "f"(yr), "f"(yi) : "memory");
+    return fminf(fminf(fabsf(v.x), fabsf(v.y)), fminf(fabsf(w.x), fabsf(w.y))) >= 0x1p-100f;
+}
+__device__ __forceinline__ void add_l2(unsigned long long *y, float2 v)
+{
+    asm volatile("red.global.add.v2.f32 [%0], {%1,%2};" ::"l"(y), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void add_here(unsigned long long *y, float2 v)
+{
+    *y = Cx<float>::add(*y, Cx<float>::make(v.x, v.y));
+}
+__device__ __forceinline__ void add_to(unsigned long long *y, float2 v)
+{
+    if (l2_add(v, v)) add_l2(y, v);
+    else add_here(y, v);
+}
+__device__ __forceinline__ void add_to(unsigned long long *y, float2 v, unsigned long long *z, float2 w)
+{
+    if (l2_add(v, w)) {
+        add_l2(y, v);
+        add_l2(z, w);
+    } else {
+        add_here(y, v);
+        add_here(z, w);
+    }
 }
 
 // Programmatic dependent launch (a no-op when the launch carries no
@@ -386,6 +424,13 @@ __global__ void __launch_bounds__(Cfg<R, NN>::KT, Cfg<R, NN>::KB) kline_kernel(c
 #pragma unroll
             for (int k = 0; k < NN; ++k) pot[k] = potential(k);
         }
+        auto sum = [&](CC<R> z, L l) {
+            R yr, yi, xr, xi;
+            times_s2(a, z, yr, yi);
+            X::split(l.x, xr, xi);
+            const R pr = fma(l.v, a.vsr, a.shr), pi = fma(l.v, a.vsi, a.shi);
+            return G2<R>{yr + (pr * xr - pi * xi), yi + (pr * xi + pi * xr)};
+        };
         line_transform<R, NN, K::KV && sizeof(R) == 4 ? 0 : 2, true>(
             v,
             [&](int k) {
@@ -398,15 +443,16 @@ __global__ void __launch_bounds__(Cfg<R, NN>::KT, Cfg<R, NN>::KB) kline_kernel(c
                 return l;
             },
             [&](int k, CC<R> z, L l) {
-                R yr, yi, xr, xi;
-                times_s2(a, z, yr, yi);
-                X::split(l.x, xr, xi);
-                const R pr = fma(l.v, a.vsr, a.shr), pi = fma(l.v, a.vsi, a.shi);
-                yr += pr * xr - pi * xi;
-                yi += pr * xi + pi * xr;
-                if constexpr (sizeof(R) == 8) y[KS * k] = X::make(l.y.x + yr, l.y.y + yi);
-                else add_to(y + KS * k, yr, yi);
-            });
+                const G2<R> s = sum(z, l);
+                if constexpr (sizeof(R) == 8) y[KS * k] = X::make(l.y.x + s.x, l.y.y + s.y);
+                else add_to(y + KS * k, s);
+            },
+            [&] {
+                if constexpr (sizeof(R) == 8) return Nothing{};
+                else return [&](int k1, CC<R> z1, L l1, int k2, CC<R> z2, L l2) {
+                    add_to(y + KS * k1, sum(z1, l1), y + KS * k2, sum(z2, l2));
+                };
+            }());
     }
 }
 
@@ -480,12 +526,21 @@ __global__ void __launch_bounds__(Cfg<R, NN>::CT, Cfg<R, NN>::CB) cube_line_kern
                         return r;
                     },
                     [&](int j, CC<R> z, L r) {
-                        R yr, yi;
-                        times_s2(a, X::add(r.s, z), yr, yi);
-                        if constexpr (!ADD) g[NN * j] = X::make(yr, yi);
-                        else if constexpr (sizeof(R) == 8) g[NN * j] = X::make(r.y.x + yr, r.y.y + yi);
-                        else add_to(g + NN * j, yr, yi);
-                    });
+                        G2<R> s;
+                        times_s2(a, X::add(r.s, z), s.x, s.y);
+                        if constexpr (!ADD) g[NN * j] = X::make(s.x, s.y);
+                        else if constexpr (sizeof(R) == 8) g[NN * j] = X::make(r.y.x + s.x, r.y.y + s.y);
+                        else add_to(g + NN * j, s);
+                    },
+                    [&] {
+                        if constexpr (!ADD || sizeof(R) == 8) return Nothing{};
+                        else return [&](int j1, CC<R> z1, L r1, int j2, CC<R> z2, L r2) {
+                            G2<R> s1, s2;
+                            times_s2(a, X::add(r1.s, z1), s1.x, s1.y);
+                            times_s2(a, X::add(r2.s, z2), s2.x, s2.y);
+                            add_to(g + NN * j1, s1, g + NN * j2, s2);
+                        };
+                    }());
             }
             if (G < NN || more) __syncthreads();
         }
@@ -508,7 +563,7 @@ template <class R>
 __global__ void __launch_bounds__(kExchThreads, 3)
     exch_add_kernel(const __grid_constant__ LineArgs<R> a, int nn, R s)
 {
-    using G = std::conditional_t<sizeof(R) == 8, double2, float2>;
+    using G = G2<R>;
     constexpr int RY = kExchThreads / 32, E = 32 / RY;
     __shared__ G ta[32][33], tb[32][33];
     __shared__ int bp[32], bq[32];
