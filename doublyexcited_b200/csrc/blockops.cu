@@ -67,6 +67,13 @@ __device__ __forceinline__ double2 ldp(const float2 *p)
     const float2 v = *p;
     return make_double2(v.x, v.y);
 }
+// a predecessor's data, widened
+template <class S>
+__device__ __forceinline__ double2 ldw_prev(const S *p)
+{
+    const S v = ld_prev(p);
+    return make_double2(v.x, v.y);
+}
 template <class S>
 __device__ __forceinline__ S st2(double x, double y);
 template <>
@@ -96,7 +103,7 @@ __device__ __forceinline__ double2 col_elem(const ColListT<S> &L, int c, int64_t
 // 32nd block, 16 loads in flight, then a fixed tree (29 us with 8 groups of one
 // warp and 1184 partials, 18 us so).
 __global__ void __launch_bounds__(256)
-    gram_reduce(const double2 *__restrict__ work, int nblk, int nl, int nr, double2 *__restrict__ out, int ldo)
+    gram_reduce(const double2 *work, int nblk, int nl, int nr, double2 *out, int ldo)
 {
     pdl_enter();
     __shared__ double2 acc[32][8];
@@ -107,7 +114,7 @@ __global__ void __launch_bounds__(256)
         double2 v[16];
 #pragma unroll
         for (int u = 0; u < 16; ++u)
-            v[u] = b + 32 * u < nblk ? __ldg(work + (int64_t)(b + 32 * u) * nout + o) : make_double2(0.0, 0.0);
+            v[u] = b + 32 * u < nblk ? ld_prev(work + (int64_t)(b + 32 * u) * nout + o) : make_double2(0.0, 0.0);
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
             sx += v[u].x;
@@ -151,8 +158,7 @@ struct UpdArith<float2, float2> {
 
 template <class SI, class SO, int NOUT>
 __global__ void __launch_bounds__(256)
-    update_kernel(const __grid_constant__ UpdListT<SI, SO> U, const double2 *__restrict__ C, int ldc,
-                  int64_t len)
+    update_kernel(const __grid_constant__ UpdListT<SI, SO> U, const double2 *C, int ldc, int64_t len)
 {
     pdl_enter();
     using T = typename UpdArith<SI, SO>::T;
@@ -224,7 +230,7 @@ __global__ void __launch_bounds__(256)
 // 7 113 -> 94 (94), 8 152 -> 105 (106).
 template <int NC>
 __global__ void __launch_bounds__(256, 3)
-    update_col(const __grid_constant__ UpdListT<double2, double2> U, const double2 *__restrict__ C, int64_t len)
+    update_col(const __grid_constant__ UpdListT<double2, double2> U, const double2 *C, int64_t len)
 {
     pdl_enter();
     __shared__ double2 cs[NC];
@@ -297,8 +303,8 @@ __global__ void axpc_kernel(const __grid_constant__ PtrPack P, double2 s, const 
 }
 
 // out = (complex64) (a + s c b) for one column (c = c_dev[0], or 1)
-__global__ void axpc_f32_kernel(float2 *__restrict__ out, const double2 *__restrict__ a,
-                                const double2 *__restrict__ b, double2 s, const double2 *c_dev, int64_t len)
+__global__ void axpc_f32_kernel(float2 *out, const double2 *a, const double2 *b, double2 s, const double2 *c_dev,
+                                int64_t len)
 {
     pdl_enter();
     const double2 c = c_dev ? c_dev[0] : make_double2(1.0, 0.0);
@@ -312,8 +318,7 @@ __global__ void axpc_f32_kernel(float2 *__restrict__ out, const double2 *__restr
 
 // out = a + s b over n contiguous elements (FP64 arithmetic, storage S)
 template <class S>
-__global__ void axpy_kernel(S *__restrict__ out, const S *__restrict__ a, const S *__restrict__ b, double2 s,
-                            int64_t n)
+__global__ void axpy_kernel(S *out, const S *a, const S *b, double2 s, int64_t n)
 {
     pdl_enter();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -385,7 +390,7 @@ __global__ void dotdiag_partial(const __grid_constant__ PtrPack P, int64_t len, 
 // One 256-thread block per output j: strided partial sums, then a fixed
 // shuffle/shared-memory tree (deterministic).
 __global__ void __launch_bounds__(256)
-    dotdiag_reduce(const double2 *__restrict__ work, int nblk, int n, double2 *__restrict__ out)
+    dotdiag_reduce(const double2 *work, int nblk, int n, double2 *out)
 {
     pdl_enter();
     __shared__ double2 acc[8];
@@ -512,7 +517,7 @@ __device__ __forceinline__ void reduce_partials(const double2 *__restrict__ part
     if (!DEEP && o < nout) {
 #pragma unroll 4
         for (unsigned b = g; b < nblk; b += groups) {
-            const double2 v = __ldcg(part + (int64_t)b * stride + o);
+            const double2 v = ld_l2(part + (int64_t)b * stride + o);
             sx += v.x;
             sy += v.y;
         }
@@ -524,7 +529,7 @@ __device__ __forceinline__ void reduce_partials(const double2 *__restrict__ part
             double2 v[16];
 #pragma unroll
             for (int u = 0; u < 16; ++u)
-                v[u] = b + u * groups < nblk ? __ldcg(part + (int64_t)(b + u * groups) * stride + o)
+                v[u] = b + u * groups < nblk ? ld_l2(part + (int64_t)(b + u * groups) * stride + o)
                                              : make_double2(0.0, 0.0);
 #pragma unroll
             for (int u = 0; u < 16; ++u) {
@@ -637,8 +642,8 @@ __global__ void __launch_bounds__(256)
 // 3-4 columns 79 -> 44-56 (35-47), 5-8 columns 133 -> 70-108 (59-94).
 template <int NC, bool SELF, bool TRI>
 __global__ void __launch_bounds__(256, 2)
-    gram_col(const __grid_constant__ ColListT<double2> L, const double2 *__restrict__ b, int64_t len, unsigned m, int herm,
-             double2 *__restrict__ work, double2 *__restrict__ out)
+    gram_col(const __grid_constant__ ColListT<double2> L, const double2 *b, int64_t len, unsigned m, int herm, double2 *work,
+             double2 *out)
 {
     pdl_enter();
     constexpr int U = 2;
@@ -660,8 +665,8 @@ __global__ void __launch_bounds__(256, 2)
             bool in = ru < len;
             if constexpr (TRI) in = in && tri_row((unsigned)ru, m, ru, wt[u]);
 #pragma unroll
-            for (int i = 0; i < NC; ++i) l[u][i] = in ? __ldg(col[i] + ru) : make_double2(0.0, 0.0);
-            if constexpr (!SELF) x[u] = in ? __ldg(b + ru) : make_double2(0.0, 0.0);
+            for (int i = 0; i < NC; ++i) l[u][i] = in ? ld_prev(col[i] + ru) : make_double2(0.0, 0.0);
+            if constexpr (!SELF) x[u] = in ? ld_prev(b + ru) : make_double2(0.0, 0.0);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -893,7 +898,7 @@ __device__ __forceinline__ void raise_flag(int *flag, int bit)
 // b^H b - |Q^H b|^2 (Pythagoras), coef = [-(Q^H b)/|w|; 1/|w|], so that
 // w/|w| = [Q, b] coef.  A |w|^2 not above 1e-28 b^H b raises flag bit 1, as
 // a cholQR breakdown does, and leaves b unchanged.
-__global__ void orth_norm_coef(const double2 *__restrict__ g, int n, double2 *__restrict__ coef, int *flag)
+__global__ void orth_norm_coef(const double2 *g, int n, double2 *coef, int *flag)
 {
     pdl_enter();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
@@ -966,7 +971,7 @@ __device__ __forceinline__ void block_upper_inverse(const double2 *R, const doub
 // Upper Cholesky R of the Hermitian G (upper triangle read, as zpotrf 'U')
 // and R^{-1}.  flag |= 1 on breakdown, 2 when G is all zero.
 __global__ void __launch_bounds__(64)
-    small_cholinv(const double2 *__restrict__ G, int k, double2 *__restrict__ Rinv, int *flag)
+    small_cholinv(const double2 *G, int k, double2 *Rinv, int *flag)
 {
     pdl_enter();
     __shared__ double2 R[16 * 16], X[16 * 16];
@@ -994,8 +999,7 @@ __global__ void __launch_bounds__(64)
 // rounding, when half of a column or more may go: then the pass is done alone (R
 // = 1) and the CholQR that follows normalises.
 __global__ void __launch_bounds__(256)
-    small_orth_chol(const double2 *__restrict__ g, int m, int k, double2 *__restrict__ rinv, double2 *__restrict__ c,
-                    int *flag)
+    small_orth_chol(const double2 *g, int m, int k, double2 *rinv, double2 *c, int *flag)
 {
     pdl_enter();
     __shared__ double2 B[64 * 16], R[16 * 16], X[16 * 16];
@@ -1047,8 +1051,8 @@ __global__ void __launch_bounds__(256)
 // C = [-(G1 + G2) W; W] with W = R1^-1 R2^-1: G1, G2 m x k (ld m and ld2), the
 // rest k x k, C (m + k) x k (ld m + k), k <= 16.
 __global__ void __launch_bounds__(256)
-    small_block_coef(const double2 *__restrict__ g1, const double2 *__restrict__ g2, int ld2, int m, int k,
-                     const double2 *__restrict__ r1, const double2 *__restrict__ r2, double2 *__restrict__ c)
+    small_block_coef(const double2 *g1, const double2 *g2, int ld2, int m, int k, const double2 *r1, const double2 *r2,
+                     double2 *c)
 {
     pdl_enter();
     __shared__ double2 w[16 * 16];
@@ -1092,7 +1096,7 @@ __global__ void small_hsqrt1(const double2 *__restrict__ g, double2 *__restrict_
 
 // harm_orthog_oneblock's self-check (harmonic_ritz_small.F90:221-242):
 // flag |= 4 when any |T - I| > 1e-10.
-__global__ void small_ortho_check(const double2 *__restrict__ t, int k, double tol, int *flag)
+__global__ void small_ortho_check(const double2 *t, int k, double tol, int *flag)
 {
     pdl_enter();
     const int o = threadIdx.x;
@@ -1183,7 +1187,7 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-__global__ void cvt_c2f_kernel(const double2 *__restrict__ x, float2 *__restrict__ y, int64_t n)
+__global__ void cvt_c2f_kernel(const double2 *x, float2 *y, int64_t n)
 {
     pdl_enter();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1513,9 +1517,9 @@ __global__ void __launch_bounds__(512)
         rbp[b] = j < nr ? R.b[j] : nullptr;
     }
     auto elem = [](const S *pa, const S *pb, double2 sgm, int64_t r) {
-        double2 v = ld2(pa + r);
+        double2 v = ldw_prev(pa + r);
         if (pb) {
-            const double2 w = ld2(pb + r);
+            const double2 w = ldw_prev(pb + r);
             v.x -= sgm.x * w.x - sgm.y * w.y;
             v.y -= sgm.x * w.y + sgm.y * w.x;
         }
@@ -1533,8 +1537,8 @@ __global__ void __launch_bounds__(512)
             double wt = 1.0;
             if constexpr (TRI) rok = rok && tri_row((unsigned)r, m, r, wt);
             if constexpr (KM8) {
-                const double2 av = rok ? ld2(la[0] + r) : make_double2(0.0, 0.0);
-                const double2 v = rok ? ld2(lb[0] + r) : make_double2(0.0, 0.0);
+                const double2 av = rok ? ldw_prev(la[0] + r) : make_double2(0.0, 0.0);
+                const double2 v = rok ? ldw_prev(lb[0] + r) : make_double2(0.0, 0.0);
                 const double2 sgm = L.sigma;
                 lv[u][0] = make_double2(av.x - (sgm.x * v.x - sgm.y * v.y), av.y - (sgm.x * v.y + sgm.y * v.x));
                 rv[u][0] = lv[u][0];
@@ -1832,8 +1836,8 @@ __global__ void __launch_bounds__(256, 2)
         S z0[NZ], z1[NZ];
 #pragma unroll
         for (int j = 0; j < NZ; ++j) {
-            z0[j] = has0 ? __ldg(zc[j] + ra) : S{0, 0};
-            z1[j] = has1 ? __ldg(zc[j] + r1) : S{0, 0};
+            z0[j] = has0 ? ld_prev(zc[j] + ra) : S{0, 0};
+            z1[j] = has1 ? ld_prev(zc[j] + r1) : S{0, 0};
         }
         double xr[NZ], xi[NZ];
 #pragma unroll
@@ -2132,7 +2136,7 @@ cudaError_t gs_pass2_launch(const float2 *const *qp, const float2 *const *vp, in
 // (D^-1 G[1:,1:] D^-1 + 1e-13 I) y = D^-1 G[1:,0] by Cholesky and returns
 // a = D^-1 y (nq values).  Flag 8 if the system is not positive definite.
 __global__ void __launch_bounds__(64)
-    small_sstep_solve(const double2 *__restrict__ G, int nz, double2 *__restrict__ a, int *flag)
+    small_sstep_solve(const double2 *G, int nz, double2 *a, int *flag)
 {
     pdl_enter();
     __shared__ double2 R[8 * 8], y[8];

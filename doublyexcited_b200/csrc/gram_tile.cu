@@ -68,7 +68,7 @@ __device__ __forceinline__ void sum_partials(const double2 *work, int nblk, int 
         double2 v[10];
 #pragma unroll
         for (int u = 0; u < 10; ++u)
-            v[u] = b + 32 * u < nblk ? __ldcg(work + (int64_t)(b + 32 * u) * nout + o) : make_double2(0.0, 0.0);
+            v[u] = b + 32 * u < nblk ? ld_l2(work + (int64_t)(b + 32 * u) * nout + o) : make_double2(0.0, 0.0);
 #pragma unroll
         for (int u = 0; u < 10; ++u) {
             x += v[u].x;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_con
 
 // Sum of the nblk partials, a warp per output.
 __global__ void __launch_bounds__(256)
-    gram_tile_reduce(const double2 *__restrict__ work, int nblk, int nl, int nr, double2 *__restrict__ out, int ldo)
+    gram_tile_reduce(const double2 *work, int nblk, int nl, int nr, double2 *out, int ldo)
 {
     pdl_enter();
     const int o = blockIdx.x * 8 + (threadIdx.x >> 5);

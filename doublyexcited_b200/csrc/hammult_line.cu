@@ -63,6 +63,7 @@
 // = 17), as did L2 prefetches of the next column (the phases wait on the SM,
 // not on DRAM) and running the two electron-2 kernels in p chunks that fit L2.
 #include "de_kernels.h"
+#include "pdl.h"
 
 #include <algorithm>
 #include <atomic>
@@ -286,7 +287,12 @@ __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.la
 //   PW, PB  plane: run of adjacent p (128 bytes where it fits), min CTAs/SM
 //   KT, KB  kline: threads, min CTAs/SM; KS stash the line in shared memory
 //           for the V x term instead of reading it again; KV all of a line's
-//           potential values loaded before the sums
+//           potential values loaded before the sums.  complex64 takes both from
+//           NN = 9 on (loads between the sums wait for their turn among the
+//           ordered memory operations: us per product without, with, at NN =
+//           11 19.0, 18.5; 17 262, 257; 21 1084, 1066); below, lines are
+//           short and more CTAs hide them.  complex128 has registers for KV at
+//           some sizes only
 //   CT, CB  cube: threads, min CTAs/SM; CG slabs of x staged at a time (NN =
 //           the whole cube; less where two cubes exceed shared memory)
 template <class R, int NN>
@@ -311,14 +317,14 @@ LINE_SHAPE(double, 23, 4, 2, 256, 1, 0, 0, 96, 1, 3)
 LINE_SHAPE(float, 3, 64, 8, 128, 10, 0, 0, 32, 31, 3)
 LINE_SHAPE(float, 5, 64, 4, 128, 9, 0, 0, 32, 31, 5)
 LINE_SHAPE(float, 7, 32, 4, 128, 8, 0, 0, 64, 20, 7)
-LINE_SHAPE(float, 9, 32, 2, 128, 8, 0, 0, 96, 13, 9)
-LINE_SHAPE(float, 11, 16, 5, 128, 6, 0, 0, 128, 9, 11)
-LINE_SHAPE(float, 13, 16, 3, 128, 6, 0, 0, 192, 6, 13)
-LINE_SHAPE(float, 15, 16, 3, 128, 5, 0, 0, 256, 3, 15)
-LINE_SHAPE(float, 17, 16, 2, 256, 2, 0, 0, 320, 2, 17)
+LINE_SHAPE(float, 9, 32, 2, 128, 6, 1, 1, 96, 13, 9)
+LINE_SHAPE(float, 11, 16, 5, 128, 6, 1, 1, 128, 7, 11)
+LINE_SHAPE(float, 13, 16, 3, 128, 6, 1, 1, 192, 6, 13)
+LINE_SHAPE(float, 15, 16, 3, 128, 4, 1, 1, 256, 3, 15)
+LINE_SHAPE(float, 17, 16, 2, 256, 2, 1, 1, 320, 2, 17)
 LINE_SHAPE(float, 19, 16, 2, 256, 3, 1, 1, 192, 2, 19)
-LINE_SHAPE(float, 21, 8, 2, 128, 4, 0, 0, 448, 1, 21)
-LINE_SHAPE(float, 23, 8, 2, 128, 4, 0, 0, 544, 1, 23)
+LINE_SHAPE(float, 21, 8, 2, 128, 3, 1, 1, 448, 1, 21)
+LINE_SHAPE(float, 23, 8, 2, 128, 3, 1, 1, 544, 1, 23)
 #undef LINE_SHAPE
 
 template <class R, int NN>
@@ -359,7 +365,7 @@ __global__ void __launch_bounds__(Cfg<R, NN>::PT, Cfg<R, NN>::PB) plane_kernel(c
             const CC<R> *g = x + (int64_t)M * NN * l;
             CC<R> *xl = xs + pp + PW * NN * l, *yl = ys + pp + PW * NN * l;
 #pragma unroll
-            for (int i = 0; i < NN; ++i) v[i] = __ldg(g + (int64_t)M * i);
+            for (int i = 0; i < NN; ++i) v[i] = ld_prev(g + (int64_t)M * i);
 #pragma unroll
             for (int i = 0; i < NN; ++i) xl[PW * i] = v[i];
             line_transform<R, NN, 0, sizeof(R) == 8>(
@@ -413,7 +419,7 @@ __global__ void __launch_bounds__(Cfg<R, NN>::KT, Cfg<R, NN>::KB) kline_kernel(c
         CC<R> *y = a.y + vec * a.vstride + idx;
         CC<R> v[NN];
 #pragma unroll
-        for (int k = 0; k < NN; ++k) v[k] = __ldg(x + KS * k);
+        for (int k = 0; k < NN; ++k) v[k] = ld_prev(x + KS * k);
         if constexpr (K::KS) {
 #pragma unroll
             for (int k = 0; k < NN; ++k) stash[T * k] = v[k];
@@ -436,7 +442,7 @@ __global__ void __launch_bounds__(Cfg<R, NN>::KT, Cfg<R, NN>::KB) kline_kernel(c
             [&](int k) {
                 L l;
                 if constexpr (K::KS) l.x = stash[T * k];
-                else l.x = __ldg(x + KS * k);
+                else l.x = ld_prev(x + KS * k);
                 if constexpr (sizeof(R) == 8) l.y = y[KS * k];
                 if constexpr (K::KV) l.v = pot[k];
                 else l.v = potential(k);
@@ -481,7 +487,7 @@ __global__ void __launch_bounds__(Cfg<R, NN>::CT, Cfg<R, NN>::CB) cube_line_kern
 #pragma unroll 1
         for (int l = t; l < P2; l += T) {
 #pragma unroll
-            for (int k = 0; k < NN; ++k) v[k] = __ldg(x + l + P2 * k);
+            for (int k = 0; k < NN; ++k) v[k] = ld_prev(x + l + P2 * k);
             if constexpr (G == NN) {
 #pragma unroll
                 for (int k = 0; k < NN; ++k) xs[l + P2 * k] = v[k];
@@ -494,7 +500,7 @@ __global__ void __launch_bounds__(Cfg<R, NN>::CT, Cfg<R, NN>::CB) cube_line_kern
         for (int k0 = 0; k0 < NN; k0 += G) {
             const int gn = G == NN ? NN : min(G, NN - k0);
             if constexpr (G < NN) {
-                for (int e = t; e < gn * P2; e += T) xs[e] = __ldg(x + k0 * P2 + e);
+                for (int e = t; e < gn * P2; e += T) xs[e] = ld_prev(x + k0 * P2 + e);
             }
             __syncthreads();
 #pragma unroll 1
@@ -597,7 +603,7 @@ __global__ void __launch_bounds__(kExchThreads, 3)
             const bool oka = p < m && q0 + c < m, okb = pt < m && p0 + c < m;
             zb[u] = okb ? y[pt + (int64_t)m * (p0 + c)] : G{R(0), R(0)};
             za[u] = oka ? y[p + (int64_t)m * (q0 + c)] : G{R(0), R(0)};
-            xa[u] = oka ? __ldg(x + p + (int64_t)m * (q0 + c)) : G{R(0), R(0)};
+            xa[u] = oka ? ld_prev(x + p + (int64_t)m * (q0 + c)) : G{R(0), R(0)};
             // in a diagonal tile both orders of a pair take the same table entry
             // (TINV's two halves agree to rounding only)
             const int lo = bi == bj ? min(c, tx) : tx, hi = bi == bj ? max(c, tx) : c;

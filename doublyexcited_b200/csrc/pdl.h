@@ -20,6 +20,39 @@ __device__ __forceinline__ void pdl_enter()
     asm volatile("griddepcontrol.launch_dependents;");
 }
 
+// Loads of what an earlier kernel wrote.  A kernel that waits inside is resident
+// while its predecessor still writes, so the non-coherent path (__ldg, and the
+// loads that const __restrict__ parameters allow the compiler), which takes the
+// data as constant from the kernel's first instruction to its last, is not for
+// them; tables that the handle's creation finished are read with __ldg.
+// volatile keeps them behind the wait; no memory clobber, so loads and stores of
+// other data may pass.
+__device__ __forceinline__ double2 ld_prev(const double2 *p)
+{
+    double2 v;
+    asm volatile("ld.global.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_prev(const float2 *p)
+{
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned long long ld_prev(const unsigned long long *p)
+{
+    unsigned long long v;
+    asm volatile("ld.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
+// the same from L2: partial sums that other blocks wrote
+__device__ __forceinline__ double2 ld_l2(const double2 *p)
+{
+    double2 v;
+    asm volatile("ld.global.cg.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
 template <class... P, class... A>
 cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
 {

@@ -33,7 +33,7 @@ __device__ __forceinline__ void tile_pair(int b, int &bi, int &bj)
 // in flight.
 template <class SI, int NOUT, int E, int IC>
 __global__ void __launch_bounds__(1024 / E, E == 4 ? 2 : 1)
-    update_sym_kernel(const __grid_constant__ UpdListT<SI, double2> U, const double2 *__restrict__ C, int ldc, int64_t m,
+    update_sym_kernel(const __grid_constant__ UpdListT<SI, double2> U, const double2 *C, int ldc, int64_t m,
                       double s, int upper)
 {
     pdl_enter();
@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(1024 / E, E == 4 ? 2 : 1)
 
 // out = (complex64) (a + s0 c b), one column, c from the device
 __global__ void __launch_bounds__(512)
-    axpc_f32_sym_kernel(float2 *__restrict__ out, const double2 *__restrict__ a, const double2 *__restrict__ b,
-                        double2 s0, const double2 *__restrict__ c_dev, int64_t m, float s)
+    axpc_f32_sym_kernel(float2 *out, const double2 *a, const double2 *b, double2 s0, const double2 *c_dev, int64_t m,
+                        float s)
 {
     pdl_enter();
     constexpr int E = 2, RY = 16;
@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(512)
     for (int u = 0; u < E; ++u) {
         const int64_t q = bj * 32 + ty + RY * u;
         const bool in = p < m && q < m;
-        av[u] = in ? __ldg(a + p + m * q) : make_double2(0.0, 0.0);
-        bv[u] = in ? __ldg(b + p + m * q) : make_double2(0.0, 0.0);
+        av[u] = in ? ld_prev(a + p + m * q) : make_double2(0.0, 0.0);
+        bv[u] = in ? ld_prev(b + p + m * q) : make_double2(0.0, 0.0);
     }
 #pragma unroll
     for (int u = 0; u < E; ++u) {
@@ -179,7 +179,7 @@ struct ResArgs {
 // full: 3 vector passes (2.5 for complex64) against 9 in separate kernels.
 template <class SW>
 __global__ void __launch_bounds__(256, 2)
-    residual_sym_kernel(const __grid_constant__ ResArgs A, int64_t m, double s, double2 *__restrict__ partial)
+    residual_sym_kernel(const __grid_constant__ ResArgs A, int64_t m, double s, double2 *partial)
 {
     pdl_enter();
     constexpr int E = 4, RY = 8;
