@@ -1126,7 +1126,9 @@ __global__ void small_gemm(const double2 *__restrict__ A, const double2 *__restr
 // Electron-exchange symmetry of an M x M block X (column-major, X(p,q) at
 // p + M q).  Tile pair (bi <= bj) of 32 x 32 tiles: PROJECT replaces X by
 // (X + s X^T)/2 in place (s = +1 singlet, -1 triplet); otherwise the block's
-// share of <X, X^T> = sum conj(X(p,q)) X(q,p) goes to work[block].
+// shares of |(X - X^T)/2|^2 and |(X + X^T)/2|^2 go to work[block].  The parts are
+// summed, and not <X, X^T> = their difference, in which a part of norm 1e-8
+// leaves no digit.
 template <bool PROJECT>
 __global__ void __launch_bounds__(256)
     exch_kernel(double2 *__restrict__ x, int64_t m, double s, double2 *__restrict__ work)
@@ -1157,13 +1159,10 @@ __global__ void __launch_bounds__(256)
             for (int c = ty; c < 32; c += 8) {
                 // pairs (p0+tx, q0+c) and its transpose partner
                 const double2 a = ta[tx][c], at = tb[c][tx];
-                double pr = a.x * at.x + a.y * at.y, pi = a.x * at.y - a.y * at.x;  // conj(a) at
-                if (bi != bj) {  // the partner tile's pair contributes conj(at) a
-                    pr += at.x * a.x + at.y * a.y;
-                    pi += at.x * a.y - at.y * a.x;
-                }
-                sr += pr;
-                si += pi;
+                const double dx = a.x - at.x, dy = a.y - at.y, ex = a.x + at.x, ey = a.y + at.y;
+                const double w = bi != bj ? 0.5 : 0.25;  // the partner tile's pair has the same two parts
+                sr += w * (dx * dx + dy * dy);
+                si += w * (ex * ex + ey * ey);
             }
         }
     }
@@ -2269,7 +2268,7 @@ cudaError_t update_exch_launch(const float2 *const *z, int nz, const double2 *co
     return cudaGetLastError();
 }
 
-cudaError_t exch_dot_launch(const double2 *x, int64_t m, double2 *out, double2 *work, cudaStream_t st)
+cudaError_t exch_parts_launch(const double2 *x, int64_t m, double2 *out, double2 *work, cudaStream_t st)
 {
     const int64_t t = (m + 31) / 32;
     if (m < 1 || t > 65535) return cudaErrorInvalidValue;

@@ -235,10 +235,10 @@ cudaError_t gs_pass2_launch(const double2 *const *qp, const double2 *const *vp, 
 cudaError_t gs_pass2_launch(const float2 *const *qp, const float2 *const *vp, int m, float2 *q, float2 *v,
                             const double2 *d2, int64_t len, double2 *cout, cudaStream_t st);
 
-// Electron-exchange symmetry of one M x M vector: out[0] = <X, X^T>
-// (Hermitian; work as for gram, >= (M/32)^2 + 1 elements), and the in-place
-// projection X <- (X + s X^T)/2.
-cudaError_t exch_dot_launch(const double2 *x, int64_t m, double2 *out, double2 *work, cudaStream_t st);
+// Electron-exchange symmetry of one M x M vector: out[0] = (|(X - X^T)/2|^2,
+// |(X + X^T)/2|^2) (work as for gram, >= (M/32)^2 + 1 elements), and the
+// in-place projection X <- (X + s X^T)/2.
+cudaError_t exch_parts_launch(const double2 *x, int64_t m, double2 *out, double2 *work, cudaStream_t st);
 // Y = sum_{i < nz} Z_i coef_i (complex64 columns, nz <= 8, coefficients on
 // the device) written projected, Y <- (Y + s Y^T)/2, in one pass.
 cudaError_t update_exch_launch(const float2 *const *z, int nz, const double2 *coef, double2 *y, int64_t m, double s,

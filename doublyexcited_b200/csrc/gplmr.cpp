@@ -79,6 +79,7 @@ struct Solver {
     // the same where the start held it to rounding (and now holds it exactly):
     // every vector of the iteration has it, and the products use it
     double exch_mult = 0.0;
+    static constexpr double kSectorRounding = 1e-14;  // relative norm outside the sector that counts as rounding
     unsigned refl_keep = 0xFFu;  // reflection sectors the start block reaches (bit c: sector c)
     bool exch_done = false;      // the last inner solve's output is already exchange-projected
     int64_t work_elems = 0;      // of h->d_work
@@ -1203,10 +1204,10 @@ struct Solver {
     // projection off.
     int detect_symmetry()
     {
-        double sign = 0.0, worst = 0.0;  // worst: largest | |<x, x^T>| - 1 |
+        double sign = 0.0, outside = 0.0;  // outside: largest squared norm outside the sector
         for (int j = 0; j < nev; ++j) {
-            cudaError_t e = exch_dot_launch(col(X, j), h->m, dR + j, h->d_work, st);
-            if (e != cudaSuccess) return cuda_error(e, "exch_dot");
+            cudaError_t e = exch_parts_launch(col(X, j), h->m, dR + j, h->d_work, st);
+            if (e != cudaSuccess) return cuda_error(e, "exch_parts");
             e = refl_corr_launch(col(X, j), h->nn, dG + 8 * j, h->d_work, st);
             if (e != cudaSuccess) return cuda_error(e, "refl_corr");
         }
@@ -1215,11 +1216,11 @@ struct Solver {
         DE_CUDA(cudaStreamSynchronize(st));
         unsigned keep = 0;
         for (int j = 0; j < nev; ++j) {
-            const double r = hbuf[j].x;
+            const double anti = hbuf[j].x, sym = hbuf[j].y, r = sym - anti;  // r = <x, x^T>
             const double sj = std::fabs(r - 1.0) < 1e-8 ? 1.0 : std::fabs(r + 1.0) < 1e-8 ? -1.0 : 0.0;
             if (j == 0) sign = sj;
             else if (sj != sign) sign = 0.0;
-            worst = std::max(worst, std::fabs(std::fabs(r) - 1.0));
+            outside = std::max(outside, std::min(anti, sym));
             const double2 *corr = hbuf + nev + 8 * j;  // <x, R_r x>, r = 0..7; r = 0 is |x|^2
             for (int c = 0; c < 8; ++c) {
                 double n2 = 0.0;
@@ -1228,15 +1229,17 @@ struct Solver {
             }
         }
         exch_sign = sign;
-        // A part of squared norm worst / 2 lies outside the sector.  Where that
-        // is rounding, the start is put into the sector exactly; every step
-        // then keeps X^T = sign X bit for bit (the products write it, the
-        // blocks are projected, and all else acts element by element).
-        // Only the default products write it.
+        // Where the part outside the sector is rounding (a start built by a few
+        // operations per element leaves 1e-16 of its norm there, the reference's
+        // guess none at all), the start is put into the sector exactly; every
+        // step then keeps X^T = sign X bit for bit (the products write it, the
+        // blocks are projected, and all else acts element by element).  A larger
+        // part is the caller's and stays in X.  Only the default products write
+        // the symmetry.
         bool exact = true;
         for (int sto = 0; sto <= (mixed ? 1 : 0); ++sto)
             for (int pass = 0; pass < 2; ++pass) exact = exact && h->ham.fam[sto][pass] == DE_MATVEC_FMA;
-        exch_mult = exact && worst < 2e-14 ? sign : 0.0;
+        exch_mult = exact && outside <= kSectorRounding * kSectorRounding ? sign : 0.0;
         if (exch_mult != 0.0) {
             for (int j = 0; j < nev; ++j) {
                 cudaError_t e = exch_project_launch(col(X, j), h->m, exch_mult, st);
