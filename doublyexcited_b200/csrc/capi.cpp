@@ -10,10 +10,6 @@
 
 #include "de_internal.h"
 
-namespace de {
-const char *last_error_str();
-}
-
 using namespace de;
 
 extern "C" {

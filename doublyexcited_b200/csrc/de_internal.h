@@ -18,6 +18,7 @@ using cplx = std::complex<double>;
 
 // ---- errors -----------------------------------------------------------
 int set_error(int code, const char *fmt, ...);
+const char *last_error_str();  // this thread's last message
 int cuda_error(cudaError_t e, const char *what);
 
 #define DE_CUDA(call)                                          \

@@ -81,6 +81,7 @@ struct Solver {
     double exch_mult = 0.0;
     static constexpr double kSectorRounding = 1e-14;  // relative norm outside the sector that counts as rounding
     unsigned refl_keep = 0xFFu;  // reflection sectors the start block reaches (bit c: sector c)
+    bool x_upper = false;        // X's lower half is not up to date (half())
     bool exch_done = false;      // the last inner solve's output is already exchange-projected
     int64_t work_elems = 0;      // of h->d_work
     bool z0_staged = false;      // the next inner solve's complex64 start Z_0 is already in Z32
@@ -1275,8 +1276,30 @@ struct Solver {
     // ---- main loop -------------------------------------------------------
     int run(double2 *x_dev, de_complex *e_out, int maxit, double tol, int outmodulus, de_stats *stats)
     {
-        auto tstart = clk::now();
         X = x_dev;
+        const int s = iterate(e_out, maxit, tol, outmodulus, stats);
+        if (s != DE_OK && x_upper) {  // the caller's X is the last iterate, in full
+            const std::string why = last_error_str();
+            if (complete_x() == DE_OK) cudaStreamSynchronize(st);
+            set_error(s, "%s", why.c_str());
+        }
+        return s;
+    }
+
+    // X's lower half, which the iteration leaves out (half())
+    int complete_x()
+    {
+        std::vector<cplx> one((size_t)nev * nev, 0.0);
+        for (int j = 0; j < nev; ++j) one[j + (size_t)nev * j] = 1.0;
+        DE_TRY(upload(one, dC));
+        DE_TRY(update(cl(X, nev), clw(X, nev), dC, nev, 1.0, 0.0));
+        x_upper = false;
+        return DE_OK;
+    }
+
+    int iterate(de_complex *e_out, int maxit, double tol, int outmodulus, de_stats *stats)
+    {
+        auto tstart = clk::now();
         DE_TRY(setup());
         DE_TRY(normalize(X, nev));
         if ((mixed || (nev > 1 && !compat)) && order > 1 && gm.usepetscflag != 0)
@@ -1425,6 +1448,7 @@ struct Solver {
                 std::vector<const double2 *> ps = cl(P, nev), aps = cl(AP, nev);
                 xs.insert(xs.end(), ps.begin(), ps.end());
                 axs.insert(axs.end(), aps.begin(), aps.end());
+                x_upper = half();
                 DE_TRY(update(xs, clw(X, nev), dC, 2 * nev, 1.0, 0.0, false));
                 DE_TRY(update(axs, clw(AX, nev), dC, 2 * nev, 1.0, 0.0, false));
             }
@@ -1438,12 +1462,7 @@ struct Solver {
             }
             ++it;
         }
-        if (half()) {  // X's lower half
-            std::vector<cplx> one((size_t)nev * nev, 0.0);
-            for (int j = 0; j < nev; ++j) one[j + (size_t)nev * j] = 1.0;
-            DE_TRY(upload(one, dC));
-            DE_TRY(update(cl(X, nev), clw(X, nev), dC, nev, 1.0, 0.0));
-        }
+        if (x_upper) DE_TRY(complete_x());
         DE_CUDA(cudaStreamSynchronize(st));
         for (int j = 0; j < nev; ++j) e_out[j] = de_complex{E[j].real(), E[j].imag()};
         if (stats) {

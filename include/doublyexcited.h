@@ -293,7 +293,9 @@ DE_API int de_heplus_orbitals(int n, const de_complex *h1, int numorbs, int herm
  * MAXIT,TOL,PRECONDITIONER,OUTMODULUS) gplmr.F90:9-374.  x is X(M,MB,NEV)
  * in/out (start vectors in, Ritz vectors out), e receives NEV eigenvalues.
  * outmodulus > 0 prints the reference's progress lines to stdout every
- * outmodulus iterations; 0 is silent.  stats may be NULL. */
+ * outmodulus iterations; 0 is silent.  stats may be NULL.  After an error in
+ * the iteration (DE_E_CHOLESKY, DE_E_ORTHO, DE_E_GEVP, ..) x of de_gplmr_eig_d
+ * holds the last iterate, x of de_gplmr_eig the start as it was passed. */
 DE_API int de_gplmr_eig(de_problem *h, de_complex *x, de_complex *e, int64_t m, int64_t mb,
                         de_complex sigma, int nev, int ns, int maxit, double tol,
                         const de_gmres *gm, int outmodulus, de_stats *stats);
