@@ -83,7 +83,6 @@ struct Solver {
     unsigned refl_keep = 0xFFu;  // reflection sectors the start block reaches (bit c: sector c)
     bool x_upper = false;        // X's lower half is not up to date (half())
     bool exch_done = false;      // the last inner solve's output is already exchange-projected
-    int64_t work_elems = 0;      // of h->d_work
     bool z0_staged = false;      // the next inner solve's complex64 start Z_0 is already in Z32
     // The mixed form's self-check: complex64 rounding amplified by the
     // conditioning of the k x k Gram (G^-1/2); a gross-failure detector.
@@ -171,9 +170,9 @@ struct Solver {
         }
         hbuf = h->h_small;  // pinned, 64 x 256 (the handle is locked for the solve)
         for (cudaEvent_t &e : up_ev) DE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        const int64_t wk = std::max<int64_t>(gram_work_elems(64, 128, D), dotdiag_work_elems(64, D));
-        DE_TRY(h->ensure_work(wk));
-        work_elems = wk;
+        // the last: normalize_residuals', behind the ticket of the fused sums
+        DE_TRY(h->ensure_work(std::max({gram_work_elems(64, 128, D), dotdiag_work_elems(64, D),
+                                        residual_sym_work_elems(nev, h->m) + 1})));
         return DE_OK;
     }
 
@@ -485,7 +484,7 @@ struct Solver {
     // x <- x / |x|, AX likewise, then the residuals: at the end of an iteration
     int normalize_residuals(std::vector<cplx> &e_host, std::vector<double> &res)
     {
-        if (!half() || residual_sym_work_elems(nev, h->m) >= work_elems) {
+        if (!half()) {
             DE_TRY(normalize(X, nev, AX));
             return residuals(e_host, res);
         }
