@@ -1718,7 +1718,7 @@ static cudaError_t gram_any(const ColListT<S> &L, const ColListT<S> &R, int64_t 
     bool one_shift = true;
     if (R.sigma.x != L.sigma.x || R.sigma.y != L.sigma.y)
         for (int j = 0; j < R.n; ++j) one_shift = one_shift && !R.b[j];
-    if (one_shift && gram_tile_supported(L.n, R.n)) return gram_tile_launch(L, R, len, herm, out, ldo, work, st, tri);
+    if (one_shift && gram_tile_supported(L, R)) return gram_tile_launch(L, R, len, herm, out, ldo, work, st, tri);
     // everything else on the FP64 tensor cores, warp tiles sized to the output
     const int mt = (L.n + 7) / 8, nt = (R.n + 7) / 8;
     if (mt == 1) return gram_tc_go<S, 1, 4>(L, R, len, herm, out, ldo, work, st, tri);

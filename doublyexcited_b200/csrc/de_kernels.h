@@ -141,8 +141,9 @@ cudaError_t gram_launch(const ColListF &L, const ColListF &R, int64_t len, int h
                         double2 *work, cudaStream_t st, int64_t tri = 0);
 
 // The same on output tiles fed through shared memory (gram_tile.cu), for the
-// shapes gram_tile_supported accepts; L and R share one shift (L.sigma).
-bool gram_tile_supported(int nl, int nr);
+// operands gram_tile_supported accepts; L and R share one shift (L.sigma).
+bool gram_tile_supported(const ColList &L, const ColList &R);
+bool gram_tile_supported(const ColListF &L, const ColListF &R);
 cudaError_t gram_tile_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out, int ldo,
                              double2 *work, cudaStream_t st, int64_t tri);
 cudaError_t gram_tile_launch(const ColListF &L, const ColListF &R, int64_t len, int herm, double2 *out, int ldo,

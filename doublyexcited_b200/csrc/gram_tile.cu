@@ -23,6 +23,7 @@
 // 8 x 16 projection stays on gram_tc's one-load form (294 us against 446).
 #include "de_kernels.h"
 #include "pdl.h"
+#include "tile_slots.h"
 #include "tri.h"
 
 #include <algorithm>
@@ -31,16 +32,13 @@
 namespace de {
 namespace {
 
-constexpr int kTile = 4;       // outputs of a warp: kTile x kTile
-constexpr int kWarps = 8;      // output tiles x row groups of a CTA
 constexpr int kFusedOut = 32;  // up to as many outputs the last CTA adds the partials
-constexpr int kMaxSlots = 40;  // distinct columns: 4 (tl + tr), and as many shift partners
 
 template <class S>
 struct GramTileArgs {
-    const S *col[kMaxSlots];            // the distinct columns
-    unsigned char shifted[kMaxSlots], partner[kMaxSlots];  // slots that become a - sigma b, and b's
-    unsigned char lslot[kTile * kWarps], rslot[kTile * kWarps];
+    const S *col[kMaxSlots];  // as TileSlots
+    unsigned char shifted[kMaxSlots], partner[kMaxSlots];
+    unsigned char lslot[kTile * kTileWarps], rslot[kTile * kTileWarps];
     double2 sigma;
     int64_t len;
     unsigned m;  // TRI: rows are the slots of an M x M upper half
@@ -86,7 +84,7 @@ __device__ __forceinline__ void sum_partials(const double2 *work, int nblk, int 
 // RT rows a stage.  Warp w: tile
 // w % (tl tr), row group w / (tl tr).
 template <class S, int RT, bool TRI>
-__global__ void __launch_bounds__(32 * kWarps) gram_tile_kernel(const __grid_constant__ GramTileArgs<S> a)
+__global__ void __launch_bounds__(32 * kTileWarps) gram_tile_kernel(const __grid_constant__ GramTileArgs<S> a)
 {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char gt_smem[];
@@ -242,7 +240,8 @@ cudaError_t tile_launch(const GramTileArgs<S> &a, int threads, size_t smem, cuda
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     int n = sms[dev].load(std::memory_order_relaxed);
     if (!n) {
-        cudaError_t e = cudaFuncSetAttribute(gram_tile_kernel<S, RT, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(gram_tile_kernel<S, RT, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kTileSmem);
         if (e != cudaSuccess) return e;
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         if (n <= 0) n = 148;
@@ -256,34 +255,24 @@ cudaError_t tile_launch(const GramTileArgs<S> &a, int threads, size_t smem, cuda
 }
 
 // One launch: L columns [l0, l0 + nl) against R columns [r0, r0 + nr), at
-// most kWarps tiles.
+// most kTileWarps tiles.
 template <class S>
 cudaError_t tile_go(const ColListT<S> &L, const ColListT<S> &R, int l0, int nl, int r0, int nr, int64_t len, int herm,
                     double2 *out, int ldo, double2 *work, cudaStream_t st, int64_t tri)
 {
     GramTileArgs<S> a{};
     a.sigma = L.sigma;
-    // slot of the column x - sigma y (y null: x)
-    const S *bs[kMaxSlots];
-    auto find = [&](const S *x, const S *y) {
-        for (int s = 0; s < a.nslots; ++s)
-            if (a.col[s] == x && bs[s] == y) return s;
-        const int s = a.nslots++;
-        a.col[s] = x;
-        bs[s] = y;
-        return s;
-    };
-    for (int i = 0; i < nl; ++i) a.lslot[i] = (unsigned char)find(L.a[l0 + i], L.b[l0 + i]);
-    for (int j = 0; j < nr; ++j) a.rslot[j] = (unsigned char)find(R.a[r0 + j], R.b[r0 + j]);
-    for (int s = 0, n = a.nslots; s < n; ++s)
-        if (bs[s]) {
-            a.shifted[a.nshift] = (unsigned char)s;
-            a.partner[a.nshift++] = (unsigned char)find(bs[s], nullptr);
-        }
+    TileSlots<S> t{};
+    if (!tile_slots(t, L.a + l0, L.b + l0, nl, R.a + r0, R.b + r0, nr)) return cudaErrorInvalidValue;
+    std::copy_n(t.col, t.n, a.col);
+    std::copy_n(t.shifted, t.nshift, a.shifted);
+    std::copy_n(t.partner, t.nshift, a.partner);
+    std::copy_n(t.l, sizeof t.l, a.lslot);
+    std::copy_n(t.r, sizeof t.r, a.rslot);
+    a.nslots = t.n;
+    a.nshift = t.nshift;
     a.tl = (nl + kTile - 1) / kTile;
     a.tr = (nr + kTile - 1) / kTile;
-    for (int i = nl; i < a.tl * kTile; ++i) a.lslot[i] = a.lslot[0];  // padding, dropped
-    for (int j = nr; j < a.tr * kTile; ++j) a.rslot[j] = a.rslot[0];
     a.len = tri ? tri_slots(tri) : len;
     a.m = (unsigned)tri;
     a.nl = nl;
@@ -292,11 +281,10 @@ cudaError_t tile_go(const ColListT<S> &L, const ColListT<S> &R, int l0, int nl, 
     a.work = work;
     a.out = out + l0 + (int64_t)ldo * r0;
     a.ldo = ldo;
-    const int tiles = a.tl * a.tr, groups = kWarps / tiles, threads = 32 * tiles * groups;
-    const int rt = groups >= 8 ? 256 : groups >= 4 ? 128 : 64;
+    const int tiles = a.tl * a.tr, threads = 32 * tiles * tile_groups(tiles), rt = tile_rows(tiles);
     const size_t stage = (size_t)a.nslots * rt * sizeof(S);
-    a.stages = (int)std::max<size_t>(2, std::min<size_t>(4, 111 * 1024 / stage));
-    const size_t smem = std::max<size_t>(stage * a.stages, kWarps * 16 * sizeof(double2));
+    a.stages = (int)std::max<size_t>(2, std::min<size_t>(4, (kTileSmem - 1024) / stage));
+    const size_t smem = std::max<size_t>(stage * a.stages, kTileWarps * 16 * sizeof(double2));
     if (tri) {
         if (rt == 256) return tile_launch<S, 256, true>(a, threads, smem, st);
         if (rt == 128) return tile_launch<S, 128, true>(a, threads, smem, st);
@@ -311,14 +299,12 @@ template <class S>
 cudaError_t tiles_go(const ColListT<S> &L, const ColListT<S> &R, int64_t len, int herm, double2 *out, int ldo,
                      double2 *work, cudaStream_t st, int64_t tri)
 {
-    if (!gram_tile_supported(L.n, R.n)) return cudaErrorInvalidValue;
-    const int tl = (L.n + kTile - 1) / kTile, tr = (R.n + kTile - 1) / kTile;
-    // blocks of at most kWarps tiles; the side with fewer tiles stays whole
-    const int bl = tr <= tl ? std::max(1, kWarps / tr) : tl, br = tr <= tl ? tr : std::max(1, kWarps / tl);
-    for (int i = 0; i < L.n; i += bl * kTile)
-        for (int j = 0; j < R.n; j += br * kTile) {
-            cudaError_t e = tile_go(L, R, i, std::min(bl * kTile, L.n - i), j, std::min(br * kTile, R.n - j), len, herm,
-                                    out, ldo, work, st, tri);
+    int bl, br;
+    tile_block(L.n, R.n, bl, br);
+    for (int i = 0; i < L.n; i += bl)
+        for (int j = 0; j < R.n; j += br) {
+            cudaError_t e = tile_go(L, R, i, std::min(bl, L.n - i), j, std::min(br, R.n - j), len, herm, out, ldo, work,
+                                    st, tri);
             if (e != cudaSuccess) return e;
         }
     return cudaSuccess;
@@ -327,12 +313,10 @@ cudaError_t tiles_go(const ColListT<S> &L, const ColListT<S> &R, int64_t len, in
 }  // namespace
 
 // Up to 24 x 24 (4.8 M rows: 2150 us against 3940 on the FP64 tensor cores); more
-// tiles re-read the columns of the other side too often: those go to gram_tc.
-bool gram_tile_supported(int nl, int nr)
-{
-    const int tl = (nl + kTile - 1) / kTile, tr = (nr + kTile - 1) / kTile;
-    return std::min(tl, tr) <= kWarps && tl * tr <= 36;
-}
+// tiles re-read the columns of the other side too often, and shifted columns
+// with too many distinct partners do not fit: those go to gram_tc.
+bool gram_tile_supported(const ColList &L, const ColList &R) { return tiles_fit(L.a, L.b, L.n, R.a, R.b, R.n); }
+bool gram_tile_supported(const ColListF &L, const ColListF &R) { return tiles_fit(L.a, L.b, L.n, R.a, R.b, R.n); }
 
 cudaError_t gram_tile_launch(const ColList &L, const ColList &R, int64_t len, int herm, double2 *out, int ldo,
                              double2 *work, cudaStream_t st, int64_t tri)
