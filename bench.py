@@ -157,9 +157,19 @@ def hammults_per_solve(w, iters):
     return nev + iters * (1 + ns) * (nev + nev * (2 * order + 1))
 
 
-def alg_flops(nn):
-    """Algorithmic FP64 flops of one vector-matvec: 6 axes x NN MACs x 2
-    flops x 2 (re, im) per element, plus the complex potential multiply-add."""
+def alg_flops(nn, exch=False):
+    """Flops that one vector-matvec of the line kernels executes: T commutes
+    with the reflection of an axis, so a line of NN = 2N+1 points takes
+    (N+1)^2 + N^2 real-by-complex multiply-adds (4 flops), and there are NN^5
+    lines per axis; then the complex potential multiply-add.  6 axes, or the 3
+    of one electron in an exchange-symmetric product."""
+    n = nn // 2
+    return (3 if exch else 6) * nn ** 5 * ((n + 1) ** 2 + n ** 2) * 4 + 8 * nn ** 6
+
+
+def dense_flops(nn):
+    """The same of the kernels that contract with the dense NN x NN matrix
+    (FP64 tensor cores)."""
     return 24 * nn ** 7 + 8 * nn ** 6
 
 
@@ -176,6 +186,57 @@ def alg_bytes(nn):
 # vector; part of it stays in L2).  Kernels without a capture report null.
 NCU_TRAFFIC_PER_VECTOR = {(13, "f32"): 237.0e6, (13, "f64"): 552.3e6, (13, "f32-exch"): 97.3e6,
                           (13, "f64-exch"): 250.3e6}
+
+def hbm_peak_gbs():
+    """(GB/s, source): the copy bandwidth measured on this kind of GPU."""
+    path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "MEASURED_PEAKS.json")
+    try:
+        with open(path) as f:
+            return float(json.load(f)["hbm_gbs"]), "MEASURED_PEAKS.json (copy bandwidth)"
+    except (OSError, ValueError, KeyError):
+        return 6650.0, "an earlier copy measurement (MEASURED_PEAKS.json is absent)"
+
+
+def product_roofline(nn, fp32, exch, seconds, flop_peak, flop_source, kernel=None, flops=None):
+    """One vector-matvec in `seconds` against both roofs.  The headline is the
+    memory side: the DRAM bytes that ncu counted for the kernels where they
+    were captured, else the least (x read and y written once).  `flops`: what
+    the kernels execute against the library GEMM's rate in that precision."""
+    key = (nn, ("f32" if fp32 else "f64") + ("-exch" if exch else ""))
+    least = (16 if fp32 else 32) * nn ** 6
+    traffic = NCU_TRAFFIC_PER_VECTOR.get(key) if kernel is None else None
+    peak, source = hbm_peak_gbs()
+    flops = alg_flops(nn, exch) if flops is None else flops
+    rate = (traffic or least) / seconds / 1e9 if seconds > 0 else 0.0
+    tf = flops / seconds / 1e12 if seconds > 0 else 0.0
+    return {"bound": "hbm", "achieved": rate, "peak": peak, "unit": "GB/s", "frac": rate / peak, "traffic": traffic,
+            "bytes": "DRAM bytes counted by ncu" if traffic else "x read and y written once (no capture)",
+            "kernel": (kernel or matvec_kernel_name(nn, fp32, exch)) + ", per vector-matvec",
+            "alg_bytes_per_vector": least, "achieved_gbs_alg": least / seconds / 1e9 if seconds > 0 else None,
+            "peak_source": source, "matvec_ms_per_vector": seconds * 1e3,
+            "flops": {"executed_per_vector": flops, "achieved": tf, "peak": flop_peak, "unit": "TFLOP/s",
+                      "frac": tf / flop_peak if flop_peak else None, "peak_source": flop_source}}
+
+
+FLOP_SOURCE = {False: "FP64 dense peak measured in this run: cuBLAS DGEMM 8192^3 (no FP64 entry in "
+                      "MEASURED_PEAKS.json)",
+               True: "FP32 CUDA-core peak measured in this run: cuBLAS SGEMM 8192^3 with TF32 off"}
+
+
+def exchange_symmetric(prob, x0, precision):
+    """Whether the solver takes its exchange-symmetric products for this start:
+    the mixed form or a block, every column exactly symmetric or every column
+    exactly antisymmetric, and the default kernels in every pass it uses."""
+    import numpy as np
+
+    if precision != "mixed" and x0.shape[1] < 2:
+        return False
+    for storage in ("c128", "c64") if precision == "mixed" else ("c128",):
+        if any(prob.get_matvec_launch(storage, p)[0] != "fma" for p in (0, 1)):
+            return False
+    cols = [x0[:, j].reshape(prob.m, prob.m) for j in range(x0.shape[1])]
+    return any(all(np.array_equal(c, s * c.T) for c in cols) for s in (1.0, -1.0))
+
 
 # The timed solves keep the library's matvec events on for the roofline
 # figures, on every 8th MATBLOCK call of each storage: all calls of one
@@ -368,14 +429,15 @@ class OracleBlockStep:
         return time.perf_counter() - t0
 
 
-def serve_roofline(reqs, matvecs, wall_s, peak_tflops):
-    """The served or batched stream's matvec work rate: the algorithmic
-    flops of every vector-matvec of every request (alg_flops at its grid)
-    over the stream's wall time.  The wall time also holds everything that
-    is not a matvec, so this is a lower bound on the matvec kernels' own
-    rate; the denominator is the measured FP32 peak, as for the mixed
-    form's matvec."""
-    flops = sum(matvecs[i] * alg_flops(2 * r["n"] + 1) for i, r in enumerate(reqs))
+def serve_roofline(reqs, matvecs, wall_s, peak_tflops, exch=False):
+    """The served or batched stream's matvec work rate: the executed flops of
+    every vector-matvec of every request (alg_flops at its grid; exch: all
+    are exchange-symmetric products, as in mixed solves from the mixes'
+    singlet and triplet starts) over the stream's wall time.  The wall time
+    also holds everything that is not a matvec, so this is a lower bound on
+    the matvec kernels' own rate; the denominator is the measured FP32 peak,
+    as for the mixed form's matvec."""
+    flops = sum(matvecs[i] * alg_flops(2 * r["n"] + 1, exch) for i, r in enumerate(reqs))
     achieved = flops / wall_s / 1e12
     return {"bound": "fp32-fma", "achieved": achieved, "peak": peak_tflops, "unit": "TFLOP/s",
             "frac": achieved / peak_tflops, "traffic": None,
@@ -535,14 +597,9 @@ def matvec_main(a):
         torch.cuda.synchronize()
         t_e2e = (time.perf_counter() - t0) / e2e_steps
     peak64, peak32 = fp64_peak_tflops(torch), fp32_peak_tflops(torch)
-    fl = alg_flops(nn) * nv
 
-    def roof(t, pk, ebytes, kernel):
-        ach = fl / t / 1e12
-        return {"bound": "tensor" if ebytes == 32 else "fp32-fma", "achieved": ach, "peak": pk, "unit": "TFLOP/s",
-                "frac": ach / pk, "traffic": NCU_TRAFFIC_PER_VECTOR.get((nn, "f64" if ebytes == 32 else "f32")),
-                "kernel": kernel, "ms_per_vector": t / nv * 1e3,
-                "achieved_gbs_alg": ebytes * nn ** 6 * nv / t / 1e9}
+    def roof(t, fp32, peak, **kw):
+        return product_roofline(nn, fp32, False, t / nv, peak, FLOP_SOURCE[fp32], **kw)
 
     cpu = None
     if not a.no_cpu_baseline:
@@ -556,12 +613,13 @@ def matvec_main(a):
                        "l2": f"block of {nv} x {16 * nn ** 6 / 1e6:.0f} MB"},
             "e2e": {"value": nv / t_e2e, "unit": "matvecs/s", "h2d_bytes_per_step": int(xh.nbytes),
                     "d2h_bytes_per_step": int(yh.nbytes)},
-            "roofline": roof(t64, peak64, 32, matvec_kernel_name(nn, False)),
+            "roofline": roof(t64, False, peak64),
             "mixed": {"value": nv / t32, "unit": "matvecs/s", "speedup_vs_fp64": t64 / t32,
                       "rel_err_vs_fp64_max": max(rel),
-                      "roofline": roof(t32, peak32, 16, matvec_kernel_name(nn, True))},
+                      "roofline": roof(t32, True, peak32)},
             "tensor_cores": {"fp64_value": nv / t64tc, "mixed_value": nv / t32tc,
-                             "fp64_roofline": roof(t64tc, peak64, 32, "hammult tc kernels <double> (DMMA)")},
+                             "fp64_roofline": roof(t64tc, False, peak64, kernel="hammult tc kernels <double> (DMMA)",
+                                                   flops=dense_flops(nn))},
             "cpu_baseline": cpu, "gpu_launches": int(launches), "clocks": clocks}
     print(json.dumps(line))
     return 0
@@ -611,7 +669,7 @@ def serve_main(a):
     # the mixed solver one solve at a time (what concurrency adds)
     mixed1 = run_served(de, seeded_start, cfg, "mixed", workers=1) if a.workload == "batch" else None
     reqs = serve_requests(cfg)
-    roofline = serve_roofline(reqs, mixed["matvecs"], mixed["wall_s"], fp32_peak_tflops(torch))
+    roofline = serve_roofline(reqs, mixed["matvecs"], mixed["wall_s"], fp32_peak_tflops(torch), exch=True)
     cpu = None if a.no_cpu_baseline else serve_cpu_baseline(cfg, reqs, mixed["iters"])
     both = [i for i in mixed["e"] if mixed["conv"][i] and fp64["conv"][i]]
     de_max = max((float(np.max(np.abs(np.sort_complex(mixed["e"][i]) - np.sort_complex(fp64["e"][i]))))
@@ -809,27 +867,17 @@ def main():
     peak = fp64_peak_tflops(torch)
     peak32 = fp32_peak_tflops(torch)
 
-    exch = a.precision == "mixed" or w["nev"] > 1
+    exch = exchange_symmetric(prob, x0, a.precision)
 
-    def roof(pr, fp32, pk, src):
+    def roof(pr, fp32, pk):
         ms = pr["pass_a_ms"] + pr["pass_b_ms"]
         vecs = max(1, pr["vectors"])
-        ach = alg_flops(nn) * vecs / (ms / 1e3) / 1e12 if ms > 0 else 0.0
-        ebytes = 16 if fp32 else 32
-        return {"bound": "tensor" if not fp32 else "fp32-fma", "achieved": ach, "peak": pk, "unit": "TFLOP/s",
-                "frac": ach / pk if pk else None,
-                "traffic": NCU_TRAFFIC_PER_VECTOR.get((nn, ("f32" if fp32 else "f64") + ("-exch" if exch else ""))),
-                "kernel": matvec_kernel_name(nn, fp32, exch) + ", per vector-matvec",
-                "alg_flops_per_vector": alg_flops(nn), "alg_bytes_per_vector": ebytes * nn ** 6,
-                "achieved_gbs_alg": ebytes * nn ** 6 * vecs / (ms / 1e3) / 1e9 if ms > 0 else None,
-                "matvec_ms_per_vector": ms / vecs, "pass_a_ms": pr["pass_a_ms"] / vecs,
-                "pass_b_ms": pr["pass_b_ms"] / vecs, "vectors": pr["vectors"], "device_ms_total": ms,
-                "peak_source": src}
+        return dict(product_roofline(nn, fp32, exch, ms / vecs / 1e3, pk, FLOP_SOURCE[fp32]),
+                    pass_a_ms=pr["pass_a_ms"] / vecs, pass_b_ms=pr["pass_b_ms"] / vecs, vectors=pr["vectors"],
+                    device_ms_total=ms)
 
-    src64 = "FP64 dense peak measured in this run: cuBLAS DGEMM 8192^3 (no FP64 entry in MEASURED_PEAKS.json)"
-    src32 = "FP32 CUDA-core peak measured in this run: cuBLAS SGEMM 8192^3 with TF32 off"
-    roof64 = roof(prof, False, peak, src64)
-    roof32 = roof(head["prof32"], True, peak32, src32) if head["prof32"]["vectors"] else None
+    roof64 = roof(prof, False, peak)
+    roof32 = roof(head["prof32"], True, peak32) if head["prof32"]["vectors"] else None
     # the dominant kernel of the run heads the line
     if roof32 and roof32["device_ms_total"] > roof64["device_ms_total"]:
         roofline, roofline_other = roof32, roof64
