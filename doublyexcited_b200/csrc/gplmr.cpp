@@ -72,7 +72,6 @@ struct Solver {
     // main-program storage keeps zero
     const cplx gm_shift{0.0, 0.0};
     double2 *GV = nullptr, *dGs = nullptr;
-    float2 *LV32 = nullptr, *LQ32 = nullptr;  // the same in complex64 (unused by the mixed s-step solve)
     float2 *Z32 = nullptr;  // mixed inner solve: the power basis Z_0..Z_order (complex64)
     bool mixed = false;
     double exch_sign = 0.0;     // +1 / -1: exchange symmetry of the start block, 0: none
@@ -84,9 +83,7 @@ struct Solver {
     bool x_upper = false;        // X's lower half is not up to date (half())
     bool exch_done = false;      // the last inner solve's output is already exchange-projected
     bool z0_staged = false;      // the next inner solve's complex64 start Z_0 is already in Z32
-    // The mixed form's self-check: complex64 rounding amplified by the
-    // conditioning of the k x k Gram (G^-1/2); a gross-failure detector.
-    static constexpr double kOrthoTolMixed = 1e-3;
+    static constexpr double kOrthoTol = 1e-10;  // the FP64 inner solve's self-check
     double2 *dG = nullptr, *dC = nullptr, *dE = nullptr, *dR = nullptr, *dT = nullptr, *dT2 = nullptr;
     double2 *dOC = nullptr;  // orth_normalize's coefficients
     double2 *dB1 = nullptr, *dB2 = nullptr, *dRinv2 = nullptr, *dVC = nullptr;  // block_orthonormalize
@@ -401,7 +398,7 @@ struct Solver {
         if (flags & 1) return set_error(DE_E_CHOLESKY, "Cholesky failed!!! (cholQR breakdown)");
         if (flags & 4)
             return set_error(DE_E_ORTHO, "AACK DOTS: inner-solve orthonormality self-check above %g",
-                             mixed ? kOrthoTolMixed : 1e-10);
+                             kOrthoTol);
         if (flags & 8) return set_error(DE_E_SVD, "inner-solve Gram matrix is singular");
         return DE_OK;
     }
@@ -515,19 +512,7 @@ struct Solver {
     }
 
     // ---- inner solve -------------------------------------------------------
-    // Storage-generic pieces: S = double2 (plain FP64) or float2 (mixed).
-    template <class S>
-    S *lv_buf()
-    {
-        if constexpr (std::is_same_v<S, double2>) return LV;
-        else return LV32;
-    }
-    template <class S>
-    S *lq_buf()
-    {
-        if constexpr (std::is_same_v<S, double2>) return LQ;
-        else return LQ32;
-    }
+    // S = double2 (plain FP64) or float2 (the mixed form's power basis)
     template <class S>
     static ColListT<S> colsT(S *base, int k, int64_t D)
     {
@@ -577,10 +562,9 @@ struct Solver {
         return DE_OK;
     }
     // Y[0..nout) -= sum_i X_i C(i, j) (in place on Y)
-    template <class S>
-    int update_sub(const S *xb, int nin, S *yb, int nout, const double2 *c, int ldc)
+    int update_sub(const double2 *xb, int nin, double2 *yb, int nout, const double2 *c, int ldc)
     {
-        UpdListT<S, S> U{};
+        UpdList U{};
         U.nin = nin;
         U.nout = nout;
         if (nin > kMaxCols || nout > 16) return set_error(DE_E_INVALID, "update too wide");
@@ -590,49 +574,29 @@ struct Solver {
             U.beta[j] = make_double2(1.0, 0.0);
         }
         U.alpha = make_double2(-1.0, 0.0);
-        cudaError_t e;
-        if constexpr (std::is_same_v<S, double2>) e = update_any(U, c, ldc);
-        else e = update_launch(U, c, ldc, D, st);
+        cudaError_t e = update_any(U, c, ldc);
         if (e != cudaSuccess) return cuda_error(e, "update");
         return DE_OK;
     }
 
-    // H x (the inner solve's callback) and (H - sigma) x
-    template <class S>
-    int mult_plain(const S *x, S *y, int k)
+    // (H - sigma) x in complex64
+    int inner_mult_shifted(const float2 *x, float2 *y, int k)
     {
-        if constexpr (std::is_same_v<S, double2>) {
-            return inner_mult(x, y, k);
-        } else {
-            mv_exec += k;
-            mv_ref += k;
-            return h->matblock32(x, y, k);
-        }
-    }
-    template <class S>
-    int mult_shifted(const S *x, S *y, int k)
-    {
-        if constexpr (std::is_same_v<S, double2>) {
-            return inner_mult_shifted(x, y, k);
-        } else {
-            mv_exec += k;
-            mv_ref += k;
-            const cplx ms = -sigma;
-            return h->matblock32(x, y, k, make_double2(ms.real(), ms.imag()), exch_mult);
-        }
+        mv_exec += k;
+        mv_ref += k;
+        const cplx ms = -sigma;
+        return h->matblock32(x, y, k, make_double2(ms.real(), ms.imag()), exch_mult);
     }
 
     // myhgramschmidt_many with factors (1,0): two classical passes of the
     // (H-sigma)-weighted Gram-Schmidt of the pair (q, v) against the first m
-    // pairs of (qbase, vbase) (default: the Krylov blocks LQ, LV).
-    template <class S>
-    int hgram(int m, S *q, S *v, S *qbase = nullptr, S *vbase = nullptr)
+    // pairs of the Krylov blocks LQ, LV.
+    int hgram(int m, double2 *q, double2 *v)
     {
-        S *LQs = qbase ? qbase : lq_buf<S>(), *LVs = vbase ? vbase : lv_buf<S>();
-        std::vector<const S *> qp(m), vp(m);
+        std::vector<const double2 *> qp(m), vp(m);
         for (int i = 0; i < m; ++i) {
-            qp[i] = LQs + (int64_t)i * D;
-            vp[i] = LVs + (int64_t)i * D;
+            qp[i] = col(LQ, i);
+            vp[i] = col(LV, i);
         }
         cudaError_t e;
         if (m == 0) {  // nothing to project: the two passes only normalise
@@ -643,7 +607,7 @@ struct Solver {
         if (m <= 16) {
             // pass 1 with the pass-2 coefficients fused into its update; the
             // intermediate normalisation of the reference cancels exactly.
-            DE_TRY(gramT(colsT(LQs, m, D), colsT(q, 1, D), dT, m));
+            DE_TRY(gramT(colsT(LQ, m, D), colsT(q, 1, D), dT, m));
             e = gs_pass1_launch(qp.data(), vp.data(), m, q, v, dT, D, h->d_work, dT2, st);
             if (e != cudaSuccess) return cuda_error(e, "gs_pass1");
             e = gs_pass2_launch(qp.data(), vp.data(), m, q, v, dT2, D, dR, st);
@@ -651,7 +615,7 @@ struct Solver {
             return DE_OK;
         }
         for (int pass = 0; pass < 2; ++pass) {
-            DE_TRY(gramT(colsT(LQs, m, D), colsT(q, 1, D), dT, m));
+            DE_TRY(gramT(colsT(LQ, m, D), colsT(q, 1, D), dT, m));
             e = gs_update_launch(qp.data(), vp.data(), m, q, v, dT, D, h->d_work, dR, st);
             if (e != cudaSuccess) return cuda_error(e, "gs_update");
         }
@@ -668,10 +632,9 @@ struct Solver {
     // V_new <- (V_new - V (C_1 + C_2)) R_1^-1 R_2^-1, which is formed at the
     // end.  For the compatibility mode, whose pairs are not q = (H - sigma) v;
     // basic_block needs no V.
-    template <class S>
-    int block_orthonormalize(S *Q, S *V, int m0, int k)
+    int block_orthonormalize(double2 *Q, double2 *V, int m0, int k)
     {
-        S *qb = Q + (int64_t)m0 * D;
+        double2 *qb = Q + (int64_t)m0 * D;
         double2 *gs[2] = {dB1, dB2}, *rs[2] = {dRinv, dRinv2};
         for (int pass = 0; m0 > 0 && pass < 2; ++pass) {
             DE_TRY(gramT(colsT(Q, m0, D), colsT(qb, k, D), gs[pass], m0));
@@ -749,7 +712,7 @@ struct Solver {
         DE_TRY(part(LQ, k, LQ, k, dC, k, 1.0, 0.0));
         mv_ref += k;  // the self-check's product (harmonic_ritz_small.F90:221-242)
         DE_TRY(gramT(colsT(LQ, k, D), colsT(LQ, k, D), dG, k));
-        cudaError_t e = small_ortho_check_launch(dG, k, dFlags, st, 1e-10);
+        cudaError_t e = small_ortho_check_launch(dG, k, dFlags, st, kOrthoTol);
         if (e != cudaSuccess) return cuda_error(e, "small_ortho_check");
         double2 *cf = dVC;  // the blocks' coefficients, one after the other
         for (int io = 0; io < order; ++io) {
@@ -818,21 +781,13 @@ struct Solver {
 
     // basicblocklansolve harmonic_ritz_small.F90:258-324 on block b (k
     // columns), in place: b <- V (Q^H V_1) G^{1/2}: one column, or the
-    // compatibility mode's blocks.  S is the storage of the Krylov blocks; b is
-    // always FP64.
-    template <class S>
+    // compatibility mode's blocks.
     int basic(double2 *b, int k)
     {
-        S *V = lv_buf<S>(), *Q = lq_buf<S>();
-        const double ortho_tol = std::is_same_v<S, double2> ? 1e-10 : kOrthoTolMixed;
+        double2 *V = LV, *Q = LQ;
         // harm_orthog_oneblock :161-244
-        if constexpr (std::is_same_v<S, double2>) {
-            DE_CUDA(cudaMemcpyAsync(V, b, (size_t)k * D * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-        } else {
-            cudaError_t e = to_f32_launch(b, V, (int64_t)k * D, st);
-            if (e != cudaSuccess) return cuda_error(e, "to_f32");
-        }
-        DE_TRY(mult_shifted(V, Q, k));
+        DE_CUDA(cudaMemcpyAsync(V, b, (size_t)k * D * sizeof(double2), cudaMemcpyDeviceToDevice, st));
+        DE_TRY(inner_mult_shifted(V, Q, k));
         std::vector<cplx> gsq;
         if (k == 1) {  // 1 x 1 Gram: its square roots on the device
             DE_TRY(gramT(colsT(Q, 1, D), colsT(Q, 1, D), dG, 1));
@@ -859,18 +814,18 @@ struct Solver {
         // as V (counted as the reference's product; the compatibility mode's
         // first-column-only product is not linear and is recomputed).
         if (compat) {
-            DE_TRY(mult_shifted(V, Q, k));
+            DE_TRY(inner_mult_shifted(V, Q, k));
         } else {
             mv_ref += k;
         }
         DE_TRY(gramT(colsT(Q, k, D), colsT(Q, k, D), dG, k));
         {
-            cudaError_t e = small_ortho_check_launch(dG, k, dFlags, st, ortho_tol);
+            cudaError_t e = small_ortho_check_launch(dG, k, dFlags, st, kOrthoTol);
             if (e != cudaSuccess) return cuda_error(e, "small_ortho_check");
         }
         // fast_harmritz_setup :86-158 (maxiter = M^2 never truncates a block)
         for (int io = 0; io < order; ++io) {
-            S *vb = V + (int64_t)io * k * D, *qb = Q + (int64_t)io * k * D;
+            double2 *vb = V + (int64_t)io * k * D, *qb = Q + (int64_t)io * k * D;
             if (io > 0 && !compat) {
                 // H v_{io-1} = (H - sigma) v_{io-1} + sigma v_{io-1} = q_{io-1} + sigma v_{io-1}:
                 // the Gram-Schmidt steps apply the same combinations to q and
@@ -881,10 +836,10 @@ struct Solver {
                 cudaError_t e = axpy_launch(vb, Q + (int64_t)(io - 1) * k * D, V + (int64_t)(io - 1) * k * D,
                                             make_double2(sigma.real(), sigma.imag()), (int64_t)k * D, st);
                 if (e != cudaSuccess) return cuda_error(e, "axpy");
-                DE_TRY(mult_shifted(vb, qb, k));
+                DE_TRY(inner_mult_shifted(vb, qb, k));
             } else if (io > 0) {
-                DE_TRY(mult_plain(V + (int64_t)(io - 1) * k * D, vb, k));
-                DE_TRY(mult_shifted(vb, qb, k));
+                DE_TRY(inner_mult(V + (int64_t)(io - 1) * k * D, vb, k));
+                DE_TRY(inner_mult_shifted(vb, qb, k));
             } else {
                 mv_ref += compat ? 1 : k;  // the reference recomputes the product checked above
             }
@@ -1086,7 +1041,7 @@ struct Solver {
         }
         z0_staged = false;
         for (int i = 1; i <= order; ++i)
-            DE_TRY(mult_shifted<float2>(Z32 + (int64_t)(i - 1) * k * D, Z32 + (int64_t)i * k * D, k));
+            DE_TRY(inner_mult_shifted(Z32 + (int64_t)(i - 1) * k * D, Z32 + (int64_t)i * k * D, k));
         mv_ref += (order + 1) * k;  // the reference forms (2 order + 1) k products
         if (k == 1 && nz <= 7) {
             // one column: the Hermitian Gram of the nz basis vectors (read
@@ -1180,7 +1135,7 @@ struct Solver {
             if (s == DE_OK) s = symmetry_project(b, k);
         } else {
             s = equilibrate(b, k);
-            if (s == DE_OK) s = k > 1 && !compat ? basic_block(b, k) : basic<double2>(b, k);
+            if (s == DE_OK) s = k > 1 && !compat ? basic_block(b, k) : basic(b, k);
             // Block solves (NEV > 1) keep the start block's sectors too: in
             // exact arithmetic the iteration never leaves them, but FP64
             // rounding leaks into the others, and GPLMR then converges to
