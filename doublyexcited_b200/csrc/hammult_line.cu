@@ -286,45 +286,39 @@ __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.la
 // more resident CTAs than that allows spill or serialise the loads).
 //   PW, PB  plane: run of adjacent p (128 bytes where it fits), min CTAs/SM
 //   KT, KB  kline: threads, min CTAs/SM; KS stash the line in shared memory
-//           for the V x term instead of reading it again; KV all of a line's
-//           potential values loaded before the sums.  complex64 takes both from
-//           NN = 9 on (loads between the sums wait for their turn among the
-//           ordered memory operations: us per product without, with, at NN =
-//           11 19.0, 18.5; 17 262, 257; 21 1084, 1066); below, lines are
-//           short and more CTAs hide them.  complex128 has registers for KV at
-//           some sizes only
+//           for the V x term instead of reading it again
 //   CT, CB  cube: threads, min CTAs/SM; CG slabs of x staged at a time (NN =
 //           the whole cube; less where two cubes exceed shared memory)
 template <class R, int NN>
 struct Shape;
-#define LINE_SHAPE(RT, NNV, PWV, PBV, KTV, KBV, KSV, KVV, CTV, CBV, CGV)                     \
+#define LINE_SHAPE(RT, NNV, PWV, PBV, KTV, KBV, KSV, CTV, CBV, CGV)                          \
     template <>                                                                              \
     struct Shape<RT, NNV> {                                                                  \
-        static constexpr int PW = PWV, PB = PBV, KT = KTV, KB = KBV, KS = KSV, KV = KVV;     \
+        static constexpr int PW = PWV, PB = PBV, KT = KTV, KB = KBV, KS = KSV;               \
         static constexpr int CT = CTV, CB = CBV, CG = CGV;                                   \
     };
-LINE_SHAPE(double, 3, 32, 8, 128, 5, 1, 0, 32, 31, 3)
-LINE_SHAPE(double, 5, 16, 8, 128, 5, 1, 0, 32, 28, 5)
-LINE_SHAPE(double, 7, 16, 5, 128, 3, 1, 1, 64, 6, 7)
-LINE_SHAPE(double, 9, 16, 2, 128, 4, 1, 0, 96, 3, 9)
-LINE_SHAPE(double, 11, 8, 6, 128, 3, 1, 0, 128, 3, 11)
-LINE_SHAPE(double, 13, 16, 2, 128, 3, 1, 0, 192, 2, 13)
-LINE_SHAPE(double, 15, 8, 3, 128, 3, 1, 1, 128, 2, 8)
-LINE_SHAPE(double, 17, 8, 2, 128, 3, 1, 1, 320, 1, 17)
-LINE_SHAPE(double, 19, 8, 2, 128, 3, 1, 1, 384, 1, 19)
-LINE_SHAPE(double, 21, 4, 2, 128, 3, 1, 0, 224, 1, 7)
-LINE_SHAPE(double, 23, 4, 2, 256, 1, 0, 0, 96, 1, 3)
-LINE_SHAPE(float, 3, 64, 8, 128, 10, 0, 0, 32, 31, 3)
-LINE_SHAPE(float, 5, 64, 4, 128, 9, 0, 0, 32, 31, 5)
-LINE_SHAPE(float, 7, 32, 4, 128, 8, 0, 0, 64, 20, 7)
-LINE_SHAPE(float, 9, 32, 2, 128, 6, 1, 1, 96, 13, 9)
-LINE_SHAPE(float, 11, 16, 5, 128, 6, 1, 1, 128, 7, 11)
-LINE_SHAPE(float, 13, 16, 3, 128, 6, 1, 1, 192, 6, 13)
-LINE_SHAPE(float, 15, 16, 3, 128, 4, 1, 1, 256, 3, 15)
-LINE_SHAPE(float, 17, 16, 2, 256, 2, 1, 1, 320, 2, 17)
-LINE_SHAPE(float, 19, 16, 2, 256, 3, 1, 1, 192, 2, 19)
-LINE_SHAPE(float, 21, 8, 2, 128, 3, 1, 1, 448, 1, 21)
-LINE_SHAPE(float, 23, 8, 2, 128, 3, 1, 1, 544, 1, 23)
+LINE_SHAPE(double, 3, 32, 8, 128, 5, 1, 32, 31, 3)
+LINE_SHAPE(double, 5, 16, 8, 128, 5, 1, 32, 28, 5)
+LINE_SHAPE(double, 7, 16, 5, 128, 3, 1, 64, 6, 7)
+LINE_SHAPE(double, 9, 16, 2, 128, 4, 1, 96, 3, 9)
+LINE_SHAPE(double, 11, 8, 6, 128, 3, 1, 128, 3, 11)
+LINE_SHAPE(double, 13, 16, 2, 128, 3, 1, 192, 2, 13)
+LINE_SHAPE(double, 15, 8, 3, 128, 3, 1, 128, 2, 8)
+LINE_SHAPE(double, 17, 8, 2, 128, 3, 1, 320, 1, 17)
+LINE_SHAPE(double, 19, 8, 2, 128, 3, 1, 384, 1, 19)
+LINE_SHAPE(double, 21, 4, 2, 128, 3, 1, 224, 1, 7)
+LINE_SHAPE(double, 23, 4, 2, 256, 1, 0, 96, 1, 3)
+LINE_SHAPE(float, 3, 64, 8, 128, 10, 1, 32, 31, 3)
+LINE_SHAPE(float, 5, 64, 4, 128, 9, 1, 32, 31, 5)
+LINE_SHAPE(float, 7, 32, 4, 128, 8, 1, 64, 20, 7)
+LINE_SHAPE(float, 9, 32, 2, 128, 6, 1, 96, 13, 9)
+LINE_SHAPE(float, 11, 16, 5, 128, 6, 1, 128, 7, 11)
+LINE_SHAPE(float, 13, 16, 3, 128, 6, 1, 192, 6, 13)
+LINE_SHAPE(float, 15, 16, 3, 128, 4, 1, 256, 3, 15)
+LINE_SHAPE(float, 17, 16, 2, 256, 2, 1, 320, 2, 17)
+LINE_SHAPE(float, 19, 16, 2, 256, 3, 1, 192, 2, 19)
+LINE_SHAPE(float, 21, 8, 2, 128, 3, 1, 448, 1, 21)
+LINE_SHAPE(float, 23, 8, 2, 128, 3, 1, 544, 1, 23)
 #undef LINE_SHAPE
 
 template <class R, int NN>
@@ -333,6 +327,12 @@ struct Cfg : Shape<R, NN> {
     static constexpr int P2 = NN * NN, M = NN * NN * NN;
     static constexpr int PT = (S::PW * NN + 31) / 32 * 32;  // plane threads
     static constexpr int RUNS = (M + S::PW - 1) / S::PW;
+    // kline: all of a line's potential values loaded before the sums, where
+    // loads wait for their turn among the ordered memory operations.  complex64
+    // has the registers for them (us per product without, with, at NN = 11 19.0,
+    // 18.5; 17 262, 257; 21 1084, 1066; equal up to 9); complex128 has not
+    // (without, with: NN = 17 682, 693; equal elsewhere, but 21 3014, 2980).
+    static constexpr bool KV = sizeof(R) == 4;
     static constexpr size_t PSMEM = (size_t)2 * S::PW * P2 * sizeof(CC<R>);
     static constexpr size_t KSMEM = S::KS ? (size_t)S::KT * NN * sizeof(CC<R>) : 0;
     static constexpr size_t CSMEM = (size_t)(NN + S::CG) * P2 * sizeof(CC<R>);
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(Cfg<R, NN>::KT, Cfg<R, NN>::KB) kline_kernel(c
             const R pr = fma(l.v, a.vsr, a.shr), pi = fma(l.v, a.vsi, a.shi);
             return G2<R>{yr + (pr * xr - pi * xi), yi + (pr * xi + pi * xr)};
         };
-        line_transform<R, NN, K::KV && sizeof(R) == 4 ? 0 : 2, true>(
+        line_transform<R, NN, K::KV ? 0 : 2, true>(
             v,
             [&](int k) {
                 L l;
@@ -465,6 +465,12 @@ __global__ void __launch_bounds__(Cfg<R, NN>::KT, Cfg<R, NN>::KB) kline_kernel(c
 // Y += S2 (T_i1 + T_j1 + T_k1) X (ADD; else Y = ...) on one column X(:, q): k
 // lines straight from global memory (lanes along i, j), the i and j lines
 // through shared memory.
+//
+// A CTA per column, so the loop over units makes one turn.  Without it the
+// compiler keeps fewer of a line's loads in flight (complex64 at NN = 11: 52
+// registers instead of 70), and the launch shapes above fit no more: blocks of 8
+// at NN = 11 took 172 us instead of 143 in complex64, 320 instead of 325 in
+// complex128.
 template <class R, int NN, bool ADD>
 __global__ void __launch_bounds__(Cfg<R, NN>::CT, Cfg<R, NN>::CB) cube_line_kernel(const __grid_constant__ LineArgs<R> a)
 {
