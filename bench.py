@@ -184,8 +184,8 @@ def alg_bytes(nn):
 # matvec-n6`), the three kernels' bytes over 2 vectors; "-exch": the two
 # kernels of an exchange-symmetric product inside the mixed solve at N=6 (one
 # vector; part of it stays in L2).  Kernels without a capture report null.
-NCU_TRAFFIC_PER_VECTOR = {(13, "f32"): 237.0e6, (13, "f64"): 552.3e6, (13, "f32-exch"): 97.3e6,
-                          (13, "f64-exch"): 250.3e6}
+NCU_TRAFFIC_PER_VECTOR = {(13, "f32"): 233.8e6, (13, "f64"): 551.0e6, (13, "f32-exch"): 97.2e6,
+                          (13, "f64-exch"): 254.2e6}
 
 def hbm_peak_gbs():
     """(GB/s, source): the copy bandwidth measured on this kind of GPU."""

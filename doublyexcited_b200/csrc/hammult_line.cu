@@ -42,21 +42,26 @@
 //   two outputs ahead instead.
 //
 // Measured on B200, us per vector, one vector per call, before (the even/odd
-// slab, streaming or cube kernels, whichever the grid had) and now, as plane +
-// kline + cube; the HBM time of 8 vector passes at 6.54 TB/s in brackets
-// where the vectors exceed L2:
+// slab, streaming or cube kernels, whichever the grid had) and now; in
+// parentheses the two passes by events between them (plane + kline, cube), in
+// brackets the HBM time of 8 vector passes at 6.54 TB/s where the vectors
+// exceed L2:
 //
-//   NN        complex128                               complex64
-//    7    16.8 ->    8.0                            14.2 ->    7.6
-//   11    64.8 ->   33.9 ( 9.3 + 10.1 + 14.8)       33.7 ->   19.5 ( 5.9 + 5.7 + 7.6)
-//   13   169   ->  117   (33   + 40   + 47  ) [94]  80.3 ->   42.3 (13 + 11 + 18)
-//   15   450   ->  314   (80   + 93   + 133 ) [223]  239 ->  123   (39 + 42 + 47) [111]
-//   17  1130   ->  636   (151  + 200  + 280 ) [472]  640 ->  257   (76 + 89 + 94) [236]
-//   19  2100   -> 1636   (338  + 399  + 640 ) [921] 1430 ->  663   (161 + 169 + 235) [460]
-//   21  6250   -> 2910   (674  + 752  + 1300) [1680] 3460 -> 1102  (312 + 302 + 477) [839]
-//   23 23700   -> 7990   (1190 + 1350 + 4210) [2900] 15400 -> 2007 (572 + 520 + 855) [1450]
+//   NN        complex128                       complex64
+//    7    16.8 ->    8.0                    14.2 ->    7.9
+//   11    64.8 ->   34.1 (  25 +   18)      33.7 ->   18.5 (  16 +   12)
+//   13   169   ->  121   (  80 +   49) [94]  80.3 ->   42.9 (  29 +   22)
+//   15   450   ->  315   ( 189 +  134) [223]  239 ->  119   (  82 +   47) [111]
+//   17  1130   ->  683   ( 405 +  287) [472]  640 ->  257   ( 170 +   96) [236]
+//   19  2100   -> 1640   ( 828 +  635) [921] 1430 ->  648   ( 338 +  230) [460]
+//   21  6250   -> 2985   (1608 + 1266) [1680] 3460 -> 1070  ( 617 +  449) [839]
+//   23 23700   -> 7950   (3046 + 4061) [2900] 15400 -> 1975 (1084 +  851) [1450]
 //
-// complex64 is at 70-92 % of the HBM time from NN = 15 on.  complex128 is held
+// From NN = 19 on the passes' sum is below the product: back to back under
+// programmatic launch the kernels cost more than by themselves (NN = 19 without
+// it: 1446 and 570).
+//
+// complex64 is at 71-93 % of the HBM time from NN = 15 on.  complex128 is held
 // back by the cube kernel: one CTA of NN^2 threads per SM from NN = 17 on (two
 // cubes of shared memory), whose load, FP64 and store phases do not overlap.
 // Staging part of the cube to fit two CTAs measured slower (340-460 us at NN
